@@ -18,6 +18,7 @@
 #include "../../include/shearbox.h"
 #include "sb_common.cuh"
 #include "sb_fac.h"
+#include "sb_fix.cuh"
 #include "sb_host.h"
 #include "sb_kernels.h"
 
@@ -65,6 +66,12 @@ struct sb_handle {
   // the host copies of phi run on the side stream beside those of omega_y
   cudaEvent_t ev_c0 = nullptr, ev_c1 = nullptr;
   cudaGraphExec_t step_exec = nullptr;
+  // boxes whose image offsets are not opposite (xoffb != -xofft): the
+  // Bloch-wave form needs one phase for both images, so while there is one
+  // the step runs the banded solves; step_bloch is the form captured
+  std::vector<char> asym;
+  int nasym = 0;
+  bool step_bloch = false;
   std::vector<void *> allocs;
   // the factor tables of the y-line solves depend on the segment plan: kept
   // apart so that a new plan (sb_set_line_segments, the autotuner) can
@@ -106,6 +113,14 @@ static int upload(sb_handle *h, const double **dst, const std::vector<double> &v
   CK(cudaMemcpy(p, v.data(), sizeof(double) * v.size(), cudaMemcpyHostToDevice));
   *dst = p;
   return 0;
+}
+
+// the y-line stage runs on Bloch waves (sb_bloch.cu)
+static bool use_bloch(const sb_handle *h) { return h->g.bloch && h->g.lform && h->nasym == 0; }
+static void note_offsets(sb_handle *h, int member, double xoffb, double xofft) {
+  const char a = (xoffb != -xofft);
+  h->nasym += a - h->asym[member];
+  h->asym[member] = a;
 }
 
 static int check_params(const sb_params *p) {
@@ -333,6 +348,47 @@ static int build_line_tables(sb_handle *h, int nseg) {
 }
 
 
+// fixed-point twiddles of length n
+static int upload_fix(sb_handle *h, const qw **dst, int n, int sign, bool scaled) {
+  const std::vector<int> v = sbh::fix_twiddles(n, sign, scaled);
+  double *q;
+  const int rc = dalloc(h, &q, 2 * (size_t)n);
+  if (rc) return rc;
+  CK(cudaMemcpy(q, v.data(), sizeof(qw) * n, cudaMemcpyHostToDevice));
+  *dst = (const qw *)q;
+  return 0;
+}
+
+// constants and tables of the Bloch-wave form (sb_bloch.cu)
+static int build_bloch_tables(sb_handle *h) {
+  Grid &g = h->g;
+  Bufs &bf = h->bf;
+  h->asym.assign((size_t)g.B, 0);
+  g.bloch = line_bloch_ok(g) ? 1 : 0;
+  if (!g.bloch) return 0;
+  sbh::Coeffs co;
+  sbh::compact_coeffs(&co);
+  const int n = g.my;
+  typedef long double ld;
+  for (int d = 1; d <= 3; d++) g.bpr1[d - 1] = co.pr1[3 + d];
+  g.bn20 = (double)((ld)g.rh2[3] + 2.0L * ((ld)g.rh2[4] + g.rh2[5] + g.rh2[6]));
+  g.bn1p = (double)((ld)g.rh1[4] - 2.0L * g.rh1[5] + 3.0L * g.rh1[6]);
+  g.bp1p = (double)(1.0L - 2.0L * ((ld)co.pr1[4] - co.pr1[5] + co.pr1[6]));
+  g.bp2p = (double)(1.0L - 2.0L * ((ld)co.pr2[4] - co.pr2[5] + co.pr2[6]));
+  const size_t m = 3 * (size_t)g.B * n * g.nkx;
+  int rc;
+  double *q;
+  if ((rc = dalloc(h, &q, 2 * m))) return rc;
+  bf.btw = (qw *)q;
+  if ((rc = dalloc(h, &bf.bl1, m)) || (rc = dalloc(h, &bf.bl2, m)) ||
+      (rc = upload_fix(h, &bf.bftw, n, -1, false)) || (rc = upload_fix(h, &bf.bitw, n, 1, true)) ||
+      (rc = upload_fix(h, &bf.bturn, 1024, -1, false)))
+    return rc;
+  if (prepare_lineQ(g, bf) != cudaSuccess)
+    return fail(3, "line kernel attributes: %s", cudaGetErrorString(cudaGetLastError()));
+  return 0;
+}
+
 static void member_defaults(const sb_params *p, const Grid &g, double Re, Member *m) {
   memset(m, 0, sizeof(Member));
   const double pi = g.pi;
@@ -365,6 +421,9 @@ static int capture_step(sb_handle *h) {
     h->step_exec = nullptr;
   }
   cudaGraph_t graph;
+  h->step_bloch = use_bloch(h);
+  h->bf.Gn = h->step_bloch ? h->bf.S : h->bf.G;
+  h->bf.Dn = h->step_bloch ? h->bf.T : h->bf.D;
   CK(cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
   cudaError_t e = cudaSuccess;
   for (int rk = 1; rk <= 3 && e == cudaSuccess; rk++) {
@@ -396,6 +455,7 @@ static int capture_step(sb_handle *h) {
           (e = cudaStreamWaitEvent(h->side, h->ev_fork, 0)) != cudaSuccess ||
           (e = launch_scalar(h->g, h->bf, rk, h->side)) != cudaSuccess ||
           (e = launch_tables(h->g, h->bf, rk, h->side)) != cudaSuccess ||
+          (h->step_bloch && (e = launch_bloch(h->g, h->bf, rk, h->side)) != cudaSuccess) ||
           (h->g.impl && (e = launch_hfac(h->g, h->bf, rk, h->side)) != cudaSuccess) ||
           (e = cudaEventRecord(h->ev_join, h->side)) != cudaSuccess ||
           (e = launch_plane(h->g, h->bf, 3, rk, h->st)) != cudaSuccess ||
@@ -408,11 +468,16 @@ static int capture_step(sb_handle *h) {
       if (h->g.les && (e = launch_les(h->g, h->bf, 5, rk, h->st)) != cudaSuccess) break;
       if ((e = launch_scalar(h->g, h->bf, rk, h->st)) != cudaSuccess) break;
       if ((e = launch_tables(h->g, h->bf, rk, h->st)) != cudaSuccess) break;
+      if (h->step_bloch && (e = launch_bloch(h->g, h->bf, rk, h->st)) != cudaSuccess) break;
       if (h->g.impl && (e = launch_hfac(h->g, h->bf, rk, h->st)) != cudaSuccess) break;
     }
     if (h->g.les && (e = launch_lineL(h->g, h->bf, h->st)) != cudaSuccess) break;
     if (h->g.impl) {
       e = launch_lineI(h->g, h->bf, rk, h->st);
+      continue;
+    }
+    if (h->step_bloch) {
+      e = launch_lineQ(h->g, h->bf, rk, h->st);
       continue;
     }
     if (h->g.lform && line_fused_ok(h->g)) {
@@ -429,6 +494,14 @@ static int capture_step(sb_handle *h) {
   CK(cudaGraphInstantiate(&h->step_exec, graph, 0));
   cudaGraphDestroy(graph);
   return 0;
+}
+
+// v from phi and the first derivatives of the state at the start of a run, by
+// the solves of the captured step (the phase tables of slot 0 first)
+static cudaError_t launch_prologue(sb_handle *h) {
+  if (!h->step_bloch) return launch_lineB(h->g, h->bf, 0, h->st);
+  cudaError_t e = launch_bloch(h->g, h->bf, 0, h->st);
+  return e != cudaSuccess ? e : launch_lineQ(h->g, h->bf, 0, h->st);
 }
 
 static int ensure_trace(sb_handle *h, int cap) {
@@ -714,7 +787,7 @@ int sb_create(const sb_params *p, int batch, int precision, sb_handle **out) {
     sb_destroy(h);
     return rc;
   }
-  if ((rc = build_line_tables(h, g.nseg))) {
+  if ((rc = build_line_tables(h, g.nseg)) || (rc = build_bloch_tables(h))) {
     sb_destroy(h);
     return rc;
   }
@@ -797,6 +870,7 @@ static int set_state_impl(sb_handle *h, int member, const double *vor, const dou
   const Grid &g = h->g;
   const size_t F = g.field;
   const size_t Fd = g.prec ? F / 2 : F;  // field size in doubles of the storage type
+  note_offsets(h, member, xoffb, xofft);
   // phi on the side stream, after the work already queued on the main one
   CK(cudaEventRecord(h->ev_c0, h->st));
   CK(cudaStreamWaitEvent(h->side, h->ev_c0, 0));
@@ -902,6 +976,7 @@ int sb_set_state_packed(sb_handle *h, int member, const double *x, const double 
   const Grid &g = h->g;
   const size_t Fd = g.prec ? g.field / 2 : g.field;
   const size_t mud = g.prec ? (size_t)g.my : 2 * (size_t)g.my;  // doubles per member's mean line
+  note_offsets(h, member, xoffb, xofft);
   CK(launch_unpack(g, x, h->bf.vor + member * Fd, h->bf.phi + member * Fd,
                    h->bf.mu + member * mud, sca, h->st));
   // the pinned staging may feed an earlier copy still in flight
@@ -1004,13 +1079,17 @@ int sb_step(sb_handle *h, int nsteps) {
   if (nsteps < 0) return fail(1, "nsteps < 0");
   int rc = ensure_trace(h, nsteps > 0 ? nsteps : 1);
   if (rc) return rc;
+  if (h->step_bloch != use_bloch(h)) {
+    CK(cudaStreamSynchronize(h->st));
+    if ((rc = capture_step(h))) return rc;
+  }
   // entry of cross(): flags and offsets, phase tables, set_conj on the state,
   // v from phi and the first derivatives (cross.f90:76-113,283-287,376-445)
   CK(launch_scalar(h->g, h->bf, 0, h->st));
   CK(launch_tables(h->g, h->bf, 0, h->st));
   CK(launch_setconj(h->g, h->bf, h->st));
   if (h->g.ydeal == 3) CK(launch_filter(h->g, h->bf, 0, h->st));
-  CK(launch_lineB(h->g, h->bf, 0, h->st));
+  CK(launch_prologue(h));
   for (int s = 0; s < nsteps; s++) CK(cudaGraphLaunch(h->step_exec, h->st));
   return 0;
 }
@@ -1109,7 +1188,7 @@ int sb_launch_stage(sb_handle *h, int stage, int rk, int count) {
   if (!h || count < 0) return fail(1, "bad argument");
   if (stage < 1 || stage > 14 || rk < 1 || rk > 3) return fail(1, "stage 1..14, rk 1..3");
   if (stage >= 7 && stage <= 11 && !h->g.les) return fail(1, "stages 7..11 need an LES handle");
-  if (stage == 12 && !line_fused_ok(h->g))
+  if (stage == 12 && !h->step_bloch && !line_fused_ok(h->g))
     return fail(1, "stage 12 (fused y-line kernel) not available for this handle");
   if (stage >= 13 && !h->g.impl) return fail(1, "stages 13, 14 need an implicit_visc handle");
   for (int q = 0; q < count; q++) {
@@ -1127,7 +1206,7 @@ int sb_launch_stage(sb_handle *h, int stage, int rk, int count) {
     else if (stage == 11)
       e = launch_lineL(h->g, h->bf, h->st);
     else if (stage == 12)
-      e = launch_lineF(h->g, h->bf, rk, h->st);
+      e = h->step_bloch ? launch_lineQ(h->g, h->bf, rk, h->st) : launch_lineF(h->g, h->bf, rk, h->st);
     else if (stage == 13)
       e = launch_hfac(h->g, h->bf, rk, h->st);
     else
@@ -1184,7 +1263,7 @@ static cudaError_t launch_step_call(sb_handle *h, int nsteps) {
       (e = launch_tables(h->g, h->bf, 0, h->st)) != cudaSuccess ||
       (e = launch_setconj(h->g, h->bf, h->st)) != cudaSuccess ||
       (h->g.ydeal == 3 && (e = launch_filter(h->g, h->bf, 0, h->st)) != cudaSuccess) ||
-      (e = launch_lineB(h->g, h->bf, 0, h->st)) != cudaSuccess)
+      (e = launch_prologue(h)) != cudaSuccess)
     return e;
   for (int s = 0; s < nsteps && e == cudaSuccess; s++) e = cudaGraphLaunch(h->step_exec, h->st);
   return e;
@@ -1256,11 +1335,16 @@ int sb_autotune(sb_handle *h, int *choice) {
   for (int c : {1, 2, 3}) {
     if (rc || e != cudaSuccess) break;
     if ((g.my - 3) / c < 6) continue;
+    if (g.bloch && h->nasym == 0 && !g.les && c != nseg) continue;
     if ((rc = build_line_tables(h, c))) break;
-    // both forms of the y-line stage where the fused one is available
-    for (int f = 1; f >= 0; f--) {
+    // both forms of the y-line stage where the fused one is available.  The
+    // Bloch-wave form needs no trial against the split kernels (192x96x96
+    // FP64: 105 us a substep against 123 + 258) and has no segments: one trial,
+    // or with LES, whose k_lineL is segmented, one per tile
+    const bool bloch = g.bloch && h->nasym == 0;
+    for (int f = 1; f >= (bloch ? 1 : 0); f--) {
       if (rc || e != cudaSuccess) break;
-      if (f == 1 && !line_fused_ok(g)) continue;
+      if (f == 1 && !bloch && !line_fused_ok(g)) continue;
       g.lform = f;
       if ((rc = capture_step(h))) break;
       for (int q = 0; q < 3 && e == cudaSuccess; q++) {
@@ -1327,7 +1411,7 @@ int sb_set_line_segments(sb_handle *h, int nseg) {
 int sb_set_line_form(sb_handle *h, int form) {
   if (!h) return fail(1, "null handle");
   if (form != 0 && form != 1) return fail(1, "line form %d (0 split, 1 fused)", form);
-  if (form == 1 && !line_fused_ok(h->g))
+  if (form == 1 && !h->g.bloch && !line_fused_ok(h->g))
     return fail(1, "fused y-line kernel not available for this handle");
   h->g.lform = form;
   return capture_step(h);
@@ -1348,7 +1432,7 @@ int sb_get_side_branch(sb_handle *h, int *mask) {
 
 int sb_get_line_form(sb_handle *h, int *form) {
   if (!h || !form) return fail(1, "null argument");
-  *form = h->g.impl ? 2 : ((h->g.lform && line_fused_ok(h->g)) ? 1 : 0);
+  *form = h->g.impl ? 2 : ((h->g.lform && (use_bloch(h) || line_fused_ok(h->g))) ? 1 : 0);
   return 0;
 }
 
@@ -1382,6 +1466,8 @@ int sb_physical_fields(sb_handle *h, int member, unsigned mask, double *out) {
   gl.nzf = 10;
   gl.temp = 0;
   Bufs bl = h->bf;
+  bl.Gn = bl.G;
+  bl.Dn = bl.D;
   const long Fd = g.prec ? g.field / 2 : g.field;
   const long Md = g.prec ? (long)g.my : 2L * g.my;
   bl.vor += member * Fd;

@@ -1,0 +1,506 @@
+// sb_bloch.cu -- the y-line work of one explicit RK3 substep on Bloch waves.
+//
+// On the uniform grid with shear-periodic images u(y + Ly) = shp u(y),
+// shp = exp(i psi), every compact operator of the substep (d/dy, d2/dy2, the
+// Helmholtz solve) is a circulant matrix twisted by that phase, so the Bloch
+// waves exp(i t_m j), t_m = (psi + 2 pi m)/my, diagonalise all of them: d/dy is
+// i l1(t), d2/dy2 is l2(t), lapcdy is 1/(l2(t) - k^2), with l1 = 2 sum rh1_d
+// sin(d t) / (1 + 2 sum pr1_d cos(d t)) and l2 alike (the symbols of the
+// compact schemes, diffy_shear_hepta.f90:68-296).  A line goes through
+//   phi      D, phi at the phase of t  -> -d(D)/dy + nu (d2/dy2 - k^2) phi,
+//            RK3 update, remap (cross.f90:565-781); phi at the phase of
+//            t + c_k dt -> v = lapcdy(phi) -> G, dv/dy -> V
+//   omega_y  nu (d2/dy2 - k^2) omega_y, update, remap; d(omega_y)/dy -> D
+//   mean     the same for u00 and w00 (nu d2/dy2, forcing, update, d/dy)
+// with the transforms in 64-bit fixed point (sb_fix.cuh): six (phi) or four
+// (omega_y) transforms of my points per line at some 80 integer instructions
+// per point, where the banded solves (sb_seg.cuh) spend six solves of 46 FP64
+// instructions per complex row at 64 cycles each.
+//
+// A block takes kCols kx columns of one kz (16 bytes x 8 columns: full lines of
+// global and conflict-free rows of shared memory).  Transform of my = R1 R2
+// points: thread (n2, column) owns the rows n2 + R2 n1 (R1-point kernels),
+// thread (k1, column) the waves k1 + R1 k2 (R2-point kernels); one exchange
+// through shared memory between them, none between a forward transform and
+// the inverse ones that follow it.
+#include <cuda_runtime.h>
+
+#include "sb_common.cuh"
+#include "sb_fix.cuh"
+#include "sb_kernels.h"
+
+// Compiled six times: SB_FLOAT_TU = 0 (FP64) or 1 (FP32-mixed) storage times
+// SB_LEN = 0 (my 32..80), 1 (96..192), 2 (256..384); unit (0, 0) also holds
+// the entry points.
+#ifndef SB_FLOAT_TU
+#define SB_FLOAT_TU 0
+#endif
+#ifndef SB_LEN
+#define SB_LEN 0
+#endif
+#define SB_CAT2(a, b, c) a##b##_##c
+#define SB_CAT(a, b, c) SB_CAT2(a, b, c)
+#define SB_LINEQ_UNIT(f, l) SB_CAT(lineQ_unit, f, l)
+
+namespace sb {
+
+namespace {
+
+constexpr int kCols = 8;
+constexpr int kNoLen = -(1 << 28);  // scale of nothing
+
+template <typename R> struct V2;
+template <> struct V2<double> { typedef double2 t; };
+template <> struct V2<float> { typedef float2 t; };
+template <typename R>
+__device__ __forceinline__ typename V2<R>::t mkv(R a, R b) {
+  typename V2<R>::t v;
+  v.x = a;
+  v.y = b;
+  return v;
+}
+template <typename V>
+__device__ __forceinline__ unsigned vtop(V v) {
+  const unsigned a = hiword(v.x), b = hiword(v.y);
+  return a > b ? a : b;
+}
+template <typename V>
+__device__ __forceinline__ q2 vfix(V v, const QScale &s) {
+  return mkq(tofix(v.x, s), tofix(v.y, s));
+}
+
+// hides where a pointer comes from, so that the loads of a loop that runs once
+// or twice are not moved ahead of it (they would not fit in the registers)
+template <typename P>
+__device__ __forceinline__ P *here(P *p) {
+  asm volatile("" : "+l"(p));
+  return p;
+}
+
+}  // namespace
+
+template <int N>
+struct LineQ {
+  static constexpr int R1 = Plan<N>::R1, R2 = Plan<N>::R2;
+  static constexpr int RM = R1 > R2 ? R1 : R2;
+  static constexpr int T = kCols * RM;
+  static constexpr int kShiftF = 2 + Plan<N>::shift;  // twist and forward transform
+  static constexpr int kBits = Plan<N>::bits + 2;     // the twist divides by 4
+  static constexpr size_t smem = 2 * sizeof(q2) * N * kCols;
+};
+SB_HD constexpr int floor_log2(int n) { return n < 2 ? 0 : 1 + floor_log2(n / 2); }
+
+// Forward transform, row part: the raw rows of thread (n2, ci) in its slots of
+// ex, scaled and twisted, to y[k1][n2] in the same slots.  Row j and y[k1][n2]
+// with j = k1 R2 + n2 share slot j, so every part works in place.
+template <int N, typename V>
+__device__ __forceinline__ void rows_forward(q2 *ex, const QScale &sc, const qw *__restrict__ twist,
+                                             int nkx, const qw *__restrict__ tw, int n2, int ci) {
+  typedef LineQ<N> L;
+  q2 v[L::R1];
+#pragma unroll
+  for (int n1 = 0; n1 < L::R1; n1++) {
+    const int j = n2 + L::R2 * n1;
+    v[n1] = qmul<false>(vfix(*(const V *)(ex + j * kCols + ci), sc), twist[(long)j * nkx]);
+  }
+  Dft<L::R1, -1>::run(v);
+#pragma unroll
+  for (int k1 = 0; k1 < L::R1; k1++)
+    ex[(k1 * L::R2 + n2) * kCols + ci] = qmul<false>(v[k1], tw[n2 * k1]);
+}
+// inverse transform, row part: y[k1][n2] of thread (n2, ci) to its rows, untwisted
+template <int N>
+__device__ __forceinline__ void rows_inverse(q2 *ex, const qw *__restrict__ twist, int nkx, int n2,
+                                             int ci) {
+  typedef LineQ<N> L;
+  q2 v[L::R1];
+#pragma unroll
+  for (int k1 = 0; k1 < L::R1; k1++) v[k1] = ex[(k1 * L::R2 + n2) * kCols + ci];
+  Dft<L::R1, 1>::run(v);
+#pragma unroll
+  for (int n1 = 0; n1 < L::R1; n1++) {
+    const int j = n2 + L::R2 * n1;
+    ex[j * kCols + ci] = qmul<true>(v[n1], twist[(long)j * nkx]);
+  }
+}
+
+// registers per thread the kernel is budgeted for: R1, R2 <= 12, and above
+#ifndef SB_LINEQ_REGS
+#define SB_LINEQ_REGS 128
+#endif
+#ifndef SB_LINEQ_REGS16
+#define SB_LINEQ_REGS16 168
+#endif
+// rk1 = 1..3: the substep; 0: the start of a run (v and the first derivatives
+// from the state, cross.f90:408-445).
+// Two passes over the same code (unrolled twice it would not fit in the
+// instruction cache, and each warp runs it only once): pass 0 takes the
+// right-hand side and the update at the phase of time t, pass 1 the outputs at
+// the phase of t + c_k dt.  A pass: rows in, forward, products, inverse, rows out.
+template <typename R, int N>
+__global__ void __launch_bounds__(
+    LineQ<N>::T, 65536 / (LineQ<N>::T * (LineQ<N>::RM > 12 ? SB_LINEQ_REGS16 : SB_LINEQ_REGS)))
+    k_lineQ(Grid g, Bufs bf, int rk1) {
+  typedef LineQ<N> L;
+  typedef typename V2<R>::t V;
+  constexpr int R1 = L::R1, R2 = L::R2;
+  constexpr int kN = floor_log2(N), kTgt = Plan<N>::bits;
+  const int b = blockIdx.y;
+  const Member &M = bf.mem[b];
+  if (M.halted) return;  // uniform per block
+  extern __shared__ __align__(16) unsigned char smq_raw[];
+  q2 *const ex = (q2 *)smq_raw;  // two buffers of N x kCols
+  __shared__ unsigned s_top[3][kCols];  // largest upper words: state, D, new state
+  __shared__ int s_len[3][kCols];       // scales of the products: right-hand side, first, second output
+  const int ncb = (g.nkx + kCols - 1) / kCols, per = g.mz * ncb;
+  const int role = blockIdx.x / per;  // 0 phi, 1 omega_y, 2 mean
+  const int r = blockIdx.x - role * per;
+  const bool mean = role == 2;
+  const int ci = threadIdx.x & (kCols - 1), n = threadIdx.x / kCols;
+  const int k = mean ? 0 : r / ncb;
+  const int i0 = mean ? ci : (r - k * ncb) * kCols + ci;
+  const bool act = mean ? ci < 2 : i0 < g.nkx;
+  const int cm = ci & 1;  // mean: u00 in column 0, w00 in column 1
+  const int i = mean ? 0 : (act ? i0 : g.nkx - 1);
+  const bool is00 = !mean && i == 0 && k == 0;
+  const int nkx = g.nkx;
+  const long ps = g.plane / 2;  // complex entries per plane
+  const long off = (long)b * (g.field / 2) + (long)k * nkx + i;
+  const bool t1 = n < R2, t2 = n < R1;  // threads of the row and of the wave kernels
+  const int rk = rk1 - 1;
+  if (threadIdx.x < 3 * kCols) {
+    (&s_top[0][0])[threadIdx.x] = 0u;
+    (&s_len[0][0])[threadIdx.x] = kNoLen;
+  }
+  __syncthreads();
+  const long tb = (long)N * nkx;
+  const double a = g.alp * i, gz = g.gam * ((k <= g.nz) ? k : k - g.mz);
+  const double k2 = mean ? 0.0 : a * a + gz * gz;
+  const double nu = is00 ? 0.0 : M.nu, nuk2 = nu * k2;
+  V *f = (V *)(role == 0 ? bf.phi : bf.vor) + off;
+  R *mf = (R *)bf.mu + (long)b * 2 * N + cm;  // mean profile of this column
+#pragma unroll 1
+  for (int ph = rk1 > 0 ? 0 : 1; ph < 2; ph++) {
+    // phase tables: slot 0 holds the phases of a step's start, slots 1 and 2
+    // those after its first and second substep, its third refills slot 0
+    const long o = ((long)((ph == 0 ? rk : rk1) % 3) * g.B + b) * tb + i;
+    const qw *tw = bf.btw + o;
+    const double *l1 = bf.bl1 + o, *l2 = bf.bl2 + o;
+    const int nf = ph == 0 && role == 0 ? 2 : 1;  // fields in: the state, D
+    const int no = ph == 1 && role == 0 ? 2 : 1;  // fields out
+    // ---- rows in (the new state is in buffer 0 already)
+    if (ph == 0 || rk1 == 0) {
+#pragma unroll 1
+      for (int q = 0; q < nf; q++) {
+        const V *src = q ? (const V *)bf.Dn + off : f;
+        unsigned top = 0;
+#pragma unroll 4
+        for (int j = n; j < N; j += L::RM) {
+          const V w = mean ? mkv<R>(mf[2 * j], (R)0) : src[(long)j * ps];
+          *(V *)(ex + (q * N + j) * kCols + ci) = w;
+          top = max(top, vtop(w));
+        }
+        atomicMax(&s_top[ph == 0 ? q : 2][ci], top);
+      }
+    }
+    __syncthreads();
+    const QScale s0 = qscale(s_top[ph == 0 ? 0 : 2][ci], L::kBits);
+    const QScale s1 = qscale(s_top[1][ci], L::kBits);
+    const bool bad = s0.bad || (nf > 1 && s1.bad);
+    if (t1)
+#pragma unroll 1
+      for (int q = 0; q < nf; q++)
+        rows_forward<N, V>(ex + q * N * kCols, q ? s1 : s0, here(tw), nkx, here(bf.bftw), n, ci);
+    __syncthreads();
+    // ---- products.  Pass 0: nu (l2 - k^2) f - i l1 D; pass 1: phi f/(l2 - k^2)
+    // and i l1 of it, else i l1 f.  The waves stay in the thread's own slots
+    // while the scale of each product is found over the whole line.
+    double c[R2];  // nu (l2 - k^2), 1/(l2 - k^2) or l1
+    if (t2) {
+#pragma unroll
+      for (int q = 0; q < R2; q++) {
+        const long p = (long)(n + R1 * q) * nkx;
+        if (ph == 0) {
+          c[q] = fma(nu, l2[p], -nuk2);
+        } else if (role == 0) {
+          // reciprocal by two Newton steps from the 20-bit estimate
+          const double den = l2[p] - k2;
+          double z;
+          asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(z) : "d"(den));
+          z = fma(z, fma(-den, z, 1.0), z);
+          z = fma(z, fma(-den, z, 1.0), z);
+          c[q] = is00 ? 0.0 : z;
+        } else {
+          c[q] = l1[p];
+        }
+      }
+#pragma unroll 1
+      for (int q = 0; q < nf; q++) {
+        q2 *e = ex + (q * N + n * R2) * kCols + ci;
+        const double *l = here(l1);
+        q2 x[R2];
+#pragma unroll
+        for (int w = 0; w < R2; w++) x[w] = e[w * kCols];
+        Dft<R2, -1>::run(x);
+        int la = kNoLen, lb = kNoLen;
+#pragma unroll
+        for (int w = 0; w < R2; w++) {
+          e[w * kCols] = x[w];
+          const int len = qlen(x[w]), e1 = qexp(l[(long)(n + R1 * w) * nkx]);
+          la = max(la, len + (q ? e1 : qexp(c[w])));
+          lb = max(lb, len + qexp(c[w]) + e1 + 1);
+        }
+        atomicMax(&s_len[ph][ci], la - (ph == 0 ? (q ? s1.p : s0.p) : 0));
+        if (no > 1) atomicMax(&s_len[2][ci], lb);
+      }
+    }
+    __syncthreads();
+    // scales of the outputs; in pass 0 of the sum of two terms
+    const int len1 = s_len[ph][ci] + (ph == 0 ? 2 : 1), len2 = s_len[2][ci] + 1;
+    if (t2) {
+      q2 y[R2];
+#pragma unroll 1
+      for (int q = max(nf, no) - 1; q >= 0; q--) {
+        // pass 0: q = 1 D, 0 f, added; pass 1: q = 1 the second output, 0 the first
+        const q2 *e = ex + ((nf > 1 ? q : 0) * N + n * R2) * kCols + ci;
+        const bool first = no > 1 || q == nf - 1;
+        const double *l = here(l1);
+        const qw *it = here(bf.bitw);
+        const int sh = kTgt - (no > 1 && q ? len2 : len1) - (ph == 0 ? (q ? s1.p : s0.p) : 0);
+#pragma unroll
+        for (int w = 0; w < R2; w++) {
+          double d = c[w];
+          if (q) {
+            d = l[(long)(n + R1 * w) * nkx];
+            if (ph == 1) d *= c[w];
+          }
+          q2 z = qscaled(e[w * kCols], d, sh);
+          // times -i (D), i (d/dy of an output) or 1
+          if (ph == 0 ? q : (role != 0 || q)) z = ph == 0 ? qrot<-1>(z) : qrot<1>(z);
+          y[w] = first ? z : y[w] + z;
+        }
+        if (no > 1 || q == 0) {
+          Dft<R2, 1>::run(y);
+          q2 *eo = ex + ((no > 1 ? q : 0) * N + n * R2) * kCols + ci;
+#pragma unroll
+          for (int w = 0; w < R2; w++) eo[w * kCols] = qmul<false>(y[w], it[w * n]);
+        }
+      }
+    }
+    __syncthreads();
+    if (t1)
+#pragma unroll 1
+      for (int q = 0; q < no; q++) rows_inverse<N>(ex + q * N * kCols, here(tw), nkx, n, ci);
+    __syncthreads();
+    // ---- rows out
+    const int eb = L::kShiftF + Plan<N>::shift + 2 - kN - kTgt;
+    if (ph == 1) {
+      const int e0 = eb - s0.p;
+      const R nn = (R)nan("");
+      if (mean) {
+        R *dst = (R *)bf.mdu + (long)b * 2 * N + cm;
+        if (act)
+#pragma unroll 1
+          for (int j = n; j < N; j += L::RM)
+            dst[2 * j] = bad ? nn : qout<R>(ex[j * kCols + ci].x, e0 + len1);
+      } else if (act) {
+#pragma unroll 1
+        for (int q = 0; q < no; q++) {
+          // the (0,0) line of v keeps the value zero it is given at the start of a run
+          if (role == 0 && q == 0 && is00 && rk1 > 0) continue;
+          V *dst = (V *)(role != 0 ? bf.D : q ? bf.V : bf.G) + off;
+          const int eo = e0 + (q ? len2 : len1);
+#pragma unroll 2
+          for (int j = n; j < N; j += L::RM) {
+            const q2 z = ex[(q * N + j) * kCols + ci];
+            dst[(long)j * ps] = bad ? mkv<R>(nn, nn) : mkv<R>(qout<R>(z.x, eo), qout<R>(z.y, eo));
+          }
+        }
+      }
+      return;
+    }
+    // RK3 accumulation and update, zeta store, remaps (cross.f90:694-781)
+    const int eo = eb + len1;
+    const R gk = (R)kGama[rk], zk = (R)kZeta[rk], dtr = (R)M.Deltat;
+    unsigned top = 0;
+    if (mean) {
+      R *mwk = (R *)bf.mwk + (long)b * 2 * N + cm;
+      const R *mrf = (const R *)bf.mrf + (long)b * 2 * N + cm;
+      const bool damp = g.damp && ci == 0, xf = g.force == -1 && ci == 0;
+#pragma unroll 1
+      for (int j = n; j < N; j += L::RM) {
+        R un = (R)0;
+        if (act) {
+          // forcing and damping (cross.f90:622-626; operators.f90:60-78)
+          R rf0 = mrf[2 * j];
+          if (xf) rf0 = (R)((double)rf0 + g.xforce);
+          if (damp) {
+            const double y = (double)j * g.dy - 0.5 * g.Ly;
+            const double hw = 1.0 - (0.25 * (1.0 + tanh(6.0 * (g.damp_a - y) / g.lz + 3.0))) *
+                                        (1.0 + tanh(6.0 * (g.damp_a + y) / g.lz + 3.0));
+            rf0 = (R)((double)rf0 - g.damp_up * hw * (double)mf[2 * j]);
+          }
+          const R rf = rf0 + (bad ? (R)nan("") : qout<R>(ex[j * kCols + ci].x, eo));
+          R wk = (rk == 0) ? gk * rf : mwk[2 * j] + gk * rf;
+          un = mf[2 * j] + dtr * wk;
+          if (rk < 2) wk = rf * zk;
+          mf[2 * j] = un;
+          mwk[2 * j] = wk;
+        }
+        const V w = mkv<R>(un, (R)0);
+        top = max(top, vtop(w));
+        *(V *)(ex + j * kCols + ci) = w;
+      }
+    } else {
+      const V *rhs = (const V *)(role == 0 ? bf.V : bf.Gn) + off;
+      V *fwk = (V *)(role == 0 ? bf.phiwk : bf.vorwk) + off;
+      const double2 *m1 = (const double2 *)bf.mf1 + (long)b * tb + i;
+      const double2 *m2 = (const double2 *)bf.mf2 + (long)b * tb + i;
+      const V none = mkv<R>((R)0, (R)0);
+#pragma unroll 2
+      for (int j = n; j < N; j += L::RM) {
+        const long q = (long)j * ps;
+        const V fo = f[q], rh = rhs[q], w0 = rk > 0 ? fwk[q] : none;
+        const q2 z = ex[j * kCols + ci];
+        V h = mkv<R>(rh.x + qout<R>(z.x, eo), rh.y + qout<R>(z.y, eo));
+        if (bad) h = mkv<R>((R)nan(""), (R)nan(""));
+        V wk = mkv<R>(w0.x + gk * h.x, w0.y + gk * h.y);
+        const double fx = (double)(fo.x + dtr * wk.x), fy = (double)(fo.y + dtr * wk.y);
+        const double2 p2 = m2[(long)j * nkx];
+        const V fn = mkv<R>((R)fma(fx, p2.x, -(fy * p2.y)), (R)fma(fy, p2.x, fx * p2.y));
+        if (rk < 2) {
+          const double2 p1 = m1[(long)j * nkx];
+          const double zx = (double)(h.x * zk), zy = (double)(h.y * zk);
+          wk = mkv<R>((R)fma(zx, p1.x, -(zy * p1.y)), (R)fma(zy, p1.x, zx * p1.y));
+        }
+        if (act) {
+          f[q] = fn;
+          fwk[q] = wk;
+        }
+        top = max(top, vtop(fn));
+        *(V *)(ex + j * kCols + ci) = fn;
+      }
+    }
+    atomicMax(&s_top[2][ci], top);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// launchers
+// ---------------------------------------------------------------------------
+template <typename R, int N>
+static cudaError_t launch_t(const Grid &g, const Bufs &bf, int rk, cudaStream_t st, bool prep) {
+  if (prep)
+    return cudaFuncSetAttribute(k_lineQ<R, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)LineQ<N>::smem);
+  const int ncb = (g.nkx + kCols - 1) / kCols;
+  k_lineQ<R, N><<<dim3((unsigned)(2 * g.mz * ncb + 1), (unsigned)g.B), LineQ<N>::T, LineQ<N>::smem,
+                  st>>>(g, bf, rk);
+  return cudaGetLastError();
+}
+#if SB_FLOAT_TU
+typedef float UnitR;
+#else
+typedef double UnitR;
+#endif
+cudaError_t SB_LINEQ_UNIT(SB_FLOAT_TU, SB_LEN)(const Grid &g, const Bufs &bf, int rk,
+                                               cudaStream_t st, bool prep) {
+  switch (g.my) {
+#if SB_LEN == 0
+    case 32: return launch_t<UnitR, 32>(g, bf, rk, st, prep);
+    case 48: return launch_t<UnitR, 48>(g, bf, rk, st, prep);
+    case 64: return launch_t<UnitR, 64>(g, bf, rk, st, prep);
+    case 80: return launch_t<UnitR, 80>(g, bf, rk, st, prep);
+#elif SB_LEN == 1
+    case 96: return launch_t<UnitR, 96>(g, bf, rk, st, prep);
+    case 128: return launch_t<UnitR, 128>(g, bf, rk, st, prep);
+    case 160: return launch_t<UnitR, 160>(g, bf, rk, st, prep);
+    case 192: return launch_t<UnitR, 192>(g, bf, rk, st, prep);
+#else
+    case 256: return launch_t<UnitR, 256>(g, bf, rk, st, prep);
+    case 320: return launch_t<UnitR, 320>(g, bf, rk, st, prep);
+    case 384: return launch_t<UnitR, 384>(g, bf, rk, st, prep);
+#endif
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+#if !SB_FLOAT_TU && SB_LEN == 0
+// ---------------------------------------------------------------------------
+// the phase tables of slot sn for a box: per (row or wave m, kx) the twist
+// exp(-i psi m/my) and the symbols l1, l2 at t = (psi + 2 pi m)/my.  psi is
+// -kx xofft as a fraction of a turn: an error of the phase itself matters no
+// more than the rounding of exp(-i kx xofft), but the twists of the rows must
+// agree with each other to better than FP64 (their noise would be amplified by
+// (my/(dy k))^2 in a second derivative), hence the fixed-point qturn.  The
+// symbols are written in sin and cos of t/2, taken from the nearer of 0 and
+// pi, so that neither the long waves nor the ends of the spectrum cancel.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(64) k_bloch(Grid g, Bufs bf, int rk) {
+  const int b = blockIdx.y;
+  const Member &M = bf.mem[b];
+  if (M.halted) return;
+  const int N = g.my, nkx = g.nkx, sn = rk % 3;
+  const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= (long)N * nkx) return;
+  const int m = (int)(p / nkx), i = (int)(p - (long)m * nkx);
+  constexpr double kPi = 3.14159265358979323846, kInv = 0.15915494309189533577;  // 1/(2 pi)
+  double turn = 0.0;
+  if (fabs(g.s) > 0.01) {
+    const double arg = (-(g.alp * i)) * M.xwt[rk];
+    const double n = rint(arg * kInv);
+    double a = fma(-n, 6.283185307179586232, arg);
+    a = fma(-n, 2.4492935982947064e-16, a);  // 2 pi less its double
+    turn = a * kInv;
+  }
+  const ll X = __double2ll_rn(turn * 18446744073709551616.0);
+  const long o = ((long)sn * g.B + b) * N * nkx + p;
+  bf.btw[o] = qturn(X, m, N, bf.bturn);
+  // t/2 = pi (turn + ms)/N for |t| <= pi/2, else pi/2 less the rest
+  const int ms = 2 * m > N ? m - N : m;
+  const bool far = 4 * (ms < 0 ? -ms : ms) > N;
+  const double sg = ms < 0 ? -1.0 : 1.0;
+  const double h = far ? (0.5 * N - sg * ms) - sg * turn : (double)ms + turn;
+  double s, c;
+  sincos(kPi * h / (double)N, &s, &c);
+  if (far) {
+    const double t = s;
+    s = sg * c;
+    c = t;
+  }
+  const double s2 = s * s, c2 = c * c, st2 = 4.0 * s2 * c2;  // sin^2 t
+  const double a3 = 3.0 - 4.0 * s2, b3 = 4.0 * c2 - 3.0;     // sin and cos of 3 t/2 over those of t/2
+  const double n1 = 4.0 * s * c * (g.bn1p + 4.0 * (g.rh1[5] * c2 - g.rh1[6] * st2));
+  const double p1 = g.bp1p + 4.0 * (g.bpr1[0] * c2 - g.bpr1[1] * st2 + g.bpr1[2] * (c2 * b3 * b3));
+  const double n2 = g.bn20 - 4.0 * (g.rh2[4] * s2 + g.rh2[5] * st2 + g.rh2[6] * (s2 * a3 * a3));
+  const double p2 = g.bp2p + 4.0 * (g.pr2[4] * c2 - g.pr2[5] * st2 + g.pr2[6] * (c2 * b3 * b3));
+  bf.bl1[o] = n1 / p1;
+  bf.bl2[o] = n2 / p2;
+}
+
+typedef cudaError_t LineQUnit(const Grid &, const Bufs &, int, cudaStream_t, bool);
+LineQUnit lineQ_unit0_1, lineQ_unit0_2, lineQ_unit1_0, lineQ_unit1_1, lineQ_unit1_2;
+static cudaError_t lineQ(const Grid &g, const Bufs &bf, int rk, cudaStream_t st, bool prep) {
+  static LineQUnit *const unit[2][3] = {{lineQ_unit0_0, lineQ_unit0_1, lineQ_unit0_2},
+                                        {lineQ_unit1_0, lineQ_unit1_1, lineQ_unit1_2}};
+  return unit[g.prec ? 1 : 0][g.my < 96 ? 0 : g.my < 256 ? 1 : 2](g, bf, rk, st, prep);
+}
+
+// the plain explicit step (LES included: its k_lineL runs before) on the
+// transform lengths; the temperature, the y filter and dealiasing and the
+// semi-implicit branch keep the banded solves
+bool line_bloch_ok(const Grid &g) { return !g.temp && !g.ydeal && !g.impl && fix_length(g.my); }
+
+cudaError_t launch_lineQ(const Grid &g, const Bufs &bf, int rk, cudaStream_t st) {
+  return lineQ(g, bf, rk, st, false);
+}
+cudaError_t prepare_lineQ(const Grid &g, const Bufs &bf) { return lineQ(g, bf, 0, 0, true); }
+cudaError_t launch_bloch(const Grid &g, const Bufs &bf, int rk, cudaStream_t st) {
+  const long n = (long)g.my * g.nkx;
+  k_bloch<<<dim3((unsigned)((n + 63) / 64), (unsigned)g.B), 64, 0, st>>>(g, bf, rk);
+  return cudaGetLastError();
+}
+
+#endif  // unit (0, 0)
+
+}  // namespace sb

@@ -19,6 +19,8 @@
 
 namespace sb {
 
+struct qw;  // fixed-point constant (sb_fix.cuh)
+
 struct cd {
   double x, y;
 };
@@ -92,6 +94,12 @@ struct Grid {
   // kz=1) with amplitude force_roll; -1 the inertial force xforce on rf0u
   int force;
   double force_roll, xforce;
+  // Bloch-wave form of the y-line stage (sb_bloch.cu): available, the
+  // off-diagonal d/dy coefficients, the numerator of the d2/dy2 symbol at
+  // t = 0, that of d/dy over sin t and both denominators at t = pi (the sums
+  // that cancel there, taken in extended precision)
+  int bloch;
+  double bpr1[3], bn20, bn1p, bp1p, bp2p;
 };
 
 // Per-member run state, owned by the device (one per box in the batch)
@@ -168,6 +176,17 @@ struct Bufs {
   // [B][mz][nkx][8]; temperature tstats [B][my][5], splt [B][mz][nkx][4];
   // hist 'p' partials [B][my][mgalz/2][warps of a stage-2 block][3]
   double *stats, *stats2, *spec, *spec2, *tstats, *tspec, *ppart;
+  // Bloch-wave tables (sb_bloch.cu), three phase slots each [3][B][my][nkx]:
+  // twist, l1, l2; transform twiddles of my points, forward and inverse (the
+  // inverse ones times 2^floor(log2 my)/my), and e^{-2 pi i t/1024}
+  qw *btw;
+  double *bl1, *bl2;
+  const qw *bftw, *bitw, *bturn;
+  // nonlinear right-hand sides of the omega_y equation and of the d/dy term
+  // of the phi equation, as plane stage 3 leaves them: G and D, or with the
+  // Bloch-wave form S and T (its blocks write v and d(omega_y)/dy to G and D
+  // while others still read these)
+  double *Gn, *Dn;
 };
 
 // Asynchronous global -> shared copy of one element of NB bytes (4, 8 or 16,

@@ -405,4 +405,28 @@ std::vector<double> fft_twiddles_factored(int n) {
   return v;
 }
 
+std::vector<int> fix_twiddles(int n, int sign, bool scaled) {
+  const long double pi = std::acos(-1.0L);
+  long double f = 4611686018427387904.0L;  // 2^62
+  if (scaled) {
+    int p = 1;
+    while (2 * p <= n) p *= 2;
+    f *= (long double)p / (long double)n;
+  }
+  std::vector<int> v(4 * (size_t)n);
+  auto put = [](long double x, int *o) {
+    const long long w = std::llround(x);
+    int lo = (int)(uint32_t)(unsigned long long)w;
+    if (lo == INT32_MIN) lo++;  // its negative is used too
+    o[0] = (int)((w - (long long)lo) / 4294967296ll);
+    o[1] = lo;
+  };
+  for (int t = 0; t < n; t++) {
+    const long double a = 2.0L * pi * (long double)t / (long double)n;
+    put(f * std::cos(a), &v[4 * t]);
+    put((sign < 0 ? -f : f) * std::sin(a), &v[4 * t + 2]);
+  }
+  return v;
+}
+
 }  // namespace sbh

@@ -56,6 +56,12 @@ void seg_factor(const BaseFac &b, int n, const SegPlan &p, SegFac *out);
 std::vector<double> fft_twiddles(int n);
 std::vector<double> fft_twiddles_factored(int n);
 
+// Fixed-point twiddles e^{sign 2 pi i t/n} at 2^62 (sb_fix.cuh): per t four
+// integers re_hi, re_lo, im_hi, im_lo with re = re_hi 2^-30 + re_lo 2^-62, both
+// halves signed; scaled: times 2^floor(log2 n)/n (the power-of-two part of the
+// 1/n of an inverse transform is left to its scale).
+std::vector<int> fix_twiddles(int n, int sign, bool scaled);
+
 // Seeded divergence-free initial field (synthetic stand-in for the reference's
 // getini spectrum, initcr.f90:664-822): random-phase Fourier modes with energy
 // spectrum E(k) ~ k^4 exp(-2 (k/k0)^2), rms velocity urms.  Outputs the

@@ -538,8 +538,9 @@ __global__ void __launch_bounds__(T) k_p3(Grid g, Bufs bf) {
   cp_async_wait_all();
   V *P = fft_batch<NZ, -1, NF * CB, T>(A, Bs, (const V *)tw_of<R>(bf, true));
   const long pbase = (long)b * g.field + (long)j * g.plane;
-  V *Dv = (V *)((R *)bf.D + pbase);
-  V *Gv = (V *)((R *)bf.G + pbase);
+  V *Dv = (V *)((R *)bf.Dn + pbase);
+  const V *Gv = (const V *)((const R *)bf.G + pbase);
+  V *Gn = (V *)((R *)bf.Gn + pbase);
   V *Vv = (V *)((R *)bf.V + pbase);
   // 1/(mgalx mgalz) of the forward transform and the 1/2 of k_p2's row split
   const R norm = (R)(0.5 / (double)(g.mgalx * g.mgalz));
@@ -587,7 +588,7 @@ __global__ void __launch_bounds__(T) k_p3(Grid g, Bufs bf) {
     // hg = -i a H3 + i gz (H1 - s v)
     tx = gz * (H1.x - s * v.x) - a * H3.x;
     ty = gz * (H1.y - s * v.y) - a * H3.y;
-    Gv[q] = mk2<R>(-ty, tx);
+    Gn[q] = mk2<R>(-ty, tx);
     // hv = -(kx^2 + kz^2) H2
     V hv = mk2<R>(-(Kk * H2.x), -(Kk * H2.y));
     if (force && i == 0 && k == 1) hv.x = (R)((double)hv.x + fj);
@@ -834,8 +835,8 @@ __global__ void __launch_bounds__(T) k_les5(Grid g, Bufs bf) {
   }
   V *P = fft_batch<NZ, -1, 6 * CB, T>(A, Bs, (const V *)tw_of<R>(bf, true));
   const long pbase = (long)b * g.field + (long)j * g.plane;
-  V *Dv = (V *)((R *)bf.D + pbase);
-  V *Gv = (V *)((R *)bf.G + pbase);
+  V *Dv = (V *)((R *)bf.Dn + pbase);
+  V *Gv = (V *)((R *)bf.Gn + pbase);
   V *L1 = (V *)((R *)bf.L1 + pbase);
   V *L2 = (V *)((R *)bf.L2 + pbase);
   // 1/(mgalx mgalz) and the 1/2 of k_les4's row split (a power of two)

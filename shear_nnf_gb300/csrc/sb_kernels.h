@@ -35,6 +35,13 @@ cudaError_t launch_lineB(const Grid &g, const Bufs &bf, int mode, cudaStream_t s
 // k_lineB, where line_fused_ok(g)
 cudaError_t launch_lineF(const Grid &g, const Bufs &bf, int rk, cudaStream_t st);
 bool line_fused_ok(const Grid &g);
+// the same on Bloch waves (k_lineQ; rk 0: the start of a run) where
+// line_bloch_ok(g) and every box has xoffb = -xofft; launch_bloch fills its
+// phase tables
+bool line_bloch_ok(const Grid &g);
+cudaError_t prepare_lineQ(const Grid &g, const Bufs &bf);
+cudaError_t launch_lineQ(const Grid &g, const Bufs &bf, int rk, cudaStream_t st);
+cudaError_t launch_bloch(const Grid &g, const Bufs &bf, int rk, cudaStream_t st);
 // the semi-implicit viscous branch: factor tables of the substep (k_hfac)
 // and the y-line kernel (k_lineI)
 cudaError_t launch_hfac(const Grid &g, const Bufs &bf, int rk, cudaStream_t st);

@@ -1046,7 +1046,7 @@ __global__ void __launch_bounds__(32 * kSeg, SB_LINE_MINB) k_lineL(Grid g, Bufs 
     const TailLoad T1{bf.tl1o + ((long)L.b * g.nkx + i) * SB_TAIL};
     SEG_SOLVE((const R *)bf.L2 + off, ps, V1, W1, T1, shp, shm, 0.0, g.rh1[4], g.rh1[5], g.rh1[6],
               true);
-    R *G = (R *)bf.G + off;
+    R *G = (R *)bf.Gn + off;
     if (L.active)
       for (int r = L.r0; r <= L.r1; r++) {
         const long q = (long)(r - 1) * ps;
