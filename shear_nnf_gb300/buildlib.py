@@ -21,6 +21,9 @@ UNITS = [("sb_kernels.cu", ["-DSB_FLOAT_TU=0"]), ("sb_kernels.cu", ["-DSB_FLOAT_
          # the y-line kernels once per (warps per line solve, precision)
          *[("sb_yline.cu", [f"-DSB_FLOAT_TU={f}", f"-DSB_KSEG={k}"]) for k in (1, 2, 3)
            for f in (0, 1)],
+         # the fixed-point plane stages: z or x, without and with the temperature
+         *[("sb_planeq.cu", [f"-DSB_PLANE={k}", f"-DSB_TEMP={t}"]) for k in (0, 1)
+           for t in (0, 1)],
          # the Bloch-wave form once per (precision, range of line lengths)
          *[("sb_bloch.cu", [f"-DSB_FLOAT_TU={f}", f"-DSB_LEN={k}"]) for k in (0, 1, 2)
            for f in (0, 1)],

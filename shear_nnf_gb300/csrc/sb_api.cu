@@ -349,13 +349,50 @@ static int build_line_tables(sb_handle *h, int nseg) {
 
 
 // fixed-point twiddles of length n
-static int upload_fix(sb_handle *h, const qw **dst, int n, int sign, bool scaled) {
-  const std::vector<int> v = sbh::fix_twiddles(n, sign, scaled);
+static int upload_qw(sb_handle *h, const qw **dst, const std::vector<int> &v) {
   double *q;
-  const int rc = dalloc(h, &q, 2 * (size_t)n);
+  const int rc = dalloc(h, &q, v.size() / 2);
   if (rc) return rc;
-  CK(cudaMemcpy(q, v.data(), sizeof(qw) * n, cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(q, v.data(), sizeof(int) * v.size(), cudaMemcpyHostToDevice));
   *dst = (const qw *)q;
+  return 0;
+}
+static int upload_fix(sb_handle *h, const qw **dst, int n, int sign, bool scaled) {
+  return upload_qw(h, dst, sbh::fix_twiddles(n, sign, scaled));
+}
+
+// tables of the fixed-point plane stages (sb_planeq.cu)
+static int build_plane_tables(sb_handle *h) {
+  Grid &g = h->g;
+  Bufs &bf = h->bf;
+  g.planeq = (!g.prec && !g.les) ? 1 : 0;
+  if (!g.planeq) return 0;
+  const int n = g.mgalx;
+  int r1 = 0, r2 = 0;
+  switch (n) {
+#define SB_CASE(N) case N: r1 = Plan<N>::R1, r2 = Plan<N>::R2; break;
+    SB_CASE(32) SB_CASE(48) SB_CASE(64) SB_CASE(80) SB_CASE(96) SB_CASE(128) SB_CASE(160)
+    SB_CASE(192) SB_CASE(256) SB_CASE(320) SB_CASE(384)
+#undef SB_CASE
+  }
+  const std::vector<int> w = sbh::fix_twiddles(n, -1, false);
+  std::vector<int> a(4 * (size_t)n), b(4 * (size_t)n);
+  for (int k = 0; k < r1; k++)
+    for (int m = 0; m < r2; m++)
+      for (int q = 0; q < 4; q++) {
+        a[4 * (k * r2 + m) + q] = w[4 * (k * m) + q];
+        b[4 * (m * r1 + k) + q] = w[4 * (k * m) + q];
+      }
+  int rc;
+  double *q;
+  const size_t nze = (size_t)g.B * g.my * g.nzf * g.nkx;
+  const size_t nxe = (size_t)g.B * g.my * (g.mgalz / 2) * g.nxf;
+  if ((rc = upload_qw(h, &bf.fxa, a)) || (rc = upload_qw(h, &bf.fxb, b)) ||
+      (rc = upload_fix(h, &bf.fz, g.mgalz, -1, false)) || (rc = dalloc(h, &q, (nze + 1) / 2)))
+    return rc;
+  bf.ze = (int *)q;
+  if ((rc = dalloc(h, &q, (nxe + 1) / 2))) return rc;
+  bf.xe = (int *)q;
   return 0;
 }
 
@@ -787,7 +824,8 @@ int sb_create(const sb_params *p, int batch, int precision, sb_handle **out) {
     sb_destroy(h);
     return rc;
   }
-  if ((rc = build_line_tables(h, g.nseg)) || (rc = build_bloch_tables(h))) {
+  if ((rc = build_line_tables(h, g.nseg)) || (rc = build_bloch_tables(h)) ||
+      (rc = build_plane_tables(h))) {
     sb_destroy(h);
     return rc;
   }
@@ -1297,6 +1335,7 @@ int sb_autotune(sb_handle *h, int *choice) {
   float best = 1e30f, t = 0.0f;
   int cb1 = g.cb1, cb3 = g.cb3, t2 = g.t2;
   for (int c : {8, 4}) {  // plane stage 1: kx columns per block
+    if (g.planeq) break;  // the fixed-point plane stages have one tile
     g.cb1 = c;
     g.ncb = (g.nkx + c - 1) / c;
     if ((e = timed(1, &t)) != cudaSuccess) break;
@@ -1307,7 +1346,7 @@ int sb_autotune(sb_handle *h, int *choice) {
   const int t2d = plane_t2_default(g.mgalx);
   best = 1e30f;
   for (int c : {t2d, 2 * t2d}) {  // plane stage 2: threads per block
-    if (e != cudaSuccess) break;
+    if (e != cudaSuccess || g.planeq) break;
     g.t2 = c;
     if ((e = timed(2, &t)) != cudaSuccess) break;
     if (t < best) best = t, t2 = c;
@@ -1315,7 +1354,7 @@ int sb_autotune(sb_handle *h, int *choice) {
   g.t2 = t2;
   best = 1e30f;
   for (int c : {8, 4}) {  // plane stage 3: kx columns per block
-    if (e != cudaSuccess) break;
+    if (e != cudaSuccess || g.planeq) break;
     if (!plane3_fits(g, c)) continue;
     g.cb3 = c;
     g.ncb3 = (g.nkx + c - 1) / c;
@@ -1463,6 +1502,7 @@ int sb_physical_fields(sb_handle *h, int member, unsigned mask, double *out) {
   Grid gl = g;
   gl.B = 1;
   gl.les = 1;
+  gl.planeq = 0;
   gl.nzf = 10;
   gl.temp = 0;
   Bufs bl = h->bf;

@@ -72,8 +72,9 @@ __global__ void __launch_bounds__(32) k_hsum(Grid g, Bufs bf) {
   for (int pp = lane; pp < nparts; pp += 32)
 #pragma unroll
     for (int q = 0; q < SB_NHIST_Q; q++) v[q] += hp[pp * SB_NHIST_Q + q];
-  // plane stage 2 leaves one triple per (row pair, warp of its block)
-  const int np2 = nzp * (g.t2 / 32);
+  // plane stage 2 leaves one triple per (row pair, warp of its block), in
+  // fixed point one per row pair
+  const int np2 = g.planeq ? nzp : nzp * (g.t2 / 32);
   const double *ph = bf.ppart + ((long)b * g.my + j) * np2 * 3;
   for (int z = lane; z < np2; z += 32)
 #pragma unroll

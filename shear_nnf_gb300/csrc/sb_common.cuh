@@ -99,6 +99,8 @@ struct Grid {
   // t = 0, that of d/dy over sin t and both denominators at t = pi (the sums
   // that cancel there, taken in extended precision)
   int bloch;
+  // plane stages in fixed point (sb_planeq.cu): FP64 handles without LES
+  int planeq;
   double bpr1[3], bn20, bn1p, bp1p, bp2p;
 };
 
@@ -187,6 +189,12 @@ struct Bufs {
   // Bloch-wave form S and T (its blocks write v and d(omega_y)/dy to G and D
   // while others still read these)
   double *Gn, *Dn;
+  // fixed-point plane stages (sb_planeq.cu): exponents of the columns of zbuf
+  // [B][my][nzf][nkx] and of the row pairs of xbuf [B][my][mgalz/2][nxf]; twiddles
+  // of the z transforms W^t and of the x transforms, W^(n2 k1) at k1 R2 + n2 and
+  // W^(k1 m) at m R1 + k1 (mgalx = R1 R2)
+  int *ze, *xe;
+  const qw *fz, *fxa, *fxb;
 };
 
 // Asynchronous global -> shared copy of one element of NB bytes (4, 8 or 16,

@@ -1584,6 +1584,11 @@ cudaError_t spectra_f32(const Grid &g, const Bufs &bf, cudaStream_t st) {
 #else
 // stage 1..3: launch; stage 0: set the kernels' shared-memory limits (once)
 cudaError_t launch_plane(const Grid &g, const Bufs &bf, int stage, int rk, cudaStream_t st) {
+  if (g.planeq) {
+    const cudaError_t e = launch_planeq(g, bf, stage, rk, st);
+    // the FP64 kernels still serve the physical fields
+    if (stage != 0 || e != cudaSuccess) return e;
+  }
   return g.prec ? plane_f32(g, bf, stage, rk, st) : launch_plane_t<double>(g, bf, stage, rk, st);
 }
 cudaError_t launch_les(const Grid &g, const Bufs &bf, int stage, int rk, cudaStream_t st) {

@@ -12,6 +12,8 @@ int plane_t2_default(int mgalx);
 bool plane3_fits(const Grid &g, int cb);
 bool supported_grid(int mgalx, int mgalz);
 cudaError_t launch_plane(const Grid &g, const Bufs &bf, int stage, int rk, cudaStream_t st);
+// the same in fixed point, where Grid::planeq
+cudaError_t launch_planeq(const Grid &g, const Bufs &bf, int stage, int rk, cudaStream_t st);
 int les_cb(int mgalz);
 cudaError_t launch_les(const Grid &g, const Bufs &bf, int stage, int rk, cudaStream_t st);
 cudaError_t launch_lineL(const Grid &g, const Bufs &bf, cudaStream_t st);
