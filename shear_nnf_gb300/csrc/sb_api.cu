@@ -417,6 +417,16 @@ static int build_bloch_tables(sb_handle *h) {
   double *q;
   if ((rc = dalloc(h, &q, 2 * m))) return rc;
   bf.btw = (qw *)q;
+  if ((rc = dalloc(h, &q, 2 * (size_t)g.B * g.field))) return rc;
+  bf.bw = (q2 *)q;
+  if ((rc = dalloc(h, &q, 4 * (size_t)g.B * n))) return rc;
+  bf.bwm = (q2 *)q;
+  if ((rc = dalloc(h, &q, (size_t)g.B * (g.plane / 2 + 2)))) return rc;
+  bf.bwp = (int *)q;
+  if ((rc = dalloc(h, &q, 2 * (m / 3)))) return rc;
+  bf.bm1 = (double2 *)q;
+  if ((rc = dalloc(h, &q, 2 * (m / 3)))) return rc;
+  bf.bm2 = (double2 *)q;
   if ((rc = dalloc(h, &bf.bl1, m)) || (rc = dalloc(h, &bf.bl2, m)) ||
       (rc = upload_fix(h, &bf.bftw, n, -1, false)) || (rc = upload_fix(h, &bf.bitw, n, 1, true)) ||
       (rc = upload_fix(h, &bf.bturn, 1024, -1, false)))
@@ -450,6 +460,14 @@ static void member_defaults(const sb_params *p, const Grid &g, double Re, Member
   m->keep_laminar = p->keep_laminar;
   // thermal diffusion CFL (initcr.f90:498-502)
   m->cflkk = p->temperature ? p->fkappa / p->CFL * mm : 0.0;
+}
+
+// the phase tables of substep rk (0: the start of a run): the Bloch-wave
+// form's, and the banded solves' where they run (with LES k_lineL does)
+static cudaError_t launch_phases(sb_handle *h, int rk, cudaStream_t st) {
+  if (!h->step_bloch) return launch_tables(h->g, h->bf, rk, st);
+  const cudaError_t e = h->g.les ? launch_tables(h->g, h->bf, rk, st) : cudaSuccess;
+  return e != cudaSuccess ? e : launch_bloch(h->g, h->bf, rk, st);
 }
 
 static int capture_step(sb_handle *h) {
@@ -491,8 +509,7 @@ static int capture_step(sb_handle *h) {
       if ((e = cudaEventRecord(h->ev_fork, h->st)) != cudaSuccess ||
           (e = cudaStreamWaitEvent(h->side, h->ev_fork, 0)) != cudaSuccess ||
           (e = launch_scalar(h->g, h->bf, rk, h->side)) != cudaSuccess ||
-          (e = launch_tables(h->g, h->bf, rk, h->side)) != cudaSuccess ||
-          (h->step_bloch && (e = launch_bloch(h->g, h->bf, rk, h->side)) != cudaSuccess) ||
+          (e = launch_phases(h, rk, h->side)) != cudaSuccess ||
           (h->g.impl && (e = launch_hfac(h->g, h->bf, rk, h->side)) != cudaSuccess) ||
           (e = cudaEventRecord(h->ev_join, h->side)) != cudaSuccess ||
           (e = launch_plane(h->g, h->bf, 3, rk, h->st)) != cudaSuccess ||
@@ -504,8 +521,7 @@ static int capture_step(sb_handle *h) {
       if ((e = launch_plane(h->g, h->bf, 3, rk, h->st)) != cudaSuccess) break;
       if (h->g.les && (e = launch_les(h->g, h->bf, 5, rk, h->st)) != cudaSuccess) break;
       if ((e = launch_scalar(h->g, h->bf, rk, h->st)) != cudaSuccess) break;
-      if ((e = launch_tables(h->g, h->bf, rk, h->st)) != cudaSuccess) break;
-      if (h->step_bloch && (e = launch_bloch(h->g, h->bf, rk, h->st)) != cudaSuccess) break;
+      if ((e = launch_phases(h, rk, h->st)) != cudaSuccess) break;
       if (h->g.impl && (e = launch_hfac(h->g, h->bf, rk, h->st)) != cudaSuccess) break;
     }
     if (h->g.les && (e = launch_lineL(h->g, h->bf, h->st)) != cudaSuccess) break;
@@ -534,11 +550,9 @@ static int capture_step(sb_handle *h) {
 }
 
 // v from phi and the first derivatives of the state at the start of a run, by
-// the solves of the captured step (the phase tables of slot 0 first)
+// the solves of the captured step
 static cudaError_t launch_prologue(sb_handle *h) {
-  if (!h->step_bloch) return launch_lineB(h->g, h->bf, 0, h->st);
-  cudaError_t e = launch_bloch(h->g, h->bf, 0, h->st);
-  return e != cudaSuccess ? e : launch_lineQ(h->g, h->bf, 0, h->st);
+  return h->step_bloch ? launch_lineQ(h->g, h->bf, 0, h->st) : launch_lineB(h->g, h->bf, 0, h->st);
 }
 
 static int ensure_trace(sb_handle *h, int cap) {
@@ -1124,7 +1138,7 @@ int sb_step(sb_handle *h, int nsteps) {
   // entry of cross(): flags and offsets, phase tables, set_conj on the state,
   // v from phi and the first derivatives (cross.f90:76-113,283-287,376-445)
   CK(launch_scalar(h->g, h->bf, 0, h->st));
-  CK(launch_tables(h->g, h->bf, 0, h->st));
+  CK(launch_phases(h, 0, h->st));
   CK(launch_setconj(h->g, h->bf, h->st));
   if (h->g.ydeal == 3) CK(launch_filter(h->g, h->bf, 0, h->st));
   CK(launch_prologue(h));
@@ -1234,7 +1248,7 @@ int sb_launch_stage(sb_handle *h, int stage, int rk, int count) {
     if (stage <= 3)
       e = launch_plane(h->g, h->bf, stage, rk, h->st);
     else if (stage == 4)
-      e = launch_tables(h->g, h->bf, rk, h->st);
+      e = launch_phases(h, rk, h->st);
     else if (stage == 5)
       e = launch_lineA(h->g, h->bf, rk, h->st);
     else if (stage == 6)
@@ -1298,7 +1312,7 @@ struct Snapshot {
 static cudaError_t launch_step_call(sb_handle *h, int nsteps) {
   cudaError_t e;
   if ((e = launch_scalar(h->g, h->bf, 0, h->st)) != cudaSuccess ||
-      (e = launch_tables(h->g, h->bf, 0, h->st)) != cudaSuccess ||
+      (e = launch_phases(h, 0, h->st)) != cudaSuccess ||
       (e = launch_setconj(h->g, h->bf, h->st)) != cudaSuccess ||
       (h->g.ydeal == 3 && (e = launch_filter(h->g, h->bf, 0, h->st)) != cudaSuccess) ||
       (e = launch_prologue(h)) != cudaSuccess)

@@ -83,10 +83,17 @@ template <int N>
 struct LineQ {
   static constexpr int R1 = Plan<N>::R1, R2 = Plan<N>::R2;
   static constexpr int RM = R1 > R2 ? R1 : R2;
-  static constexpr int T = kCols * RM;
+  // threads of a block.  Wide: one item a thread in the widest kernel, the
+  // shortest chain (one 64x32x32 box: 23 us against 37 with 32 threads,
+  // 384x192x192: 755 us against 1223 with 64).  Narrow, for lines up to 96 and
+  // enough blocks to fill the GPU: few idle threads between the barriers
+  // (192x96x96: 90 us with 64 against 101 with 128; 64 boxes of 64x32x32: 180 us
+  // with 32 against 199 with 64)
+  static constexpr int kWide = N == 32 ? 64 : N == 48 ? 96 : 128;
+  static constexpr int kNarrow = N < 64 ? 32 : N <= 96 ? 64 : 128;
   static constexpr int kShiftF = 2 + Plan<N>::shift;  // twist and forward transform
   static constexpr int kBits = Plan<N>::bits + 2;     // the twist divides by 4
-  static constexpr size_t smem = 2 * sizeof(q2) * N * kCols;
+  static constexpr size_t smem = (2 * sizeof(q2) + sizeof(double)) * N * kCols;
 };
 SB_HD constexpr int floor_log2(int n) { return n < 2 ? 0 : 1 + floor_log2(n / 2); }
 
@@ -124,23 +131,20 @@ __device__ __forceinline__ void rows_inverse(q2 *ex, const qw *__restrict__ twis
   }
 }
 
-// registers per thread the kernel is budgeted for: R1, R2 <= 12, and above
-#ifndef SB_LINEQ_REGS
-#define SB_LINEQ_REGS 128
-#endif
-#ifndef SB_LINEQ_REGS16
-#define SB_LINEQ_REGS16 168
-#endif
+// registers per thread the kernel is budgeted for (192x96x96: 90 us at 128, 94 at
+// 104; 384x192x192: 760 us at 168, 966 at 224)
+template <int N>
+struct LineQRegs {
+  static constexpr int n = LineQ<N>::RM > 12 ? 168 : 128;
+};
 // rk1 = 1..3: the substep; 0: the start of a run (v and the first derivatives
 // from the state, cross.f90:408-445).
 // Two passes over the same code (unrolled twice it would not fit in the
 // instruction cache, and each warp runs it only once): pass 0 takes the
 // right-hand side and the update at the phase of time t, pass 1 the outputs at
 // the phase of t + c_k dt.  A pass: rows in, forward, products, inverse, rows out.
-template <typename R, int N>
-__global__ void __launch_bounds__(
-    LineQ<N>::T, 65536 / (LineQ<N>::T * (LineQ<N>::RM > 12 ? SB_LINEQ_REGS16 : SB_LINEQ_REGS)))
-    k_lineQ(Grid g, Bufs bf, int rk1) {
+template <typename R, int N, int T>
+__global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid g, Bufs bf, int rk1) {
   typedef LineQ<N> L;
   typedef typename V2<R>::t V;
   constexpr int R1 = L::R1, R2 = L::R2;
@@ -149,8 +153,9 @@ __global__ void __launch_bounds__(
   const Member &M = bf.mem[b];
   if (M.halted) return;  // uniform per block
   extern __shared__ __align__(16) unsigned char smq_raw[];
-  q2 *const ex = (q2 *)smq_raw;  // two buffers of N x kCols
-  __shared__ unsigned s_top[3][kCols];  // largest upper words: state, D, new state
+  q2 *const ex = (q2 *)smq_raw;              // two buffers of N x kCols
+  double *const sc = (double *)(ex + 2 * N * kCols);  // factors of the waves
+  __shared__ unsigned s_top[2][kCols];  // largest upper words: D, the new state
   __shared__ int s_len[3][kCols];       // scales of the products: right-hand side, first, second output
   const int ncb = (g.nkx + kCols - 1) / kCols, per = g.mz * ncb;
   const int role = blockIdx.x / per;  // 0 phi, 1 omega_y, 2 mean
@@ -166,10 +171,10 @@ __global__ void __launch_bounds__(
   const int nkx = g.nkx;
   const long ps = g.plane / 2;  // complex entries per plane
   const long off = (long)b * (g.field / 2) + (long)k * nkx + i;
-  const bool t1 = n < R2, t2 = n < R1;  // threads of the row and of the wave kernels
   const int rk = rk1 - 1;
+  static_assert(T >= 3 * kCols, "one thread per slot");
   if (threadIdx.x < 3 * kCols) {
-    (&s_top[0][0])[threadIdx.x] = 0u;
+    if (threadIdx.x < 2 * kCols) (&s_top[0][0])[threadIdx.x] = 0u;
     (&s_len[0][0])[threadIdx.x] = kNoLen;
   }
   __syncthreads();
@@ -179,6 +184,11 @@ __global__ void __launch_bounds__(
   const double nu = is00 ? 0.0 : M.nu, nuk2 = nu * k2;
   V *f = (V *)(role == 0 ? bf.phi : bf.vor) + off;
   R *mf = (R *)bf.mu + (long)b * 2 * N + cm;  // mean profile of this column
+  // the waves of the state, kept from pass 1 for the next substep's pass 0 (the
+  // same phase), and their scale
+  const long wst = mean ? 2 : ps, nl = ps + 2;
+  q2 *waves = mean ? bf.bwm + (long)b * 2 * N + cm : bf.bw + role * (g.B * (g.field / 2)) + off;
+  int *wscale = bf.bwp + ((long)role % 2 * g.B + b) * nl + (mean ? ps + cm : (long)k * nkx + i);
 #pragma unroll 1
   for (int ph = rk1 > 0 ? 0 : 1; ph < 2; ph++) {
     // phase tables: slot 0 holds the phases of a step's start, slots 1 and 2
@@ -188,40 +198,46 @@ __global__ void __launch_bounds__(
     const double *l1 = bf.bl1 + o, *l2 = bf.bl2 + o;
     const int nf = ph == 0 && role == 0 ? 2 : 1;  // fields in: the state, D
     const int no = ph == 1 && role == 0 ? 2 : 1;  // fields out
-    // ---- rows in (the new state is in buffer 0 already)
-    if (ph == 0 || rk1 == 0) {
-#pragma unroll 1
-      for (int q = 0; q < nf; q++) {
-        const V *src = q ? (const V *)bf.Dn + off : f;
-        unsigned top = 0;
+    // ---- rows in: D to buffer 1 (phi, pass 0), the state of the start of a run
+    // to buffer 0 (in pass 1 the new state is there already)
+    const bool rows = ph == 1 || role == 0;
+    if (ph == 0 ? role == 0 : rk1 == 0) {
+      const V *src = ph == 0 ? (const V *)bf.Dn + off : f;
+      unsigned top = 0;
 #pragma unroll 4
-        for (int j = n; j < N; j += L::RM) {
-          const V w = mean ? mkv<R>(mf[2 * j], (R)0) : src[(long)j * ps];
-          *(V *)(ex + (q * N + j) * kCols + ci) = w;
-          top = max(top, vtop(w));
-        }
-        atomicMax(&s_top[ph == 0 ? q : 2][ci], top);
+      for (int j = n; j < N; j += T / kCols) {
+        const V w = mean ? mkv<R>(mf[2 * j], (R)0) : src[(long)j * ps];
+        *(V *)(ex + ((1 - ph) * N + j) * kCols + ci) = w;
+        top = max(top, vtop(w));
       }
+      atomicMax(&s_top[ph][ci], top);
     }
-    __syncthreads();
-    const QScale s0 = qscale(s_top[ph == 0 ? 0 : 2][ci], L::kBits);
-    const QScale s1 = qscale(s_top[1][ci], L::kBits);
-    const bool bad = s0.bad || (nf > 1 && s1.bad);
-    if (t1)
+    if (rows) __syncthreads();
+    // scales: 0 the state (pass 0: of the waves kept from the last pass 1), 1 D
+    const QScale sr = qscale(s_top[ph][ci], L::kBits);
+    const int kept = ph == 0 ? *wscale : 0;
+    const int w0 = ph == 0 ? kept : sr.weight(), w1 = sr.weight();
+    const bool bad = (ph == 0 && kept == kNoLen) || (rows && sr.bad);
+    if (rows) {
 #pragma unroll 1
-      for (int q = 0; q < nf; q++)
-        rows_forward<N, V>(ex + q * N * kCols, q ? s1 : s0, here(tw), nkx, here(bf.bftw), n, ci);
-    __syncthreads();
+      for (int it = n; it < R2; it += T / kCols)
+        rows_forward<N, V>(ex + (1 - ph) * N * kCols, sr, tw, nkx, bf.bftw, it, ci);
+      __syncthreads();
+    }
     // ---- products.  Pass 0: nu (l2 - k^2) f - i l1 D; pass 1: phi f/(l2 - k^2)
     // and i l1 of it, else i l1 f.  The waves stay in the thread's own slots
     // while the scale of each product is found over the whole line.
-    double c[R2];  // nu (l2 - k^2), 1/(l2 - k^2) or l1
-    if (t2) {
+#pragma unroll 1
+    for (int k1 = n; k1 < R1; k1 += T / kCols) {
+      const long p0 = (long)k1 * nkx;
+      double *cw = sc + k1 * R2 * kCols + ci;
+      // nu (l2 - k^2), 1/(l2 - k^2) or l1
 #pragma unroll
       for (int q = 0; q < R2; q++) {
-        const long p = (long)(n + R1 * q) * nkx;
+        const long p = p0 + (long)(R1 * q) * nkx;
+        double c;
         if (ph == 0) {
-          c[q] = fma(nu, l2[p], -nuk2);
+          c = fma(nu, l2[p], -nuk2);
         } else if (role == 0) {
           // reciprocal by two Newton steps from the 20-bit estimate
           const double den = l2[p] - k2;
@@ -229,50 +245,65 @@ __global__ void __launch_bounds__(
           asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(z) : "d"(den));
           z = fma(z, fma(-den, z, 1.0), z);
           z = fma(z, fma(-den, z, 1.0), z);
-          c[q] = is00 ? 0.0 : z;
+          c = is00 ? 0.0 : z;
         } else {
-          c[q] = l1[p];
+          c = l1[p];
         }
+        cw[q * kCols] = c;
       }
 #pragma unroll 1
       for (int q = 0; q < nf; q++) {
-        q2 *e = ex + (q * N + n * R2) * kCols + ci;
-        const double *l = here(l1);
+        q2 *e = ex + (q * N + k1 * R2) * kCols + ci;
+        const double *l = here(l1) + p0;
         q2 x[R2];
+        if (ph == 0 && q == 0) {
+          const q2 *wv = waves + k1 * wst;
 #pragma unroll
-        for (int w = 0; w < R2; w++) x[w] = e[w * kCols];
-        Dft<R2, -1>::run(x);
+          for (int w = 0; w < R2; w++) x[w] = wv[(long)(R1 * w) * wst];
+        } else {
+#pragma unroll
+          for (int w = 0; w < R2; w++) x[w] = e[w * kCols];
+          Dft<R2, -1>::run(x);
+        }
+        if (ph == 1 && act) {
+          q2 *wv = waves + k1 * wst;
+#pragma unroll
+          for (int w = 0; w < R2; w++) wv[(long)(R1 * w) * wst] = x[w];
+        }
         int la = kNoLen, lb = kNoLen;
 #pragma unroll
         for (int w = 0; w < R2; w++) {
           e[w * kCols] = x[w];
-          const int len = qlen(x[w]), e1 = qexp(l[(long)(n + R1 * w) * nkx]);
-          la = max(la, len + (q ? e1 : qexp(c[w])));
-          lb = max(lb, len + qexp(c[w]) + e1 + 1);
+          const int len = qlen(x[w]), e1 = qexp(l[(long)(R1 * w) * nkx]), ec = qexp(cw[w * kCols]);
+          la = max(la, len + (q ? e1 : ec));
+          lb = max(lb, len + ec + e1 + 1);
         }
-        atomicMax(&s_len[ph][ci], la - (ph == 0 ? (q ? s1.p : s0.p) : 0));
+        atomicMax(&s_len[ph][ci], la - (ph == 0 ? (q ? w1 : w0) : 0));
         if (no > 1) atomicMax(&s_len[2][ci], lb);
       }
+      if (ph == 1 && k1 == 0 && act) *wscale = bad ? kNoLen : w0;
     }
     __syncthreads();
     // scales of the outputs; in pass 0 of the sum of two terms
     const int len1 = s_len[ph][ci] + (ph == 0 ? 2 : 1), len2 = s_len[2][ci] + 1;
-    if (t2) {
+#pragma unroll 1
+    for (int k1 = n; k1 < R1; k1 += T / kCols) {
+      const double *cw = sc + k1 * R2 * kCols + ci;
       q2 y[R2];
 #pragma unroll 1
       for (int q = max(nf, no) - 1; q >= 0; q--) {
         // pass 0: q = 1 D, 0 f, added; pass 1: q = 1 the second output, 0 the first
-        const q2 *e = ex + ((nf > 1 ? q : 0) * N + n * R2) * kCols + ci;
+        const q2 *e = ex + ((nf > 1 ? q : 0) * N + k1 * R2) * kCols + ci;
         const bool first = no > 1 || q == nf - 1;
-        const double *l = here(l1);
+        const double *l = here(l1) + (long)k1 * nkx;
         const qw *it = here(bf.bitw);
-        const int sh = kTgt - (no > 1 && q ? len2 : len1) - (ph == 0 ? (q ? s1.p : s0.p) : 0);
+        const int sh = kTgt - (no > 1 && q ? len2 : len1) - (ph == 0 ? (q ? w1 : w0) : 0);
 #pragma unroll
         for (int w = 0; w < R2; w++) {
-          double d = c[w];
+          double d = cw[w * kCols];
           if (q) {
-            d = l[(long)(n + R1 * w) * nkx];
-            if (ph == 1) d *= c[w];
+            const double m = l[(long)(R1 * w) * nkx];
+            d = ph == 1 ? d * m : m;
           }
           q2 z = qscaled(e[w * kCols], d, sh);
           // times -i (D), i (d/dy of an output) or 1
@@ -281,28 +312,31 @@ __global__ void __launch_bounds__(
         }
         if (no > 1 || q == 0) {
           Dft<R2, 1>::run(y);
-          q2 *eo = ex + ((no > 1 ? q : 0) * N + n * R2) * kCols + ci;
+          q2 *eo = ex + ((no > 1 ? q : 0) * N + k1 * R2) * kCols + ci;
 #pragma unroll
-          for (int w = 0; w < R2; w++) eo[w * kCols] = qmul<false>(y[w], it[w * n]);
+          for (int w = 0; w < R2; w++) eo[w * kCols] = qmul<false>(y[w], it[w * k1]);
         }
       }
     }
     __syncthreads();
-    if (t1)
 #pragma unroll 1
-      for (int q = 0; q < no; q++) rows_inverse<N>(ex + q * N * kCols, here(tw), nkx, n, ci);
+    for (int it = n; it < no * R2; it += T / kCols) {
+      const int q = it >= R2;
+      rows_inverse<N>(ex + q * N * kCols, here(tw), nkx, it - q * R2, ci);
+    }
     __syncthreads();
     // ---- rows out
     const int eb = L::kShiftF + Plan<N>::shift + 2 - kN - kTgt;
     if (ph == 1) {
-      const int e0 = eb - s0.p;
+      const int e0 = eb - w0;
+      const bool nan1 = bad || qrange(e0 + len1), nan2 = bad || qrange(e0 + len2);
       const R nn = (R)nan("");
       if (mean) {
         R *dst = (R *)bf.mdu + (long)b * 2 * N + cm;
         if (act)
 #pragma unroll 1
-          for (int j = n; j < N; j += L::RM)
-            dst[2 * j] = bad ? nn : qout<R>(ex[j * kCols + ci].x, e0 + len1);
+          for (int j = n; j < N; j += T / kCols)
+            dst[2 * j] = nan1 ? nn : qout<R>(ex[j * kCols + ci].x, e0 + len1);
       } else if (act) {
 #pragma unroll 1
         for (int q = 0; q < no; q++) {
@@ -310,10 +344,11 @@ __global__ void __launch_bounds__(
           if (role == 0 && q == 0 && is00 && rk1 > 0) continue;
           V *dst = (V *)(role != 0 ? bf.D : q ? bf.V : bf.G) + off;
           const int eo = e0 + (q ? len2 : len1);
+          const bool none = q ? nan2 : nan1;
 #pragma unroll 2
-          for (int j = n; j < N; j += L::RM) {
+          for (int j = n; j < N; j += T / kCols) {
             const q2 z = ex[(q * N + j) * kCols + ci];
-            dst[(long)j * ps] = bad ? mkv<R>(nn, nn) : mkv<R>(qout<R>(z.x, eo), qout<R>(z.y, eo));
+            dst[(long)j * ps] = none ? mkv<R>(nn, nn) : mkv<R>(qout<R>(z.x, eo), qout<R>(z.y, eo));
           }
         }
       }
@@ -321,6 +356,7 @@ __global__ void __launch_bounds__(
     }
     // RK3 accumulation and update, zeta store, remaps (cross.f90:694-781)
     const int eo = eb + len1;
+    const bool nanr = bad || qrange(eo);
     const R gk = (R)kGama[rk], zk = (R)kZeta[rk], dtr = (R)M.Deltat;
     unsigned top = 0;
     if (mean) {
@@ -328,7 +364,7 @@ __global__ void __launch_bounds__(
       const R *mrf = (const R *)bf.mrf + (long)b * 2 * N + cm;
       const bool damp = g.damp && ci == 0, xf = g.force == -1 && ci == 0;
 #pragma unroll 1
-      for (int j = n; j < N; j += L::RM) {
+      for (int j = n; j < N; j += T / kCols) {
         R un = (R)0;
         if (act) {
           // forcing and damping (cross.f90:622-626; operators.f90:60-78)
@@ -340,7 +376,7 @@ __global__ void __launch_bounds__(
                                         (1.0 + tanh(6.0 * (g.damp_a + y) / g.lz + 3.0));
             rf0 = (R)((double)rf0 - g.damp_up * hw * (double)mf[2 * j]);
           }
-          const R rf = rf0 + (bad ? (R)nan("") : qout<R>(ex[j * kCols + ci].x, eo));
+          const R rf = rf0 + (nanr ? (R)nan("") : qout<R>(ex[j * kCols + ci].x, eo));
           R wk = (rk == 0) ? gk * rf : mwk[2 * j] + gk * rf;
           un = mf[2 * j] + dtr * wk;
           if (rk < 2) wk = rf * zk;
@@ -354,24 +390,24 @@ __global__ void __launch_bounds__(
     } else {
       const V *rhs = (const V *)(role == 0 ? bf.V : bf.Gn) + off;
       V *fwk = (V *)(role == 0 ? bf.phiwk : bf.vorwk) + off;
-      const double2 *m1 = (const double2 *)bf.mf1 + (long)b * tb + i;
-      const double2 *m2 = (const double2 *)bf.mf2 + (long)b * tb + i;
+      const double2 *m1 = bf.bm1 + (long)b * tb + i, *m2 = bf.bm2 + (long)b * tb + i;
       const V none = mkv<R>((R)0, (R)0);
 #pragma unroll 2
-      for (int j = n; j < N; j += L::RM) {
+      for (int j = n; j < N; j += T / kCols) {
         const long q = (long)j * ps;
         const V fo = f[q], rh = rhs[q], w0 = rk > 0 ? fwk[q] : none;
         const q2 z = ex[j * kCols + ci];
         V h = mkv<R>(rh.x + qout<R>(z.x, eo), rh.y + qout<R>(z.y, eo));
-        if (bad) h = mkv<R>((R)nan(""), (R)nan(""));
+        if (nanr) h = mkv<R>((R)nan(""), (R)nan(""));
         V wk = mkv<R>(w0.x + gk * h.x, w0.y + gk * h.y);
-        const double fx = (double)(fo.x + dtr * wk.x), fy = (double)(fo.y + dtr * wk.y);
         const double2 p2 = m2[(long)j * nkx];
+        const double fx = (double)(fo.x + dtr * wk.x), fy = (double)(fo.y + dtr * wk.y);
         const V fn = mkv<R>((R)fma(fx, p2.x, -(fy * p2.y)), (R)fma(fy, p2.x, fx * p2.y));
         if (rk < 2) {
+          // zeta_k h in the frame of the next substep; zeta_k is in the phase
           const double2 p1 = m1[(long)j * nkx];
-          const double zx = (double)(h.x * zk), zy = (double)(h.y * zk);
-          wk = mkv<R>((R)fma(zx, p1.x, -(zy * p1.y)), (R)fma(zy, p1.x, zx * p1.y));
+          const double hx = (double)h.x, hy = (double)h.y;
+          wk = mkv<R>((R)fma(hx, p1.x, -(hy * p1.y)), (R)fma(hy, p1.x, hx * p1.y));
         }
         if (act) {
           f[q] = fn;
@@ -381,23 +417,37 @@ __global__ void __launch_bounds__(
         *(V *)(ex + j * kCols + ci) = fn;
       }
     }
-    atomicMax(&s_top[2][ci], top);
+    atomicMax(&s_top[1][ci], top);
   }
 }
 
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-template <typename R, int N>
-static cudaError_t launch_t(const Grid &g, const Bufs &bf, int rk, cudaStream_t st, bool prep) {
+template <typename R, int N, int T>
+static cudaError_t launch_n(const Grid &g, const Bufs &bf, int rk, cudaStream_t st, bool prep,
+                            unsigned blocks) {
   if (prep)
-    return cudaFuncSetAttribute(k_lineQ<R, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(k_lineQ<R, N, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)LineQ<N>::smem);
-  const int ncb = (g.nkx + kCols - 1) / kCols;
-  k_lineQ<R, N><<<dim3((unsigned)(2 * g.mz * ncb + 1), (unsigned)g.B), LineQ<N>::T, LineQ<N>::smem,
-                  st>>>(g, bf, rk);
+  k_lineQ<R, N, T><<<dim3(blocks, (unsigned)g.B), T, LineQ<N>::smem, st>>>(g, bf, rk);
   return cudaGetLastError();
 }
+template <typename R, int N>
+static cudaError_t launch_t(const Grid &g, const Bufs &bf, int rk, cudaStream_t st, bool prep) {
+  constexpr int W = LineQ<N>::kWide, S = LineQ<N>::kNarrow;
+  const unsigned blocks = (unsigned)(2 * g.mz * ((g.nkx + kCols - 1) / kCols) + 1);
+  if constexpr (W != S) {
+    if (prep) {
+      const cudaError_t e = launch_n<R, N, S>(g, bf, rk, st, true, blocks);
+      if (e != cudaSuccess) return e;
+    } else if ((long)blocks * g.B >= 5 * 152) {
+      return launch_n<R, N, S>(g, bf, rk, st, false, blocks);
+    }
+  }
+  return launch_n<R, N, W>(g, bf, rk, st, prep, blocks);
+}
+
 #if SB_FLOAT_TU
 typedef float UnitR;
 #else
@@ -454,6 +504,22 @@ __global__ void __launch_bounds__(64) k_bloch(Grid g, Bufs bf, int rk) {
     turn = a * kInv;
   }
   const ll X = __double2ll_rn(turn * 18446744073709551616.0);
+  if (rk > 0) {
+    // moving-frame phases exp(i kx y_j tau) (operators.f90:119-123), the work
+    // array's with zeta_k (cross.f90:752-781)
+    const double Dt = M.Deltat, ay = (g.alp * i) * ((double)m * g.dy - 0.5 * g.Ly);
+    const double f1 = (rk == 1) ? -(kGama[0] * Dt * g.s) : -((kGama[1] + kZeta[0]) * Dt * g.s);
+    const double f2 = (rk == 1) ? -(g.s * (kCa[0] * Dt)) : -(g.s * (kCa[rk - 1] - kCa[rk - 2]) * Dt);
+    auto phase = [&](double f, double z) {
+      const double t = ay * f * kInv;
+      const qw w = qturn(__double2ll_rn((rint(t) - t) * 18446744073709551616.0), 1, 1, bf.bturn);
+      return make_double2(z * fromfix((ll)((ull)(ll)w.hr << 32) + w.lr, -62),
+                          z * fromfix((ll)((ull)(ll)w.hi << 32) + w.li, -62));
+    };
+    const long q = (long)b * N * nkx + p;
+    bf.bm2[q] = phase(f2, 1.0);
+    if (rk < 3) bf.bm1[q] = phase(f1, kZeta[rk - 1]);
+  }
   const long o = ((long)sn * g.B + b) * N * nkx + p;
   bf.btw[o] = qturn(X, m, N, bf.bturn);
   // t/2 = pi (turn + ms)/N for |t| <= pi/2, else pi/2 less the rest

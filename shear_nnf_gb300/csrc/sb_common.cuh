@@ -20,6 +20,7 @@
 namespace sb {
 
 struct qw;  // fixed-point constant (sb_fix.cuh)
+struct q2;  // fixed-point complex number
 
 struct cd {
   double x, y;
@@ -181,8 +182,15 @@ struct Bufs {
   // Bloch-wave tables (sb_bloch.cu), three phase slots each [3][B][my][nkx]:
   // twist, l1, l2; transform twiddles of my points, forward and inverse (the
   // inverse ones times 2^floor(log2 my)/my), and e^{-2 pi i t/1024}
+  // moving-frame phases of the substep [B][my][nkx], zeta_k exp(i kx y tau) of
+  // the work array and exp(i kx y tau) of the state
   qw *btw;
+  double2 *bm1, *bm2;
   double *bl1, *bl2;
+  // waves of phi and omega_y at the end of a substep [2][B][my][mz][nkx], those
+  // of the mean profiles [B][my][2] and the scales of all [2][B][mz nkx + 2]
+  q2 *bw, *bwm;
+  int *bwp;
   const qw *bftw, *bitw, *bturn;
   // nonlinear right-hand sides of the omega_y equation and of the d/dy term
   // of the phi equation, as plane stage 3 leaves them: G and D, or with the

@@ -346,43 +346,42 @@ SB_HD unsigned hiword(float f) {
   return u < 0x00800000u ? 0u : (u >> 3) + (896u << 20);
 }
 // scale of a block: the integers are x 2^p.  Zero blocks and blocks below
-// 2^-958 count as zero (their integers are zero); a block with an infinity or
-// a NaN is flagged
+// 2^-958 count as zero (a scale at which every shift empties the integer); a
+// block with an infinity or a NaN is flagged
+constexpr int kZeroScale = -4000;
 struct QScale {
   int p;
   bool bad;
-  bool zero;
+  // the scale as an exponent: the integers of a zero block weigh nothing
+  SB_HD int weight() const { return p == kZeroScale ? -kZeroScale : p; }
 };
 // from the largest component alone: |x| 2^p < 2^bits
 SB_HD QScale qscale(unsigned top, int bits) {
   QScale s;
   const int E = (int)(top >> 20);
-  s.p = bits - (E - 1022);
+  s.p = E < 64 ? kZeroScale : bits - (E - 1022);
   s.bad = E == 0x7ff;
-  s.zero = E < 64;
   return s;
 }
-// x 2^p to nearest; |result| <= 2^62 where |x| 2^p <= 2^62
+// x 2^p to nearest; |x| 2^p < 2^62
 SB_HD ll tofix(double d, const QScale &s) {
   const ull u = dbits64(d);
   const int e = (int)((u >> 52) & 0x7ff);
   const ull m = ((u & 0xfffffffffffffull) | 0x10000000000000ull) << 10;
   int sh = 1084 - s.p - e;  // 10 - (p + e - 1075) less the rounding bit
   if (sh > 63) sh = 63;
-  const ll r = (ll)(((m >> sh) + 1) >> 1);
-  const ll g = (ll)u >> 63;
-  return s.zero ? 0 : (r ^ g) - g;
+  const ll r = (ll)(((m >> sh) + 1) >> 1), g = (ll)u >> 63;
+  return (r ^ g) - g;
 }
 SB_HD ll tofix(float f, const QScale &s) {
   const unsigned u = fbits32(f);
   int e = (int)((u >> 23) & 0xff);
   const ull m = (ull)((u & 0x7fffffu) | (e ? 0x800000u : 0u)) << 39;
-  e = e ? e : 1;  // subnormal
+  e = e ? e : 1;            // subnormal
   int sh = 188 - s.p - e;  // 39 - (p + e - 150) less the rounding bit
   if (sh > 63) sh = 63;
-  const ll r = (ll)(((m >> sh) + 1) >> 1);
-  const ll g = -(ll)(u >> 31);
-  return s.zero ? 0 : (r ^ g) - g;
+  const ll r = (ll)(((m >> sh) + 1) >> 1), g = -(ll)(u >> 31);
+  return (r ^ g) - g;
 }
 SB_HD int qclz(ull a) {
 #ifdef __CUDA_ARCH__
@@ -391,31 +390,29 @@ SB_HD int qclz(ull a) {
   return a ? __builtin_clzll(a) : 64;
 #endif
 }
-// v 2^t as a double, rounded to nearest; results below the normal range are
-// zero, above it infinite
+// v 2^t, rounded to nearest (|v| < 2^63).  The exponent t comes from a block's
+// scale: blocks whose results could pass the range of R are flagged by
+// qrange() first, and exponents below it give results of no size (zero for a
+// float, below 2^-900 for a double)
+SB_HD bool qrange(int t) { return t > 900; }
 SB_HD double fromfix(ll v, int t) {
   const ll g = v >> 63;
   ull a = (ull)((v ^ g) - g);
   const int lz = qclz(a);
-  const int E = t + 1085 - lz;  // biased exponent less the implicit one
-  a <<= lz & 63;
-  ull r = (a >> 11) + ((a >> 10) & 1);
-  r += (ull)(ll)E << 52;
-  if (v == 0 || E < 0) r = 0;
-  if (E >= 2046 && v != 0) r = 0x7ff0000000000000ull;
-  return bits64d(r | ((ull)g & 0x8000000000000000ull));
+  a = ((a << ((lz - 1) & 63)) + 0x200) >> 10;  // the leading bit at 52
+  const int E = (t < -1000 ? -1000 : t) + 1085 - lz;  // biased exponent less the implicit one
+  const ull r = a + ((ull)(unsigned)E << 52);
+  return v == 0 ? 0.0 : bits64d(r | ((ull)g & 0x8000000000000000ull));
 }
 SB_HD float fromfixf(ll v, int t) {
   const ll g = v >> 63;
   ull a = (ull)((v ^ g) - g);
   const int lz = qclz(a);
   const int E = t + 63 - lz + 126;
-  a <<= lz & 63;
-  unsigned r = (unsigned)(a >> 40) + ((unsigned)(a >> 39) & 1u);
-  if (v == 0 || E < -24) return bits32f((unsigned)g & 0x80000000u);
-  if (E < 0) return bits32f((r >> -E) | ((unsigned)g & 0x80000000u));  // subnormal
-  if (E >= 254) return bits32f(0x7f800000u | ((unsigned)g & 0x80000000u));
-  r += (unsigned)E << 23;
+  unsigned r = (unsigned)(((a << ((lz - 1) & 63)) + (1ull << 38)) >> 39);  // the leading bit at 23
+  if (v == 0 || E < -24) return 0.0f;
+  if (E >= 254) r = 0x7f800000u;
+  else r = E < 0 ? r >> -E : r + ((unsigned)E << 23);
   return bits32f(r | ((unsigned)g & 0x80000000u));
 }
 template <typename R> SB_HD R qout(ll v, int t);

@@ -43,6 +43,10 @@ __device__ __forceinline__ q2 qshift(q2 x, int s) {
   return mkq((ll)((ull)x.x << l) >> r, (ll)((ull)x.y << l) >> r);
 }
 __device__ __forceinline__ int bitlen(unsigned v) { return 32 - __clz((int)v); }
+// v 2^t, past the range as a large number (its step is stopped as diverged)
+__device__ __forceinline__ double fromfix_big(ll v, int t) {
+  return qrange(t) ? (v == 0 ? 0.0 : v < 0 ? -1e300 : 1e300) : fromfix(v, t);
+}
 // a b / 2^64; |a|, |b| <= 2^62
 __device__ __forceinline__ ll qprod(ll a, ll b) { return qmulr(a, qhi(b), qlo(b)); }
 
@@ -62,12 +66,17 @@ __device__ __forceinline__ bool gap(int n1, int j, int keep) {
 template <int NZ>
 struct Z1 {
   static constexpr int R1 = Plan<NZ>::R1, R2 = Plan<NZ>::R2;
-  static constexpr int T = 128;
+  // threads as the row kernels' items (64 boxes of 64x32x32: 112 us with 64
+  // against 172 with 128; 192 points: 370 us with 128 against 519 and, with 256,
+  // 452), and more warps where the registers allow (96 points: 50.9 us at 85
+  // registers against 55.5 at 128; 192 points 394 against 370)
+  static constexpr int T = NZ < 64 ? 64 : 128;
+  static constexpr int kMinB = NZ <= 96 ? 768 / T : NZ <= 192 ? 4 : 2;
   static constexpr size_t smem = 2 * sizeof(q2) * NZ * kCols;
 };
 
 template <int NZ, bool TEMP>
-__global__ void __launch_bounds__(Z1<NZ>::T, NZ <= 192 ? 4 : 2) k_z1(Grid g, Bufs bf) {
+__global__ void __launch_bounds__(Z1<NZ>::T, Z1<NZ>::kMinB) k_z1(Grid g, Bufs bf) {
   constexpr int R1 = Z1<NZ>::R1, R2 = Z1<NZ>::R2, T = Z1<NZ>::T;
   const int ncb = (g.nkx + kCols - 1) / kCols;
   const int round = blockIdx.x / ncb, cb = blockIdx.x - round * ncb;
@@ -157,10 +166,11 @@ __global__ void __launch_bounds__(Z1<NZ>::T, NZ <= 192 ? 4 : 2) k_z1(Grid g, Buf
   for (int f = 0; f < 2; f++) {
     const QScale s = qscale(s_top[f][ci], Plan<NZ>::bits);
     // sum < s_sum 2^(E - 1043), E the exponent field
-    p[f] = max(s.p, 1105 - (int)(s_top[f][ci] >> 20) - bitlen(s_sum[f][ci]));
+    p[f] = s.p == kZeroScale ? s.p : max(s.p, 1105 - (int)(s_top[f][ci] >> 20) - bitlen(s_sum[f][ci]));
     if (threadIdx.x < kCols && f < nfl && act) {
       const int fz = TEMP && round == g.tround ? g.tzf : 2 * round + f;
-      bf.ze[(((long)b * g.my + j) * g.nzf + fz) * nkx + i] = s.bad ? kBad : Plan<NZ>::shift - p[f];
+      bf.ze[(((long)b * g.my + j) * g.nzf + fz) * nkx + i] =
+          s.bad ? kBad : p[f] == kZeroScale ? kZeroScale : Plan<NZ>::shift - p[f];
     }
   }
 #pragma unroll 1
@@ -169,7 +179,6 @@ __global__ void __launch_bounds__(Z1<NZ>::T, NZ <= 192 ? 4 : 2) k_z1(Grid g, Buf
     q2 *e = ex + f * NZ * kCols + ci;
     QScale s;
     s.p = p[f];
-    s.zero = (s_top[f][ci] >> 20) < 64;
     const double2 *rows = (const double2 *)e;
     q2 v[R1];
 #pragma unroll
@@ -205,19 +214,26 @@ __global__ void __launch_bounds__(Z1<NZ>::T, NZ <= 192 ? 4 : 2) k_z1(Grid g, Buf
 // ---------------------------------------------------------------------------
 // plane stage 2
 // ---------------------------------------------------------------------------
-template <int NX, bool TEMP>
+// NP row pairs of a block: two where the blocks fill the GPU and fit in shared
+// memory, else one (64x32x32 alone: 10.4 us against 14.1; 384x192x192: 802 us
+// against 1065, where two pairs leave two blocks an SM)
+template <int NX, bool TEMP, int NP>
 struct X2 {
   static constexpr int R1 = Plan<NX>::R1, R2 = Plan<NX>::R2;
   static constexpr int NF = TEMP ? 7 : 6, NO = TEMP ? 6 : 3;
   static constexpr int T = R2 == 16 ? 96 : R2 == 8 ? 64 : 32;
+  // registers per thread: the 16-point kernels want 168 (192x96x96: 99.7 us
+  // against 102 at 128 and 105 at 104), the smaller ones more warps (64 boxes
+  // of 64x32x32: 233 us at 104 against 244 and 274)
+  static constexpr int kRegs = R2 == 16 ? 168 : 104;
   static constexpr int BS = R1 * (R2 + 1);
-  static constexpr size_t smem = sizeof(q2) * 2 * NF * BS;
+  static constexpr size_t smem = sizeof(q2) * NP * NF * BS;
 };
 
-template <int NX, bool TEMP>
-__global__ void __launch_bounds__(X2<NX, TEMP>::T, 65536 / (X2<NX, TEMP>::T * (NX <= 256 ? 128 : 168)))
-k_x2(Grid g, Bufs bf, int rk) {
-  typedef X2<NX, TEMP> C;
+template <int NX, bool TEMP, int NP>
+__global__ void __launch_bounds__(X2<NX, TEMP, NP>::T, 65536 / (X2<NX, TEMP, NP>::T * X2<NX, TEMP, NP>::kRegs))
+    k_x2(Grid g, Bufs bf, int rk) {
+  typedef X2<NX, TEMP, NP> C;
   constexpr int R1 = C::R1, R2 = C::R2, NF = C::NF, NO = C::NO, T = C::T, BS = C::BS;
   constexpr int IT = (NX / 3 + 31) / 32, kSh = Plan<NX>::shift, kBits = Plan<NX>::bits;
   const int j = blockIdx.y, b = blockIdx.z;
@@ -225,14 +241,14 @@ k_x2(Grid g, Bufs bf, int rk) {
   if (M.halted) return;
   extern __shared__ __align__(16) unsigned char smx_raw[];
   q2 *ex = (q2 *)smx_raw;
-  __shared__ int s_e[2 * NF], s_len[2 * NF], s_ho[2 * NO], s_hl[2 * NO];
-  __shared__ ll s_third[2][3];
-  const int nkx = g.nkx, NZ = g.mgalz, z0 = 4 * blockIdx.x;
+  __shared__ int s_e[NP * NF], s_len[NP * NF], s_ho[NP * NO], s_hl[NP * NO];
+  __shared__ ll s_third[NP][3];
+  const int nkx = g.nkx, NZ = g.mgalz, z0 = 2 * NP * blockIdx.x;
   const int lane = threadIdx.x & 31;
   auto P = [](int x) { return x + x / R2; };
-  if (threadIdx.x < 2 * NF) s_len[threadIdx.x] = kNoLen;
-  if (threadIdx.x < 2 * NO) s_hl[threadIdx.x] = kNoLen;
-  if (threadIdx.x < 6) (&s_third[0][0])[threadIdx.x] = 0;
+  if (threadIdx.x < NP * NF) s_len[threadIdx.x] = kNoLen;
+  if (threadIdx.x < NP * NO) s_hl[threadIdx.x] = kNoLen;
+  if (threadIdx.x < 3 * NP) (&s_third[0][0])[threadIdx.x] = 0;
   // ---- rows in: one warp per sequence.  Two rows in one complex sequence
   // (Hermitian extension; FFTW's c2r ignores the imaginary part of kx = 0)
   {
@@ -240,7 +256,7 @@ k_x2(Grid g, Bufs bf, int rk) {
     const q2 *zb = (const q2 *)bf.zbuf + pj * NZ * g.nzf * nkx;
     const int *ze = bf.ze + pj * g.nzf * nkx;
 #pragma unroll 1
-    for (int s = threadIdx.x >> 5; s < 2 * NF; s += T / 32) {
+    for (int s = threadIdx.x >> 5; s < NP * NF; s += T / 32) {
       const int p = s / NF, f = s - p * NF, zf = f < 6 ? f : g.tzf, z = z0 + 2 * p;
       q2 X1[IT], X2[IT];
       int e[IT], len = kNoLen, emax = kNoLen;
@@ -290,7 +306,7 @@ k_x2(Grid g, Bufs bf, int rk) {
   __syncthreads();
   // ---- backward transforms, to the order x = k1 + R1 k2 at slot (k1, k2)
 #pragma unroll 1
-  for (int it = threadIdx.x; it < 2 * NF * R2; it += T) {
+  for (int it = threadIdx.x; it < NP * NF * R2; it += T) {
     const int s = it / R2, n2 = it - s * R2;
     q2 *x = ex + s * BS + n2;
     q2 v[R1];
@@ -304,7 +320,7 @@ k_x2(Grid g, Bufs bf, int rk) {
   }
   __syncthreads();
 #pragma unroll 1
-  for (int it = threadIdx.x; it < 2 * NF * R1; it += T) {
+  for (int it = threadIdx.x; it < NP * NF * R1; it += T) {
     const int s = it / R1, k1 = it - s * R1;
     q2 *x = ex + s * BS + k1 * (R2 + 1);
     q2 v[R2];
@@ -327,7 +343,7 @@ k_x2(Grid g, Bufs bf, int rk) {
   const double sy = g.s * ((double)j * g.dy - 0.5 * g.Ly);
   double m0 = 0.0, m1 = 0.0, m2 = 0.0, m3 = 0.0, mt = 0.0;
 #pragma unroll 1
-  for (int p = 0; p < 2; p++) {
+  for (int p = 0; p < NP; p++) {
     int sh[NF], e[NF];
     bool bad = false;
 #pragma unroll
@@ -436,12 +452,12 @@ k_x2(Grid g, Bufs bf, int rk) {
       }
     }
     if (rk == 1 && !bad && umx >= umn) {
-      const double hi = fromfix(umx, e[0]), lo = fromfix(umn, e[0]);
+      const double hi = fromfix_big(umx, e[0]), lo = fromfix_big(umn, e[0]);
       m0 = fmax(m0, fmax(fabs(hi), fabs(lo)));
       m1 = fmax(m1, fmax(fabs(hi + sy), fabs(lo + sy)));
-      m2 = fmax(m2, fromfix(vm, e[4]));
-      m3 = fmax(m3, fromfix(wm, e[1]));
-      if (TEMP) mt = fmax(mt, fromfix(tm, e[NF - 1]));
+      m2 = fmax(m2, fromfix_big(vm, e[4]));
+      m3 = fmax(m3, fromfix_big(wm, e[1]));
+      if (TEMP) mt = fmax(mt, fromfix_big(tm, e[NF - 1]));
     }
     if (hist) {
       atomicAdd((ull *)&s_third[p][0], (ull)t1);
@@ -458,7 +474,7 @@ k_x2(Grid g, Bufs bf, int rk) {
     }
   }
   __syncthreads();
-  if (hist && threadIdx.x < 6) {
+  if (hist && threadIdx.x < 3 * NP) {
     // one triple per (plane, row pair); k_hsum adds the pairs
     const int p = threadIdx.x / 3, q = threadIdx.x - 3 * p;
     auto ef = [&](int f) { return s_e[p * NF + f] - (61 - s_len[p * NF + f]); };
@@ -466,11 +482,11 @@ k_x2(Grid g, Bufs bf, int rk) {
     for (int f = 0; f < NF; f++) bad |= s_e[p * NF + f] >= kBad;
     const int e2 = q == 0 ? ef(0) : q == 1 ? ef(1) : ef(4);
     bf.ppart[(((long)b * g.my + j) * (NZ / 2) + z0 / 2 + p) * 3 + q] =
-        bad ? nan("") : fromfix(s_third[p][q], ef(4) + 2 * e2 + 128 + 6);
+        bad ? nan("") : fromfix_big(s_third[p][q], ef(4) + 2 * e2 + 128 + 6);
   }
   // ---- forward transforms, to natural order
 #pragma unroll 1
-  for (int it = threadIdx.x; it < 2 * NO * R1; it += T) {
+  for (int it = threadIdx.x; it < NP * NO * R1; it += T) {
     const int s = it / R1, k1 = it - s * R1, p = s / NO, o = s - p * NO;
     q2 *x = ex + (p * NF + o) * BS + k1 * (R2 + 1);
     const int sh = kBits - s_hl[s];
@@ -484,7 +500,7 @@ k_x2(Grid g, Bufs bf, int rk) {
   }
   __syncthreads();
 #pragma unroll 1
-  for (int it = threadIdx.x; it < 2 * NO * R2; it += T) {
+  for (int it = threadIdx.x; it < NP * NO * R2; it += T) {
     const int s = it / R2, m = it - s * R2, p = s / NO, o = s - p * NO;
     q2 *x = ex + (p * NF + o) * BS + m;
     q2 v[R1];
@@ -498,13 +514,13 @@ k_x2(Grid g, Bufs bf, int rk) {
   // ---- the two rows' spectra, (Z_k + conj Z_-k)/2 and -i (Z_k - conj Z_-k)/2
   const long pj = (long)b * g.my + j;
   q2 *xb = (q2 *)bf.xbuf + pj * NZ * NO * nkx;
-  if (threadIdx.x < 2 * NO) {
+  if (threadIdx.x < NP * NO) {
     const int p = threadIdx.x / NO, o = threadIdx.x - p * NO;
     bf.xe[(pj * (NZ / 2) + z0 / 2 + p) * NO + o] =
         s_ho[threadIdx.x] >= kBad ? kBad : s_ho[threadIdx.x] - (kBits - s_hl[threadIdx.x]) + kSh;
   }
 #pragma unroll 1
-  for (int s = threadIdx.x >> 5; s < 2 * NO; s += T / 32) {
+  for (int s = threadIdx.x >> 5; s < NP * NO; s += T / 32) {
     const int p = s / NO, o = s - p * NO, z = z0 + 2 * p;
     const q2 *x = ex + (p * NF + o) * BS;
     for (int i = lane; i < nkx; i += 32) {
@@ -521,12 +537,14 @@ k_x2(Grid g, Bufs bf, int rk) {
 template <int NZ, bool TEMP>
 struct Z3 {
   static constexpr int R1 = Plan<NZ>::R1, R2 = Plan<NZ>::R2;
-  static constexpr int NO = TEMP ? 6 : 3, T = 128;
+  static constexpr int NO = TEMP ? 6 : 3;
+  static constexpr int T = NZ < 64 ? 64 : 128;
+  static constexpr int kMinB = NZ < 64 ? 12 : NZ <= 96 ? 5 : NZ <= 256 ? 4 : 2;  // as Z1
   static constexpr size_t smem = sizeof(q2) * NO * NZ * kCols;
 };
 
 template <int NZ, bool TEMP>
-__global__ void __launch_bounds__(128, NZ <= 256 ? 4 : 2) k_z3(Grid g, Bufs bf) {
+__global__ void __launch_bounds__(Z3<NZ, TEMP>::T, Z3<NZ, TEMP>::kMinB) k_z3(Grid g, Bufs bf) {
   typedef Z3<NZ, TEMP> C;
   constexpr int R1 = C::R1, R2 = C::R2, NO = C::NO, T = C::T;
   const int j = blockIdx.y, b = blockIdx.z;
@@ -599,6 +617,9 @@ __global__ void __launch_bounds__(128, NZ <= 256 ? 4 : 2) k_z3(Grid g, Bufs bf) 
   int eo[NO];
 #pragma unroll
   for (int o = 0; o < NO; o++) eo[o] = Plan<NZ>::shift - (Plan<NZ>::bits - s_len[o][ci]);
+  bool bad = s_bad != 0;
+#pragma unroll
+  for (int o = 0; o < NO; o++) bad |= qrange(eo[o]);
   // streamwise-roll force of this plane on hv(kx=0, kz=1) (operators.f90:14-37)
   const bool force = g.force > 0;
   double fj = 0.0;
@@ -617,7 +638,7 @@ __global__ void __launch_bounds__(128, NZ <= 256 ? 4 : 2) k_z3(Grid g, Bufs bf) 
     };
     double2 H1 = get(0), H2 = get(1), H3 = get(2);
     const double nn = nan("");
-    if (s_bad) H1 = H2 = H3 = make_double2(nn, nn);
+    if (bad) H1 = H2 = H3 = make_double2(nn, nn);
     const double gz = g.gam * ((k <= nz) ? k : k - mz), gn = gz * norm;
     const long q = (long)k * nkx + i;
     const double2 v = Gv[q];
@@ -625,7 +646,7 @@ __global__ void __launch_bounds__(128, NZ <= 256 ? 4 : 2) k_z3(Grid g, Bufs bf) 
       // ht = -i a uT - i gz wT - bym v with the input v, and -vT
       // (crosst.f90:1148-1152,1691-1692)
       double2 uT = get(NO - 3), wT = get(NO - 2), vT = get(NO - 1);
-      if (s_bad) uT = wT = vT = make_double2(nn, nn);
+      if (bad) uT = wT = vT = make_double2(nn, nn);
       ((double2 *)bf.Ht + pb)[q] = make_double2(fma(-g.bym, v.x, fma(an, uT.y, gn * wT.y)),
                                                 fma(-g.bym, v.y, -fma(an, uT.x, gn * wT.x)));
       ((double2 *)bf.R2 + pb)[q] = make_double2(-(norm * vT.x), -(norm * vT.y));
@@ -667,13 +688,28 @@ static cudaError_t launch_zt(const Grid &g, const Bufs &bf, int stage, cudaStrea
     k_z3<NZ, TEMP><<<dim3(ncb, (unsigned)g.my, (unsigned)g.B), Z3<NZ, TEMP>::T, Z3<NZ, TEMP>::smem, st>>>(g, bf);
   return cudaGetLastError();
 }
+template <int NX, bool TEMP, int NP>
+static cudaError_t launch_xn(const Grid &g, const Bufs &bf, int stage, int rk, cudaStream_t st) {
+  typedef X2<NX, TEMP, NP> C;
+  if (stage == 0)
+    return cudaFuncSetAttribute(k_x2<NX, TEMP, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)C::smem);
+  k_x2<NX, TEMP, NP><<<dim3((unsigned)(g.mgalz / (2 * NP)), (unsigned)g.my, (unsigned)g.B), C::T,
+                       C::smem, st>>>(g, bf, rk);
+  return cudaGetLastError();
+}
 template <int NX, bool TEMP>
 static cudaError_t launch_xt(const Grid &g, const Bufs &bf, int stage, int rk, cudaStream_t st) {
-  typedef X2<NX, TEMP> C;
-  if (stage == 0)
-    return cudaFuncSetAttribute(k_x2<NX, TEMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem);
-  k_x2<NX, TEMP><<<dim3((unsigned)(g.mgalz / 4), (unsigned)g.my, (unsigned)g.B), C::T, C::smem, st>>>(g, bf, rk);
-  return cudaGetLastError();
+  if constexpr (NX < 320) {
+    const long blocks = (long)(g.mgalz / 4) * g.my * g.B;
+    if (stage == 0) {
+      const cudaError_t e = launch_xn<NX, TEMP, 2>(g, bf, 0, rk, st);
+      if (e != cudaSuccess) return e;
+    } else if (blocks >= 5 * 152) {
+      return launch_xn<NX, TEMP, 2>(g, bf, stage, rk, st);
+    }
+  }
+  return launch_xn<NX, TEMP, 1>(g, bf, stage, rk, st);
 }
 template <bool TEMP>
 static cudaError_t launch_z(const Grid &g, const Bufs &bf, int stage, cudaStream_t st) {
