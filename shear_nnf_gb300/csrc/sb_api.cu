@@ -78,6 +78,13 @@ struct sb_handle {
   // replace them
   std::vector<void *> line_allocs;
   std::vector<void *> *alloc_to = nullptr;
+  // small arrays of the handle come from chunks (an allocation and its
+  // zeroing cost some 25 us each, and a handle has about a hundred)
+  char *chunk = nullptr;
+  size_t chunk_used = 0, chunk_size = 0;
+  // the per-line Helmholtz tables of the banded solves are built: handles
+  // on Bloch waves build them when a banded solve is first asked for
+  bool banded = false;
   double *d_pen = nullptr;  // staging buffers, one pencil-layout field each
   double *d_pen2 = nullptr;
   // pinned host staging of the small per-call values (mean profiles, time and
@@ -97,13 +104,26 @@ int handle_batch(const sb_handle *h) { return h->g.B; }
 int handle_trace_len(const sb_handle *h) { return h->g.tlen; }
 }  // namespace sb
 
+static int dmalloc(sb_handle *h, void **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) return fail(4, "cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
+  cudaMemset(*p, 0, bytes);
+  (h->alloc_to ? *h->alloc_to : h->allocs).push_back(*p);
+  return 0;
+}
+// n zeroed doubles, 256-byte aligned
 static int dalloc(sb_handle *h, double **p, size_t n) {
-  void *q = nullptr;
-  cudaError_t e = cudaMalloc(&q, sizeof(double) * (n ? n : 1));
-  if (e != cudaSuccess) return fail(4, "cudaMalloc(%zu doubles): %s", n, cudaGetErrorString(e));
-  cudaMemset(q, 0, sizeof(double) * (n ? n : 1));
-  (h->alloc_to ? *h->alloc_to : h->allocs).push_back(q);
-  *p = (double *)q;
+  const size_t bytes = (sizeof(double) * (n ? n : 1) + 255) / 256 * 256;
+  constexpr size_t kChunk = 4 << 20;
+  if (h->alloc_to || bytes > kChunk / 4) return dmalloc(h, (void **)p, bytes);
+  if (h->chunk_used + bytes > h->chunk_size) {
+    const int rc = dmalloc(h, (void **)&h->chunk, kChunk);
+    if (rc) return rc;
+    h->chunk_used = 0;
+    h->chunk_size = kChunk;
+  }
+  *p = (double *)(h->chunk + h->chunk_used);
+  h->chunk_used += bytes;
   return 0;
 }
 static int upload(sb_handle *h, const double **dst, const std::vector<double> &v) {
@@ -248,7 +268,7 @@ static int build_line_tables(sb_handle *h, int nseg) {
       (rc = upload_uniform(h, &bf.d2, co.pr2, g.my)) ||
       (g.ydeal == 3 && (rc = upload_uniform(h, &bf.flt, flhs, g.my))))
     return rc;
-  {
+  if (h->banded) {
     // lines (kx, kz) and (kx, -kz) share k^2 and so their factors: the table
     // holds the kz >= 0 lines only (hz_line maps a line to its entry)
     const int nlh = g.nkx * (g.nz + 1);
@@ -347,6 +367,15 @@ static int build_line_tables(sb_handle *h, int nseg) {
   return 0;
 }
 
+
+// the banded solves' tables, where the handle has done without so far
+static int ensure_banded(sb_handle *h) {
+  if (h->banded) return 0;
+  h->banded = true;
+  const int rc = build_line_tables(h, h->g.nseg);
+  h->banded = rc == 0;
+  return rc;
+}
 
 // fixed-point twiddles of length n
 static int upload_qw(sb_handle *h, const qw **dst, const std::vector<int> &v) {
@@ -471,6 +500,10 @@ static cudaError_t launch_phases(sb_handle *h, int rk, cudaStream_t st) {
 }
 
 static int capture_step(sb_handle *h) {
+  if (!use_bloch(h)) {
+    const int rc = ensure_banded(h);
+    if (rc) return rc;
+  }
   if (h->step_exec) {
     cudaGraphExecDestroy(h->step_exec);
     h->step_exec = nullptr;
@@ -553,6 +586,13 @@ static int capture_step(sb_handle *h) {
 // the solves of the captured step
 static cudaError_t launch_prologue(sb_handle *h) {
   return h->step_bloch ? launch_lineQ(h->g, h->bf, 0, h->st) : launch_lineB(h->g, h->bf, 0, h->st);
+}
+
+// the step graph's form for the boxes' current offsets
+static int ensure_form(sb_handle *h) {
+  if (h->step_bloch == use_bloch(h)) return 0;
+  CK(cudaStreamSynchronize(h->st));
+  return capture_step(h);
 }
 
 static int ensure_trace(sb_handle *h, int cap) {
@@ -838,6 +878,7 @@ int sb_create(const sb_params *p, int batch, int precision, sb_handle **out) {
     sb_destroy(h);
     return rc;
   }
+  h->banded = !line_bloch_ok(g);
   if ((rc = build_line_tables(h, g.nseg)) || (rc = build_bloch_tables(h)) ||
       (rc = build_plane_tables(h))) {
     sb_destroy(h);
@@ -1131,10 +1172,7 @@ int sb_step(sb_handle *h, int nsteps) {
   if (nsteps < 0) return fail(1, "nsteps < 0");
   int rc = ensure_trace(h, nsteps > 0 ? nsteps : 1);
   if (rc) return rc;
-  if (h->step_bloch != use_bloch(h)) {
-    CK(cudaStreamSynchronize(h->st));
-    if ((rc = capture_step(h))) return rc;
-  }
+  if ((rc = ensure_form(h))) return rc;
   // entry of cross(): flags and offsets, phase tables, set_conj on the state,
   // v from phi and the first derivatives (cross.f90:76-113,283-287,376-445)
   CK(launch_scalar(h->g, h->bf, 0, h->st));
@@ -1243,6 +1281,11 @@ int sb_launch_stage(sb_handle *h, int stage, int rk, int count) {
   if (stage == 12 && !h->step_bloch && !line_fused_ok(h->g))
     return fail(1, "stage 12 (fused y-line kernel) not available for this handle");
   if (stage >= 13 && !h->g.impl) return fail(1, "stages 13, 14 need an implicit_visc handle");
+  if ((stage == 5 || stage == 6) && !h->banded) {
+    // the tables it replaces may be those of the step graph
+    int rc = ensure_banded(h);
+    if (rc || (rc = capture_step(h))) return rc;
+  }
   for (int q = 0; q < count; q++) {
     cudaError_t e;
     if (stage <= 3)
@@ -1326,11 +1369,13 @@ int sb_autotune(sb_handle *h, int *choice) {
   Grid &g = h->g;
   cudaStream_t st = h->st;
   // the derived fields of the current state, as at the entry of a call
+  int rc = ensure_form(h);
+  if (rc) return rc;
   CK(launch_scalar(g, h->bf, 0, st));
-  CK(launch_tables(g, h->bf, 0, st));
+  CK(launch_phases(h, 0, st));
   CK(launch_setconj(g, h->bf, st));
   if (g.ydeal == 3) CK(launch_filter(g, h->bf, 0, st));
-  CK(launch_lineB(g, h->bf, 0, st));
+  CK(launch_prologue(h));
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
@@ -1384,7 +1429,7 @@ int sb_autotune(sb_handle *h, int *choice) {
   int nseg = g.nseg, lform = g.lform;
   best = 1e30f;
   Snapshot snap;
-  int rc = snap.take(h);
+  rc = snap.take(h);
   for (int c : {1, 2, 3}) {
     if (rc || e != cudaSuccess) break;
     if ((g.my - 3) / c < 6) continue;
@@ -1508,10 +1553,12 @@ int sb_physical_fields(sb_handle *h, int member, unsigned mask, double *out) {
   cudaStream_t st = h->st;
   // the derived fields of the current state (v, dv/dy, d(omega_y)/dy, mean
   // derivatives), as at the entry of a call
+  const int frc = ensure_form(h);
+  if (frc) return frc;
   CK(launch_scalar(g, h->bf, 0, st));
-  CK(launch_tables(g, h->bf, 0, st));
+  CK(launch_phases(h, 0, st));
   CK(launch_setconj(g, h->bf, st));
-  CK(launch_lineB(g, h->bf, 0, st));
+  CK(launch_prologue(h));
   // one box: member-offset buffers, plane stage 1 with the extra z-transforms
   Grid gl = g;
   gl.B = 1;
