@@ -326,7 +326,7 @@ static int build_line_tables(sb_handle *h, int nseg) {
     }
     H.stride = nlh;
   }
-  if (g.impl) {
+  if (g.impl && h->banded) {
     // the semi-implicit Helmholtz tables, filled by k_hfac every substep:
     // boxes x (lines (kx, kz >= 0) + the mean line)
     const size_t n = g.my, L = (size_t)g.B * (g.nkx * (g.nz + 1) + 1);
@@ -514,6 +514,7 @@ static int capture_step(sb_handle *h) {
   h->bf.Dn = h->step_bloch ? h->bf.T : h->bf.D;
   CK(cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
   cudaError_t e = cudaSuccess;
+  const bool hfac = h->g.impl && !h->step_bloch;  // the factors of k_lineI
   for (int rk = 1; rk <= 3 && e == cudaSuccess; rk++) {
     if (h->g.ydeal == 3 && (e = launch_filter(h->g, h->bf, rk, h->st)) != cudaSuccess) break;
     if ((h->g.ydeal == 1 || h->g.ydeal == 2) &&
@@ -543,7 +544,7 @@ static int capture_step(sb_handle *h) {
           (e = cudaStreamWaitEvent(h->side, h->ev_fork, 0)) != cudaSuccess ||
           (e = launch_scalar(h->g, h->bf, rk, h->side)) != cudaSuccess ||
           (e = launch_phases(h, rk, h->side)) != cudaSuccess ||
-          (h->g.impl && (e = launch_hfac(h->g, h->bf, rk, h->side)) != cudaSuccess) ||
+          (hfac && (e = launch_hfac(h->g, h->bf, rk, h->side)) != cudaSuccess) ||
           (e = cudaEventRecord(h->ev_join, h->side)) != cudaSuccess ||
           (e = launch_plane(h->g, h->bf, 3, rk, h->st)) != cudaSuccess ||
           (e = cudaStreamWaitEvent(h->st, h->ev_join, 0)) != cudaSuccess)
@@ -555,15 +556,15 @@ static int capture_step(sb_handle *h) {
       if (h->g.les && (e = launch_les(h->g, h->bf, 5, rk, h->st)) != cudaSuccess) break;
       if ((e = launch_scalar(h->g, h->bf, rk, h->st)) != cudaSuccess) break;
       if ((e = launch_phases(h, rk, h->st)) != cudaSuccess) break;
-      if (h->g.impl && (e = launch_hfac(h->g, h->bf, rk, h->st)) != cudaSuccess) break;
+      if (hfac && (e = launch_hfac(h->g, h->bf, rk, h->st)) != cudaSuccess) break;
     }
     if (h->g.les && (e = launch_lineL(h->g, h->bf, h->st)) != cudaSuccess) break;
-    if (h->g.impl) {
-      e = launch_lineI(h->g, h->bf, rk, h->st);
-      continue;
-    }
     if (h->step_bloch) {
       e = launch_lineQ(h->g, h->bf, rk, h->st);
+      continue;
+    }
+    if (h->g.impl) {
+      e = launch_lineI(h->g, h->bf, rk, h->st);
       continue;
     }
     if (h->g.lform && line_fused_ok(h->g)) {
@@ -1281,7 +1282,7 @@ int sb_launch_stage(sb_handle *h, int stage, int rk, int count) {
   if (stage == 12 && !h->step_bloch && !line_fused_ok(h->g))
     return fail(1, "stage 12 (fused y-line kernel) not available for this handle");
   if (stage >= 13 && !h->g.impl) return fail(1, "stages 13, 14 need an implicit_visc handle");
-  if ((stage == 5 || stage == 6) && !h->banded) {
+  if ((stage == 5 || stage == 6 || stage >= 13) && !h->banded) {
     // the tables it replaces may be those of the step graph
     int rc = ensure_banded(h);
     if (rc || (rc = capture_step(h))) return rc;
@@ -1443,7 +1444,7 @@ int sb_autotune(sb_handle *h, int *choice) {
     for (int f = 1; f >= (bloch ? 1 : 0); f--) {
       if (rc || e != cudaSuccess) break;
       if (f == 1 && !bloch && !line_fused_ok(g)) continue;
-      g.lform = f;
+      if (!g.impl) g.lform = f;
       if ((rc = capture_step(h))) break;
       for (int q = 0; q < 3 && e == cudaSuccess; q++) {
         if ((rc = snap.restore(h))) break;
@@ -1456,7 +1457,7 @@ int sb_autotune(sb_handle *h, int *choice) {
         if (q == 1) t = tq;
         if (q == 2) t = t < tq ? t : tq;
       }
-      if (!rc && e == cudaSuccess && t < best) best = t, nseg = c, lform = f;
+      if (!rc && e == cudaSuccess && t < best) best = t, nseg = c, lform = g.lform;
     }
   }
   // which side work runs as a concurrent graph branch, on the chosen tile:
@@ -1509,7 +1510,7 @@ int sb_set_line_segments(sb_handle *h, int nseg) {
 int sb_set_line_form(sb_handle *h, int form) {
   if (!h) return fail(1, "null handle");
   if (form != 0 && form != 1) return fail(1, "line form %d (0 split, 1 fused)", form);
-  if (form == 1 && !h->g.bloch && !line_fused_ok(h->g))
+  if (form == 1 && (!h->g.bloch || h->g.impl) && !line_fused_ok(h->g))
     return fail(1, "fused y-line kernel not available for this handle");
   h->g.lform = form;
   return capture_step(h);

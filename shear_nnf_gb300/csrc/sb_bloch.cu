@@ -29,18 +29,21 @@
 #include "sb_fix.cuh"
 #include "sb_kernels.h"
 
-// Compiled six times: SB_FLOAT_TU = 0 (FP64) or 1 (FP32-mixed) storage times
-// SB_LEN = 0 (my 32..80), 1 (96..192), 2 (256..384); unit (0, 0) also holds
-// the entry points.
+// Compiled twelve times: SB_FLOAT_TU = 0 (FP64) or 1 (FP32-mixed) storage times
+// SB_LEN = 0 (my 32..80), 1 (96..192), 2 (256..384) times SB_IMPL = 0 (explicit)
+// or 1 (semi-implicit viscous branch); unit (0, 0, 0) also holds the entry points.
 #ifndef SB_FLOAT_TU
 #define SB_FLOAT_TU 0
 #endif
 #ifndef SB_LEN
 #define SB_LEN 0
 #endif
-#define SB_CAT2(a, b, c) a##b##_##c
-#define SB_CAT(a, b, c) SB_CAT2(a, b, c)
-#define SB_LINEQ_UNIT(f, l) SB_CAT(lineQ_unit, f, l)
+#ifndef SB_IMPL
+#define SB_IMPL 0
+#endif
+#define SB_CAT2(a, b, c, d) a##b##_##c##_##d
+#define SB_CAT(a, b, c, d) SB_CAT2(a, b, c, d)
+#define SB_LINEQ_UNIT(f, l, i) SB_CAT(lineQ_unit, f, l, i)
 
 namespace sb {
 
@@ -67,6 +70,14 @@ __device__ __forceinline__ unsigned vtop(V v) {
 template <typename V>
 __device__ __forceinline__ q2 vfix(V v, const QScale &s) {
   return mkq(tofix(v.x, s), tofix(v.y, s));
+}
+
+// 1/x by two Newton steps from the 20-bit estimate
+__device__ __forceinline__ double recip(double x) {
+  double z;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(z) : "d"(x));
+  z = fma(z, fma(-x, z, 1.0), z);
+  return fma(z, fma(-x, z, 1.0), z);
 }
 
 // hides where a pointer comes from, so that the loads of a loop that runs once
@@ -143,7 +154,13 @@ struct LineQRegs {
 // instruction cache, and each warp runs it only once): pass 0 takes the
 // right-hand side and the update at the phase of time t, pass 1 the outputs at
 // the phase of t + c_k dt.  A pass: rows in, forward, products, inverse, rows out.
-template <typename R, int N, int T>
+// IM: the semi-implicit viscous branch (explicit = 0, cross.f90:797-989).  Pass 0
+// gives the viscous term and (phi) -d(D)/dy apart, the update forms the
+// right-hand side -Re ibeta_k (wk + alpha_k nu lap f + f/Dt) of the Helmholtz
+// equation in the frame of t + c_k Dt, and pass 1 solves it on the waves,
+// f = rhs/(l2 - k^2 - Re ibeta_k/Dt), before the outputs; the state is one
+// more output.  The (0,0) line keeps its state.
+template <typename R, int N, int T, bool IM>
 __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid g, Bufs bf, int rk1) {
   typedef LineQ<N> L;
   typedef typename V2<R>::t V;
@@ -156,7 +173,10 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
   q2 *const ex = (q2 *)smq_raw;              // two buffers of N x kCols
   double *const sc = (double *)(ex + 2 * N * kCols);  // factors of the waves
   __shared__ unsigned s_top[2][kCols];  // largest upper words: D, the new state
-  __shared__ int s_len[3][kCols];       // scales of the products: right-hand side, first, second output
+  // scales of the products: right-hand side, first, second output; IM: the
+  // second of pass 0, the Helmholtz solve
+  constexpr int kLens = IM ? 5 : 3;
+  __shared__ int s_len[kLens][kCols];
   const int ncb = (g.nkx + kCols - 1) / kCols, per = g.mz * ncb;
   const int role = blockIdx.x / per;  // 0 phi, 1 omega_y, 2 mean
   const int r = blockIdx.x - role * per;
@@ -172,8 +192,8 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
   const long ps = g.plane / 2;  // complex entries per plane
   const long off = (long)b * (g.field / 2) + (long)k * nkx + i;
   const int rk = rk1 - 1;
-  static_assert(T >= 3 * kCols, "one thread per slot");
-  if (threadIdx.x < 3 * kCols) {
+  static_assert(T >= kLens * kCols, "one thread per slot");
+  if (threadIdx.x < kLens * kCols) {
     if (threadIdx.x < 2 * kCols) (&s_top[0][0])[threadIdx.x] = 0u;
     (&s_len[0][0])[threadIdx.x] = kNoLen;
   }
@@ -181,7 +201,10 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
   const long tb = (long)N * nkx;
   const double a = g.alp * i, gz = g.gam * ((k <= g.nz) ? k : k - g.mz);
   const double k2 = mean ? 0.0 : a * a + gz * gz;
-  const double nu = is00 ? 0.0 : M.nu, nuk2 = nu * k2;
+  const double Dt = M.Deltat;
+  // of the viscous term of pass 0, and for IM the scales of the right-hand side
+  const double nu = is00 ? 0.0 : IM && rk1 > 0 ? kAlpha[rk] * M.nu : M.nu, nuk2 = nu * k2;
+  const double fb = IM && rk1 > 0 ? -M.Re * kIbeta[rk] : 0.0, rdt = IM ? 1.0 / Dt : 0.0;
   V *f = (V *)(role == 0 ? bf.phi : bf.vor) + off;
   R *mf = (R *)bf.mu + (long)b * 2 * N + cm;  // mean profile of this column
   // the waves of the state, kept from pass 1 for the next substep's pass 0 (the
@@ -197,7 +220,7 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
     const qw *tw = bf.btw + o;
     const double *l1 = bf.bl1 + o, *l2 = bf.bl2 + o;
     const int nf = ph == 0 && role == 0 ? 2 : 1;  // fields in: the state, D
-    const int no = ph == 1 && role == 0 ? 2 : 1;  // fields out
+    const int no = (IM || ph == 1) && role == 0 ? 2 : 1;  // fields out
     // ---- rows in: D to buffer 1 (phi, pass 0), the state of the start of a run
     // to buffer 0 (in pass 1 the new state is there already)
     const bool rows = ph == 1 || role == 0;
@@ -216,13 +239,72 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
     // scales: 0 the state (pass 0: of the waves kept from the last pass 1), 1 D
     const QScale sr = qscale(s_top[ph][ci], L::kBits);
     const int kept = ph == 0 ? *wscale : 0;
-    const int w0 = ph == 0 ? kept : sr.weight(), w1 = sr.weight();
+    int w0 = ph == 0 ? kept : sr.weight();
+    const int w1 = sr.weight();
     const bool bad = (ph == 0 && kept == kNoLen) || (rows && sr.bad);
     if (rows) {
 #pragma unroll 1
       for (int it = n; it < R2; it += T / kCols)
         rows_forward<N, V>(ex + (1 - ph) * N * kCols, sr, tw, nkx, bf.bftw, it, ci);
       __syncthreads();
+    }
+    const int eb = L::kShiftF + Plan<N>::shift + 2 - kN - kTgt;
+    const bool solve = IM && ph == 1 && rk1 > 0;
+    if constexpr (IM) {
+      if (solve) {
+        // ---- the Helmholtz solve; the waves of the new state stay in buffer 0
+        const double dtr = M.Re * kIbeta[rk] * rdt;
+#pragma unroll 1
+        for (int k1 = n; k1 < R1; k1 += T / kCols) {
+          const double *l = l2 + (long)k1 * nkx;
+          q2 *e = ex + k1 * R2 * kCols + ci;
+          q2 x[R2];
+#pragma unroll
+          for (int w = 0; w < R2; w++) x[w] = e[w * kCols];
+          Dft<R2, -1>::run(x);
+          int la = kNoLen;
+#pragma unroll
+          for (int w = 0; w < R2; w++) {
+            const double c = is00 ? 1.0 : recip(l[(long)(R1 * w) * nkx] - k2 - dtr);
+            sc[(k1 * R2 + w) * kCols + ci] = c;
+            e[w * kCols] = x[w];
+            la = max(la, qlen(x[w]) + qexp(c));
+          }
+          atomicMax(&s_len[4][ci], la);
+        }
+        __syncthreads();
+        const int len = s_len[4][ci] + 1, sh = kTgt - len;
+#pragma unroll 1
+        for (int k1 = n; k1 < R1; k1 += T / kCols) {
+          q2 *e = ex + k1 * R2 * kCols + ci;
+          q2 x[R2];
+#pragma unroll
+          for (int w = 0; w < R2; w++) {
+            x[w] = qscaled(e[w * kCols], sc[(k1 * R2 + w) * kCols + ci], sh);
+            e[w * kCols] = x[w];
+          }
+          Dft<R2, 1>::run(x);
+#pragma unroll
+          for (int w = 0; w < R2; w++) e[(N + w) * kCols] = qmul<false>(x[w], bf.bitw[w * k1]);
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int it = n; it < R2; it += T / kCols)
+          rows_inverse<N>(ex + N * kCols, here(tw), nkx, it, ci);
+        __syncthreads();
+        const bool none = bad || qrange(eb - w0 + len);
+        const R nn = (R)nan("");
+        if (act && !is00)
+#pragma unroll 1
+          for (int j = n; j < N; j += T / kCols) {
+            const q2 z = ex[(N + j) * kCols + ci];
+            const V v = none ? mkv<R>(nn, nn)
+                             : mkv<R>(qout<R>(z.x, eb - w0 + len), qout<R>(z.y, eb - w0 + len));
+            if (mean) mf[2 * j] = v.x;
+            else f[(long)j * ps] = v;
+          }
+        w0 += sh;
+      }
     }
     // ---- products.  Pass 0: nu (l2 - k^2) f - i l1 D; pass 1: phi f/(l2 - k^2)
     // and i l1 of it, else i l1 f.  The waves stay in the thread's own slots
@@ -239,13 +321,7 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
         if (ph == 0) {
           c = fma(nu, l2[p], -nuk2);
         } else if (role == 0) {
-          // reciprocal by two Newton steps from the 20-bit estimate
-          const double den = l2[p] - k2;
-          double z;
-          asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(z) : "d"(den));
-          z = fma(z, fma(-den, z, 1.0), z);
-          z = fma(z, fma(-den, z, 1.0), z);
-          c = is00 ? 0.0 : z;
+          c = is00 ? 0.0 : recip(l2[p] - k2);
         } else {
           c = l1[p];
         }
@@ -263,7 +339,7 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
         } else {
 #pragma unroll
           for (int w = 0; w < R2; w++) x[w] = e[w * kCols];
-          Dft<R2, -1>::run(x);
+          if (!solve) Dft<R2, -1>::run(x);
         }
         if (ph == 1 && act) {
           q2 *wv = waves + k1 * wst;
@@ -278,14 +354,15 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
           la = max(la, len + (q ? e1 : ec));
           lb = max(lb, len + ec + e1 + 1);
         }
-        atomicMax(&s_len[ph][ci], la - (ph == 0 ? (q ? w1 : w0) : 0));
-        if (no > 1) atomicMax(&s_len[2][ci], lb);
+        atomicMax(&s_len[IM && ph == 0 && q ? 3 : ph][ci], la - (ph == 0 ? (q ? w1 : w0) : 0));
+        if (ph == 1 && no > 1) atomicMax(&s_len[2][ci], lb);
       }
       if (ph == 1 && k1 == 0 && act) *wscale = bad ? kNoLen : w0;
     }
     __syncthreads();
     // scales of the outputs; in pass 0 of the sum of two terms
-    const int len1 = s_len[ph][ci] + (ph == 0 ? 2 : 1), len2 = s_len[2][ci] + 1;
+    const int len1 = s_len[ph][ci] + (!IM && ph == 0 ? 2 : 1);
+    const int len2 = s_len[IM && ph == 0 ? 3 : 2][ci] + 1;
 #pragma unroll 1
     for (int k1 = n; k1 < R1; k1 += T / kCols) {
       const double *cw = sc + k1 * R2 * kCols + ci;
@@ -326,7 +403,6 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
     }
     __syncthreads();
     // ---- rows out
-    const int eb = L::kShiftF + Plan<N>::shift + 2 - kN - kTgt;
     if (ph == 1) {
       const int e0 = eb - w0;
       const bool nan1 = bad || qrange(e0 + len1), nan2 = bad || qrange(e0 + len2);
@@ -356,8 +432,9 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
     }
     // RK3 accumulation and update, zeta store, remaps (cross.f90:694-781)
     const int eo = eb + len1;
-    const bool nanr = bad || qrange(eo);
-    const R gk = (R)kGama[rk], zk = (R)kZeta[rk], dtr = (R)M.Deltat;
+    const int ed = eb + len2;  // IM: of -d(D)/dy
+    const bool nanr = bad || qrange(eo) || (IM && no > 1 && qrange(ed));
+    const R gk = (R)kGama[rk], zk = (R)kZeta[rk], dtr = (R)Dt;
     unsigned top = 0;
     if (mean) {
       R *mwk = (R *)bf.mwk + (long)b * 2 * N + cm;
@@ -376,12 +453,20 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
                                         (1.0 + tanh(6.0 * (g.damp_a + y) / g.lz + 3.0));
             rf0 = (R)((double)rf0 - g.damp_up * hw * (double)mf[2 * j]);
           }
-          const R rf = rf0 + (nanr ? (R)nan("") : qout<R>(ex[j * kCols + ci].x, eo));
-          R wk = (rk == 0) ? gk * rf : mwk[2 * j] + gk * rf;
-          un = mf[2 * j] + dtr * wk;
-          if (rk < 2) wk = rf * zk;
-          mf[2 * j] = un;
-          mwk[2 * j] = wk;
+          const ll z = ex[j * kCols + ci].x;
+          if constexpr (IM) {
+            const R wk = (rk == 0) ? gk * rf0 : mwk[2 * j] + gk * rf0;
+            const double vis = nanr ? nan("") : fromfix(z, eo);
+            un = (R)(fb * (((double)wk + vis) + rdt * (double)mf[2 * j]));
+            if (rk < 2) mwk[2 * j] = zk * rf0;
+          } else {
+            const R rf = rf0 + (nanr ? (R)nan("") : qout<R>(z, eo));
+            R wk = (rk == 0) ? gk * rf : mwk[2 * j] + gk * rf;
+            un = mf[2 * j] + dtr * wk;
+            if (rk < 2) wk = rf * zk;
+            mf[2 * j] = un;
+            mwk[2 * j] = wk;
+          }
         }
         const V w = mkv<R>(un, (R)0);
         top = max(top, vtop(w));
@@ -397,12 +482,25 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
         const long q = (long)j * ps;
         const V fo = f[q], rh = rhs[q], w0 = rk > 0 ? fwk[q] : none;
         const q2 z = ex[j * kCols + ci];
-        V h = mkv<R>(rh.x + qout<R>(z.x, eo), rh.y + qout<R>(z.y, eo));
+        V h = rh;
+        if constexpr (!IM) {
+          h = mkv<R>(rh.x + qout<R>(z.x, eo), rh.y + qout<R>(z.y, eo));
+        } else if (role == 0) {
+          const q2 d = ex[(N + j) * kCols + ci];
+          h = mkv<R>(rh.x + qout<R>(d.x, ed), rh.y + qout<R>(d.y, ed));
+        }
         if (nanr) h = mkv<R>((R)nan(""), (R)nan(""));
         V wk = mkv<R>(w0.x + gk * h.x, w0.y + gk * h.y);
         const double2 p2 = m2[(long)j * nkx];
-        const double fx = (double)(fo.x + dtr * wk.x), fy = (double)(fo.y + dtr * wk.y);
-        const V fn = mkv<R>((R)fma(fx, p2.x, -(fy * p2.y)), (R)fma(fy, p2.x, fx * p2.y));
+        double fx, fy;
+        if constexpr (IM) {
+          fx = fb * (((double)wk.x + fromfix(z.x, eo)) + rdt * (double)fo.x);
+          fy = fb * (((double)wk.y + fromfix(z.y, eo)) + rdt * (double)fo.y);
+        } else {
+          fx = (double)(fo.x + dtr * wk.x), fy = (double)(fo.y + dtr * wk.y);
+        }
+        V fn = mkv<R>((R)fma(fx, p2.x, -(fy * p2.y)), (R)fma(fy, p2.x, fx * p2.y));
+        if (IM && is00) fn = fo;
         if (rk < 2) {
           // zeta_k h in the frame of the next substep; zeta_k is in the phase
           const double2 p1 = m1[(long)j * nkx];
@@ -410,8 +508,8 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
           wk = mkv<R>((R)fma(hx, p1.x, -(hy * p1.y)), (R)fma(hy, p1.x, hx * p1.y));
         }
         if (act) {
-          f[q] = fn;
-          fwk[q] = wk;
+          if (!IM) f[q] = fn;
+          if (!IM || rk < 2) fwk[q] = wk;
         }
         top = max(top, vtop(fn));
         *(V *)(ex + j * kCols + ci) = fn;
@@ -424,28 +522,28 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-template <typename R, int N, int T>
+template <typename R, int N, int T, bool IM>
 static cudaError_t launch_n(const Grid &g, const Bufs &bf, int rk, cudaStream_t st, bool prep,
                             unsigned blocks) {
   if (prep)
-    return cudaFuncSetAttribute(k_lineQ<R, N, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(k_lineQ<R, N, T, IM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)LineQ<N>::smem);
-  k_lineQ<R, N, T><<<dim3(blocks, (unsigned)g.B), T, LineQ<N>::smem, st>>>(g, bf, rk);
+  k_lineQ<R, N, T, IM><<<dim3(blocks, (unsigned)g.B), T, LineQ<N>::smem, st>>>(g, bf, rk);
   return cudaGetLastError();
 }
-template <typename R, int N>
+template <typename R, int N, bool IM>
 static cudaError_t launch_t(const Grid &g, const Bufs &bf, int rk, cudaStream_t st, bool prep) {
   constexpr int W = LineQ<N>::kWide, S = LineQ<N>::kNarrow;
   const unsigned blocks = (unsigned)(2 * g.mz * ((g.nkx + kCols - 1) / kCols) + 1);
-  if constexpr (W != S) {
+  if constexpr (W != S && !IM) {
     if (prep) {
-      const cudaError_t e = launch_n<R, N, S>(g, bf, rk, st, true, blocks);
+      const cudaError_t e = launch_n<R, N, S, IM>(g, bf, rk, st, true, blocks);
       if (e != cudaSuccess) return e;
     } else if ((long)blocks * g.B >= 5 * 152) {
-      return launch_n<R, N, S>(g, bf, rk, st, false, blocks);
+      return launch_n<R, N, S, IM>(g, bf, rk, st, false, blocks);
     }
   }
-  return launch_n<R, N, W>(g, bf, rk, st, prep, blocks);
+  return launch_n<R, N, W, IM>(g, bf, rk, st, prep, blocks);
 }
 
 #if SB_FLOAT_TU
@@ -453,29 +551,30 @@ typedef float UnitR;
 #else
 typedef double UnitR;
 #endif
-cudaError_t SB_LINEQ_UNIT(SB_FLOAT_TU, SB_LEN)(const Grid &g, const Bufs &bf, int rk,
-                                               cudaStream_t st, bool prep) {
+cudaError_t SB_LINEQ_UNIT(SB_FLOAT_TU, SB_LEN, SB_IMPL)(const Grid &g, const Bufs &bf, int rk,
+                                                        cudaStream_t st, bool prep) {
+  constexpr bool I = SB_IMPL != 0;
   switch (g.my) {
 #if SB_LEN == 0
-    case 32: return launch_t<UnitR, 32>(g, bf, rk, st, prep);
-    case 48: return launch_t<UnitR, 48>(g, bf, rk, st, prep);
-    case 64: return launch_t<UnitR, 64>(g, bf, rk, st, prep);
-    case 80: return launch_t<UnitR, 80>(g, bf, rk, st, prep);
+    case 32: return launch_t<UnitR, 32, I>(g, bf, rk, st, prep);
+    case 48: return launch_t<UnitR, 48, I>(g, bf, rk, st, prep);
+    case 64: return launch_t<UnitR, 64, I>(g, bf, rk, st, prep);
+    case 80: return launch_t<UnitR, 80, I>(g, bf, rk, st, prep);
 #elif SB_LEN == 1
-    case 96: return launch_t<UnitR, 96>(g, bf, rk, st, prep);
-    case 128: return launch_t<UnitR, 128>(g, bf, rk, st, prep);
-    case 160: return launch_t<UnitR, 160>(g, bf, rk, st, prep);
-    case 192: return launch_t<UnitR, 192>(g, bf, rk, st, prep);
+    case 96: return launch_t<UnitR, 96, I>(g, bf, rk, st, prep);
+    case 128: return launch_t<UnitR, 128, I>(g, bf, rk, st, prep);
+    case 160: return launch_t<UnitR, 160, I>(g, bf, rk, st, prep);
+    case 192: return launch_t<UnitR, 192, I>(g, bf, rk, st, prep);
 #else
-    case 256: return launch_t<UnitR, 256>(g, bf, rk, st, prep);
-    case 320: return launch_t<UnitR, 320>(g, bf, rk, st, prep);
-    case 384: return launch_t<UnitR, 384>(g, bf, rk, st, prep);
+    case 256: return launch_t<UnitR, 256, I>(g, bf, rk, st, prep);
+    case 320: return launch_t<UnitR, 320, I>(g, bf, rk, st, prep);
+    case 384: return launch_t<UnitR, 384, I>(g, bf, rk, st, prep);
 #endif
     default: return cudaErrorInvalidValue;
   }
 }
 
-#if !SB_FLOAT_TU && SB_LEN == 0
+#if !SB_FLOAT_TU && SB_LEN == 0 && !SB_IMPL
 // ---------------------------------------------------------------------------
 // the phase tables of slot sn for a box: per (row or wave m, kx) the twist
 // exp(-i psi m/my) and the symbols l1, l2 at t = (psi + 2 pi m)/my.  psi is
@@ -545,17 +644,23 @@ __global__ void __launch_bounds__(64) k_bloch(Grid g, Bufs bf, int rk) {
 }
 
 typedef cudaError_t LineQUnit(const Grid &, const Bufs &, int, cudaStream_t, bool);
-LineQUnit lineQ_unit0_1, lineQ_unit0_2, lineQ_unit1_0, lineQ_unit1_1, lineQ_unit1_2;
+LineQUnit lineQ_unit0_1_0, lineQ_unit0_2_0, lineQ_unit1_0_0, lineQ_unit1_1_0, lineQ_unit1_2_0;
+LineQUnit lineQ_unit0_0_1, lineQ_unit0_1_1, lineQ_unit0_2_1, lineQ_unit1_0_1, lineQ_unit1_1_1,
+    lineQ_unit1_2_1;
 static cudaError_t lineQ(const Grid &g, const Bufs &bf, int rk, cudaStream_t st, bool prep) {
-  static LineQUnit *const unit[2][3] = {{lineQ_unit0_0, lineQ_unit0_1, lineQ_unit0_2},
-                                        {lineQ_unit1_0, lineQ_unit1_1, lineQ_unit1_2}};
-  return unit[g.prec ? 1 : 0][g.my < 96 ? 0 : g.my < 256 ? 1 : 2](g, bf, rk, st, prep);
+  static LineQUnit *const unit[2][2][3] = {
+      {{lineQ_unit0_0_0, lineQ_unit0_1_0, lineQ_unit0_2_0},
+       {lineQ_unit1_0_0, lineQ_unit1_1_0, lineQ_unit1_2_0}},
+      {{lineQ_unit0_0_1, lineQ_unit0_1_1, lineQ_unit0_2_1},
+       {lineQ_unit1_0_1, lineQ_unit1_1_1, lineQ_unit1_2_1}}};
+  return unit[g.impl ? 1 : 0][g.prec ? 1 : 0][g.my < 96 ? 0 : g.my < 256 ? 1 : 2](g, bf, rk, st,
+                                                                                 prep);
 }
 
-// the plain explicit step (LES included: its k_lineL runs before) on the
-// transform lengths; the temperature, the y filter and dealiasing and the
-// semi-implicit branch keep the banded solves
-bool line_bloch_ok(const Grid &g) { return !g.temp && !g.ydeal && !g.impl && fix_length(g.my); }
+// the plain step, explicit (LES included: its k_lineL runs before) or
+// semi-implicit, on the transform lengths; the temperature, the y filter and
+// dealiasing keep the banded solves
+bool line_bloch_ok(const Grid &g) { return !g.temp && !g.ydeal && fix_length(g.my); }
 
 cudaError_t launch_lineQ(const Grid &g, const Bufs &bf, int rk, cudaStream_t st) {
   return lineQ(g, bf, rk, st, false);
@@ -567,6 +672,6 @@ cudaError_t launch_bloch(const Grid &g, const Bufs &bf, int rk, cudaStream_t st)
   return cudaGetLastError();
 }
 
-#endif  // unit (0, 0)
+#endif  // unit (0, 0, 0)
 
 }  // namespace sb

@@ -134,6 +134,9 @@ enum { SBF_DIVERGED = 1, SBF_NAN = 2, SBF_LAMINAR = 4, SBF_ETIME = 8 };
 // (cross.f90:17-24)
 __device__ __constant__ static const double kGama[3] = {8.0 / 15.0, 5.0 / 12.0, 3.0 / 4.0};
 __device__ __constant__ static const double kZeta[3] = {-17.0 / 60.0, -5.0 / 12.0, 0.0};
+// the semi-implicit branch (cross.f90:800-830)
+__device__ __constant__ static const double kAlpha[3] = {29.0 / 96.0, -3.0 / 40.0, 1.0 / 6.0};
+__device__ __constant__ static const double kIbeta[3] = {160.0 / 37.0, 24.0 / 5.0, 6.0};
 __device__ __constant__ static const double kCa[3] = {8.0 / 15.0, 2.0 / 3.0, 1.0};
 
 // Device arrays of one handle

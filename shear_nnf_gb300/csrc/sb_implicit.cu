@@ -23,7 +23,6 @@
 
 namespace sb {
 
-__device__ __constant__ static const double kIbeta[3] = {160.0 / 37.0, 24.0 / 5.0, 6.0};
 
 // Lanes: (part, line) = (lane / kHfLines, lane % kHfLines), 10 lines per warp
 // and three parts per line (lanes 30, 31 idle).  GB300 issues an FP64 warp

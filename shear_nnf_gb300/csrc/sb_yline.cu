@@ -720,8 +720,6 @@ __global__ void __launch_bounds__(64 * kSeg, SB_LINEF_WARPS / (2 * kSeg) > 0 ? S
 // (d(-vT00)/dy -> mtr in phase 1, tb00'' in phase 2, the right-hand side
 // through mtr in phase 3, the solve of dtr1k in phase 4).  The (0,0) line
 // keeps its state (cross.f90 and crosst.f90 skip it).
-__device__ __constant__ static const double kAlpha[3] = {29.0 / 96.0, -3.0 / 40.0, 1.0 / 6.0};
-__device__ __constant__ static const double kIbetaL[3] = {160.0 / 37.0, 24.0 / 5.0, 6.0};
 
 template <typename R, bool TEMP>
 __global__ void __launch_bounds__((TEMP ? 96 : 64) * kSeg, 1) k_lineI(Grid g, Bufs bf, int rk1) {
@@ -738,9 +736,9 @@ __global__ void __launch_bounds__((TEMP ? 96 : 64) * kSeg, 1) k_lineI(Grid g, Bu
   const FacView V1(bf.d1, 0), V2(bf.d2, 0);
   const SegView W1(bf.d1, 0), W2(bf.d2, 0);
   const double Dt = M.Deltat, nu = M.nu;
-  const double fa = kAlpha[rk] * nu, fb = -M.Re * kIbetaL[rk], rdt = 1.0 / Dt;
+  const double fa = kAlpha[rk] * nu, fb = -M.Re * kIbeta[rk], rdt = 1.0 / Dt;
   const double fat = TEMP ? kAlpha[rk] * g.kappa : 0.0;
-  const double fbt = TEMP ? -(1.0 / g.kappa) * kIbetaL[rk] : 0.0;
+  const double fbt = TEMP ? -(1.0 / g.kappa) * kIbeta[rk] : 0.0;
   const R gk = (R)kGama[rk], zk = (R)kZeta[rk];
   // this box's entries of the implicit factors: lines (kx, kz >= 0), then the mean line
   const int nl = g.nkx * (g.nz + 1);

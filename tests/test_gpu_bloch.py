@@ -71,6 +71,40 @@ def test_mixed_close_to_the_banded_form(my):
         assert rel_l2(out["fused"][k], out["split"][k]) < 1e-6, k
 
 
+@pytest.mark.parametrize("my", LENGTHS)
+def test_semi_implicit_at_every_length(my):
+    """implicit_visc = 1: two steps against the oracle, and in the FP32-mixed
+    form against the banded solves (set_line_form("split"))."""
+    import shear_nnf_gb300 as sb
+    pp = box_params(48, my, 32, rez=1500.0, implicit_visc=1,
+                    fixed_dt=0.3 * 2 * np.pi / my / 4)
+    p = sb.make_params(**pp)
+    st = _state(p, my, 1.3)
+    box, _ = _parity(pp, st, nstep=2, tol=4 * ONE_STEP)
+    assert box.tuning()["line_form"] == "implicit"
+    out = {}
+    for form in ("split", "waves"):
+        box = sb.ShearBox(p, precision=sb.SB_MIXED)
+        if form == "split":
+            box.set_line_form(form)
+        s = copy_state(st)
+        box.cross(s, 2)
+        out[form] = s
+    for k in ("vor", "phi", "u00"):
+        assert rel_l2(out["waves"][k], out["split"][k]) < 1e-6, k
+
+
+def test_semi_implicit_options():
+    """Damping and forcing of the mean, and unequal offsets (banded)."""
+    import shear_nnf_gb300 as sb
+    pp = box_params(48, 96, 32, rez=1500.0, implicit_visc=1, fixed_dt=0.003, damping=1,
+                    damp_up=0.5, damp_aa=0.2, force=-1, xforce=0.03)
+    p = sb.make_params(**pp)
+    box, _ = _parity(pp, _state(p, 2, -0.8), nstep=2, tol=4 * ONE_STEP)
+    _parity(pp, _state(p, 2, 1.1, xoffb=-0.9), nstep=2, tol=4 * ONE_STEP, box=box)
+    _parity(pp, _state(p, 3, 0.7), nstep=2, tol=4 * ONE_STEP, box=box)
+
+
 def test_unequal_offsets_keep_the_banded_solves():
     """xoffb != -xofft: one handle steps such a state (banded), then opposite
     offsets again, with the bits of a fresh handle."""
