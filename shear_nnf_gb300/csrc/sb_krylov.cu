@@ -22,6 +22,7 @@
 
 #include "../../include/shearbox.h"
 #include "sb_common.cuh"
+#include "sb_fix.cuh"
 #include "sb_kernels.h"
 
 namespace sb {
@@ -49,6 +50,7 @@ int kfail(int code, const char *fmt, ...) {
   } while (0)
 
 constexpr int kThreads = 256;
+constexpr int kUThreads = 128;  // of the fixed-point update
 constexpr int kTA = 4;  // columns of the left block per gram tile
 constexpr int kTB = 8;  // columns of the right block per gram tile
 constexpr int kMaxSrc = 8;
@@ -105,13 +107,184 @@ k_gram(const double *__restrict__ V, long ld, long r0, long r1, long chunk, int 
   }
 }
 
-__global__ void k_gram_sum(const double *__restrict__ part, int nchunk, int m, int p,
-                           double *__restrict__ C) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= m * p) return;
+// 32 products and 32 chunk lanes per block: each lane sums every 32nd chunk,
+// then the lanes in order
+__global__ void __launch_bounds__(1024)
+k_gram_sum(const double *__restrict__ part, int nchunk, int m, int p, double *__restrict__ C) {
+  __shared__ double s[32][33];
+  const int q = blockIdx.x * 32 + threadIdx.x;
   double v = 0.0;
-  for (int c = 0; c < nchunk; c++) v += part[(long)c * m * p + q];
-  C[q] = v;
+  if (q < m * p)
+    for (int c = threadIdx.y; c < nchunk; c += 32) v += part[(long)c * m * p + q];
+  s[threadIdx.y][threadIdx.x] = v;
+  __syncthreads();
+  for (int o = 16; o > 0; o >>= 1) {
+    if ((int)threadIdx.y < o) s[threadIdx.y][threadIdx.x] += s[threadIdx.y + o][threadIdx.x];
+    __syncthreads();
+  }
+  if (threadIdx.y == 0 && q < m * p) C[q] = s[0][threadIdx.x];
+}
+
+// ---------------------------------------------------------------------------
+// The same products in block fixed point.  A column's 128 rows of a chunk share
+// a power of two taken from their largest entry, |x| 2^p < 2^58, split into
+// two signed halves at 2^30; a product keeps hi*hi and the two cross terms
+// (three 32 x 32 + 64 bit multiply-adds, 6 issue cycles against 64 for one
+// FP64 fused multiply-add) and drops lo*lo, 2^-59 of the largest product.  The
+// chunk's sums are exact, |sum| < 2^123, kept to 2^60, and meet in FP64.  At
+// most 16 rows meet in one cross sum (< 2^62) before its upper bits move to hi.
+// Chunks that hold an infinity, a NaN or numbers beyond 2^+-400 take FP64 sums.
+//
+// Tile: 64 x 16 columns, 4 x 4 products per thread, the rows split over ks
+// threads.  The chunk comes by asynchronous copies into shared memory and is
+// converted in place, a warp per column: with the loads in registers instead a
+// block waited for memory ten times a stage (187488 rows, 48 x 16: 200 us).
+// ---------------------------------------------------------------------------
+constexpr int kQBits = 58, kQLow = 30;
+constexpr int kQA = 64, kQB = 16;  // columns of a tile
+constexpr int kQR = 128;           // rows of a chunk
+constexpr int kQS = kQR + 2;       // column stride: odd in 16-byte units
+constexpr int kQLim = 400;
+
+__device__ __forceinline__ int2 qsplit(long long x) {
+  const int lo = ((int)x << (32 - kQLow)) >> (32 - kQLow);
+  return make_int2(lo, (int)((x - lo) >> kQLow));
+}
+// 8 bytes global -> shared, zeros where !on
+__device__ __forceinline__ void copy8(void *dst, const void *src, bool on) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(on ? 8 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void copy_wait() {
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(kThreads, 2)
+k_gramq(const double *__restrict__ V, long ld, long r0, long r1, int ks, int a0, int m, int b0,
+        int p, double *__restrict__ part) {
+  extern __shared__ __align__(16) int2 sx[];
+  __shared__ int sp[kQA + kQB];  // the columns' powers of two
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ta = blockIdx.y * kQA, tb = blockIdx.z * kQB;
+  const int mt = min(kQA, m - ta), pt = min(kQB, p - tb), nc = mt + pt;
+  const int GA = (mt + 3) / 4, GB = (pt + 3) / 4, nq = GA * GB;
+  // product tile and row slice; for the sums over the slices (q, sl = product)
+  const int q = tid % nq, sl = tid / nq;
+  const int ga = q % GA, gb = q / GA;
+  auto col = [&](int c) { return V + (long)(c < mt ? a0 + ta + c : b0 + tb + c - mt) * ld; };
+  int pa[4], pb[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    pa[i] = min(ga + i * GA, mt - 1) * kQS;
+    pb[i] = (mt + min(gb + i * GB, pt - 1)) * kQS;
+  }
+  double out[4] = {0.0, 0.0, 0.0, 0.0};
+  for (long lo = r0 + (long)blockIdx.x * kQR; lo < r1; lo += (long)gridDim.x * kQR) {
+    const int nr = (int)min((long)kQR, r1 - lo);
+    for (int c = warp; c < nc; c += kThreads / 32) {
+      const double *x = col(c) + lo;
+#pragma unroll
+      for (int r = lane; r < kQR; r += 32) copy8(sx + c * kQS + r, x + min(r, nr - 1), r < nr);
+    }
+    copy_wait();  // a warp converts the columns that it copied
+    __syncwarp();
+    bool bad = false;
+#pragma unroll 2
+    for (int c = warp; c < nc; c += kThreads / 32) {
+      double x[kQR / 32];
+      unsigned t = 0;
+#pragma unroll
+      for (int u = 0; u < kQR / 32; u++) {
+        x[u] = *reinterpret_cast<const double *>(sx + c * kQS + lane + 32 * u);
+        t = max(t, sb::hiword(x[u]));
+      }
+      t = __reduce_max_sync(0xffffffffu, t);
+      const int E = (int)(t >> 20) - 1023;
+      bad |= t != 0 && (E > kQLim || E < -kQLim);
+      const sb::QScale sc = sb::qscale(t, kQBits);
+#pragma unroll
+      for (int u = 0; u < kQR / 32; u++) sx[c * kQS + lane + 32 * u] = qsplit(sb::tofix(x[u], sc));
+      if (lane == 0) sp[c] = t ? sc.p : 0;
+    }
+    if (__syncthreads_or(bad)) {
+      for (int i = 0; i < 4; i++) {
+        const int a = ga + i * GA, b = gb + sl * GB;
+        if (sl < 4 && a < mt && b < pt) {
+          const double *x = col(a) + lo, *y = col(mt + b) + lo;
+          double v = 0.0;
+          for (int r = 0; r < nr; r++) v = fma(x[r], y[r], v);
+          out[i] += v;
+        }
+      }
+      __syncthreads();
+      continue;
+    }
+    long long hi[4][4], cr[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) hi[i][j] = cr[i][j] = 0;
+    if (sl < ks) {
+      for (int r = 2 * sl; r < nr;) {
+        const int end = min(nr, r + 16 * ks);
+#pragma unroll 2
+        for (; r < end; r += 2 * ks) {
+          int4 a[4], b[4];
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            a[i] = *reinterpret_cast<const int4 *>(sx + pa[i] + r);
+            b[i] = *reinterpret_cast<const int4 *>(sx + pb[i] + r);
+          }
+#pragma unroll
+          for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+              hi[i][j] += (long long)a[i].y * b[j].y;
+              cr[i][j] += (long long)a[i].x * b[j].y;
+              cr[i][j] += (long long)a[i].y * b[j].x;
+              hi[i][j] += (long long)a[i].w * b[j].w;
+              cr[i][j] += (long long)a[i].z * b[j].w;
+              cr[i][j] += (long long)a[i].w * b[j].z;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            hi[i][j] += cr[i][j] >> kQLow;
+            cr[i][j] &= (1 << kQLow) - 1;
+          }
+      }
+    }
+    __syncthreads();
+    // the slices' sums, in integers (rounded: a bias would add up over the chunks)
+    long long *red = reinterpret_cast<long long *>(sx);
+    if (sl < ks)
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+          red[((sl * 4 + i) * 4 + j) * nq + q] = hi[i][j] + (cr[i][j] >> (kQLow - 1));
+    __syncthreads();
+    if (sl < 4) {
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        long long t = 0;
+        for (int k = 0; k < ks; k++) t += red[((k * 4 + i) * 4 + sl) * nq + q];
+        const int a = min(ga + i * GA, mt - 1), b = mt + min(gb + sl * GB, pt - 1);
+        out[i] += sb::fromfix(t, 2 * kQLow - sp[a] - sp[b]);
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int a = ga + i * GA, b = gb + sl * GB;
+    if (sl < 4 && a < mt && b < pt)
+      part[((long)blockIdx.x * m + ta + a) * p + tb + b] = out[i];
+  }
 }
 
 // W[r, b0 + b] += alpha * sum_a V[r, a0 + a] C[a][b] over rows [r0, r1)
@@ -137,6 +310,135 @@ k_update(double *__restrict__ V, long ld, long r0, long r1, int a0, int m, int b
         *w = fma(alpha, acc[b], *w);
       }
   }
+}
+
+// a b + c, one instruction: left to itself the compiler widens the row's halves
+// once and multiplies 64 x 64 bits (187488 rows, 48 x 16: 150 us against 95)
+__device__ __forceinline__ long long qmad(int a, int b, long long c) {
+  asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(c) : "r"(a), "r"(b));
+  return c;
+}
+
+// The same update in block fixed point, NB columns of W per pass.  The
+// coefficients come as 58-bit integers C'[a][b] 2^pc[b] in halves, where
+// C' = C 2^-da[a] has entries of about one in every row, and the row's scaled
+// entries V 2^da share a power of two, so that neither badly scaled columns
+// nor the range over the rows (wavenumbers) lose digits.  Three multiply-adds
+// a product as above; at most 64 products meet in one sum.  Rows with an
+// infinity, a NaN or numbers beyond 2^+-400 take the FP64 sums.  The rows come
+// by asynchronous copies, a thread its own, before the scale is taken.
+template <int NB>
+__global__ void __launch_bounds__(kUThreads)
+k_updateq(double *__restrict__ V, long ld, long r0, long r1, int a0, int m, int b0, int p,
+          const double *__restrict__ C, const int2 *__restrict__ CQ, const int *__restrict__ da,
+          const int *__restrict__ pc, double alpha) {
+  extern __shared__ __align__(16) int2 sx[];
+  const int mx = min(m, 64);
+  int2 *sc = sx;                                 // coefficients [mx][NB]
+  double *sv = (double *)(sx + mx * NB);         // rows of V [mx][kUThreads]
+  int *sd = (int *)(sv + mx * kUThreads);        // exponents [mx]
+  const int pp = (p + NB - 1) / NB * NB;
+  const long r = r0 + (long)blockIdx.x * kUThreads + threadIdx.x;
+  const int g = blockIdx.y * NB, nb = min(NB, p - g);
+  const bool on = r < r1;
+  for (int c0 = 0; c0 < m; c0 += 64) {
+    const int mc = min(64, m - c0);
+    const double *v = V + (long)(a0 + c0) * ld + (on ? r : r1 - 1);
+    __syncthreads();
+#pragma unroll 8
+    for (int a = 0; a < mc; a++) copy8(sv + a * kUThreads + threadIdx.x, v + (long)a * ld, on);
+    for (int k = threadIdx.x; k < mc * NB; k += kUThreads)
+      sc[k] = CQ[(long)(c0 + k / NB) * pp + g + k % NB];
+    for (int k = threadIdx.x; k < mc; k += kUThreads) sd[k] = da[c0 + k];
+    copy_wait();
+    __syncthreads();
+    if (!on) continue;
+    double *w = V + (long)(b0 + g) * ld + r;
+    const double *mv = sv + threadIdx.x;
+    int top = -100000, raw = 0;
+#pragma unroll 8
+    for (int a = 0; a < mc; a++) {
+      const int e = (int)(sb::hiword(mv[a * kUThreads]) >> 20);
+      raw = max(raw, e);
+      if (e) top = max(top, e + sd[a]);
+    }
+    if (raw == 0x7ff || top > 1023 + kQLim || top < 1023 - kQLim) {
+      for (int b = 0; b < nb; b++) {
+        double acc = 0.0;
+        for (int a = 0; a < mc; a++)
+          acc = fma(mv[a * kUThreads], C[(long)(c0 + a) * p + g + b], acc);
+        w[(long)b * ld] = fma(alpha, acc, w[(long)b * ld]);
+      }
+      continue;
+    }
+    const int pr = kQBits - (top - 1022);
+    long long hi[NB], cr[NB];
+#pragma unroll
+    for (int b = 0; b < NB; b++) hi[b] = cr[b] = 0;
+    for (int a = 0; a < mc;) {
+      const int end = min(mc, a + 16);
+#pragma unroll 2
+      for (; a < end; a++) {
+        sb::QScale s;
+        s.p = pr + sd[a];
+        const int2 x = qsplit(sb::tofix(mv[a * kUThreads], s));
+#pragma unroll
+        for (int b = 0; b < NB; b += 2) {
+          const int4 c = *reinterpret_cast<const int4 *>(sc + a * NB + b);
+          hi[b] = qmad(x.y, c.y, hi[b]);
+          cr[b] = qmad(x.x, c.y, cr[b]);
+          cr[b] = qmad(x.y, c.x, cr[b]);
+          hi[b + 1] = qmad(x.y, c.w, hi[b + 1]);
+          cr[b + 1] = qmad(x.x, c.w, cr[b + 1]);
+          cr[b + 1] = qmad(x.y, c.z, cr[b + 1]);
+        }
+      }
+#pragma unroll
+      for (int b = 0; b < NB; b++) {
+        hi[b] += cr[b] >> kQLow;
+        cr[b] &= (1 << kQLow) - 1;
+      }
+    }
+    // hi < 2^(56 + bits of mc): the sum as one integer, 2^(60 - up)
+    const int up = mc > 32 ? 0 : mc > 16 ? 1 : mc > 8 ? 2 : 3;
+#pragma unroll
+    for (int b = 0; b < NB; b++)
+      if (b < nb) {
+        const long long t = (hi[b] << up) + ((cr[b] + (1ll << (kQLow - 1 - up))) >> (kQLow - up));
+        const double acc = sb::fromfix(t, 2 * kQLow - up - pr - pc[g + b]);
+        w[(long)b * ld] = fma(alpha, acc, w[(long)b * ld]);
+      }
+  }
+}
+
+// the coefficients' integers and exponents for k_updateq; false where a
+// number is not finite or too far from one
+bool fix_coefs(const double *C, int m, int p, int pp, int2 *q, int *da, int *pc) {
+  std::vector<int> top(p, -100000);
+  for (int a = 0; a < m; a++) {
+    int e = 0;
+    for (int b = 0; b < p; b++) e = std::max(e, (int)(sb::hiword(C[(long)a * p + b]) >> 20));
+    if (e && std::abs(e - 1023) > kQLim) return false;
+    da[a] = e ? e - 1023 : -20000;  // a row of zeros weighs nothing
+    for (int b = 0; b < p; b++) {
+      const int x = (int)(sb::hiword(C[(long)a * p + b]) >> 20);
+      if (x) top[b] = std::max(top[b], x - da[a]);
+    }
+  }
+  for (int b = 0; b < p; b++) {
+    if (top[b] < 0) top[b] = 1023;
+    if (top[b] < 1023 - kQLim) return false;
+    pc[b] = kQBits - (top[b] - 1022);
+  }
+  for (int a = 0; a < m; a++)
+    for (int b = 0; b < pp; b++) {
+      sb::QScale s{};
+      if (b < p) s.p = pc[b] - da[a];
+      const long long v = b < p && da[a] != -20000 ? sb::tofix(C[(long)a * p + b], s) : 0;
+      const long long lo = ((v & ((1ll << kQLow) - 1)) ^ (1ll << (kQLow - 1))) - (1ll << (kQLow - 1));
+      q[(long)a * pp + b] = make_int2((int)lo, (int)((v - lo) >> kQLow));
+    }
+  return true;
 }
 
 // W[r, b0 + b] = sum_a W[r, b0 + a] M[a][b] (in place, p <= 64 columns)
@@ -332,6 +634,42 @@ long chunk_rows(long rows, long *nchunk) {
   return ch;
 }
 
+// the row split of k_gramq: slices of a chunk, blocks, shared memory
+void gramq_plan(long rows, int m, int p, int *ks, int *nblk, size_t *smem) {
+  const int mt = std::min(m, kQA), pt = std::min(p, kQB);
+  const int nq = ((mt + 3) / 4) * ((pt + 3) / 4);
+  // the fewest warp passes over a chunk's row pairs
+  long best = 0;
+  for (int k = 4; k <= 32 && k * nq <= kThreads; k++) {
+    const long c = (long)((nq * k + 31) / 32) * ((kQR / 2 + k - 1) / k);
+    if (!best || c < best) {
+      best = c;
+      *ks = k;
+    }
+  }
+  const int tiles = ((m + kQA - 1) / kQA) * ((p + kQB - 1) / kQB);
+  const long chunks = (rows + kQR - 1) / kQR, slots = std::max(1, 2 * 152 / tiles);
+  // as many chunks to every block
+  const long each = (chunks + slots - 1) / slots;
+  *nblk = (int)((chunks + each - 1) / each);
+  *smem = std::max(sizeof(int2) * (size_t)(mt + pt) * kQS, sizeof(long long) * 16 * nq * *ks);
+}
+constexpr int kGramSmem = (int)sizeof(int2) * (kQA + kQB) * kQS;
+constexpr int kUpdSmem = 64 * (16 * (int)sizeof(int2) + kUThreads * (int)sizeof(double) + 4);
+cudaError_t prepare_fixed() {
+  constexpr auto A = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  cudaError_t e = cudaFuncSetAttribute(k_gramq, A, kGramSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_updateq<4>, A, kUpdSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_updateq<8>, A, kUpdSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_updateq<16>, A, kUpdSmem);
+  return e;
+}
+// The fixed-point forms from 16 coefficients on.  187488 rows, whole calls,
+// FP64 against fixed point: products 48 x 16 489 -> 144 us, 32 x 1 179 -> 80,
+// 16 x 2 118 -> 57, 4 x 4 the same (56); updates 260 -> 100, 106 -> 37,
+// 63 -> 26, 27 -> 18.  Below, the conversions cost what the sums save.
+bool fixed_ok(int m, int p) { return (long)m * p >= 16; }
+
 }  // namespace
 
 namespace sb {
@@ -433,6 +771,7 @@ int sb_kspace_create(long n, int cols, void *stream, sb_kspace **out) {
   cudaGetDevice(&ks->dev);
   cudaError_t e = cudaMalloc((void **)&ks->V, sizeof(double) * (size_t)ks->ld * cols);
   if (e == cudaSuccess) e = cudaMemset(ks->V, 0, sizeof(double) * (size_t)ks->ld * cols);
+  if (e == cudaSuccess) e = prepare_fixed();
   if (e == cudaSuccess && !stream) {
     e = cudaStreamCreateWithFlags(&ks->st, cudaStreamNonBlocking);
     ks->own_stream = true;
@@ -472,9 +811,17 @@ int sb_kspace_gram(sb_kspace *ks, long r0, long r1, int a0, int m, int b0, int p
   if ((rc = check_rows(ks, r0, r1)) || (rc = check_cols(ks, a0, m)) || (rc = check_cols(ks, b0, p)))
     return rc;
   if (m == 0 || p == 0) return 0;
-  long nchunk;
   const long rows = r1 - r0;
-  const long ch = chunk_rows(rows > 0 ? rows : 1, &nchunk);
+  const bool fixed = fixed_ok(m, p) && rows > 0;
+  long nchunk, ch = 0;
+  int slices = 0, qblk = 0;
+  size_t smem = 0;
+  if (fixed) {
+    gramq_plan(rows, m, p, &slices, &qblk, &smem);
+    nchunk = qblk;
+  } else {
+    ch = chunk_rows(rows > 0 ? rows : 1, &nchunk);
+  }
   const long need = nchunk * (long)m * p;
   if (need > ks->part_cap) {
     if (ks->part) cudaFree(ks->part);
@@ -484,12 +831,18 @@ int sb_kspace_gram(sb_kspace *ks, long r0, long r1, int a0, int m, int b0, int p
     ks->part_cap = need;
   }
   if ((rc = ensure_small(ks, (long)m * p))) return rc;
-  const dim3 grid((unsigned)nchunk, (unsigned)((m + kTA - 1) / kTA), (unsigned)((p + kTB - 1) / kTB));
-  if (grid.y > 65535 || grid.z > 65535) return kfail(1, "sb_kspace_gram: block too large");
-  k_gram<<<grid, kThreads, 0, ks->st>>>(ks->V, ks->ld, r0, r1, ch, a0, m, b0, p, ks->part);
+  const int ca = fixed ? kQA : kTA, cb = fixed ? kQB : kTB;
+  const dim3 grid((unsigned)nchunk, (unsigned)((m + ca - 1) / ca), (unsigned)((p + cb - 1) / cb));
+  if ((m + kTA - 1) / kTA > 65535 || (p + kTB - 1) / kTB > 65535)
+    return kfail(1, "sb_kspace_gram: block too large");
+  if (fixed)
+    k_gramq<<<grid, kThreads, smem, ks->st>>>(ks->V, ks->ld, r0, r1, slices, a0, m, b0, p,
+                                              ks->part);
+  else
+    k_gram<<<grid, kThreads, 0, ks->st>>>(ks->V, ks->ld, r0, r1, ch, a0, m, b0, p, ks->part);
   KCK(cudaGetLastError());
-  k_gram_sum<<<(unsigned)((m * p + 255) / 256), 256, 0, ks->st>>>(ks->part, (int)nchunk, m, p,
-                                                                   ks->small);
+  k_gram_sum<<<(unsigned)((m * p + 31) / 32), dim3(32, 32), 0, ks->st>>>(ks->part, (int)nchunk, m,
+                                                                         p, ks->small);
   KCK(cudaGetLastError());
   KCK(cudaMemcpyAsync(ks->hsmall, ks->small, sizeof(double) * m * p, cudaMemcpyDeviceToHost,
                       ks->st));
@@ -506,14 +859,36 @@ int sb_kspace_update(sb_kspace *ks, long r0, long r1, int a0, int m, int b0, int
     return rc;
   if (a0 < b0 + p && b0 < a0 + m) return kfail(1, "sb_kspace_update: overlapping column ranges");
   if (m == 0 || p == 0 || r1 == r0) return 0;
-  if ((rc = ensure_small(ks, (long)m * p))) return rc;
+  const int nb = p > 8 ? 16 : p > 4 ? 8 : 4, pp = (p + nb - 1) / nb * nb;
+  const bool fixed = fixed_ok(m, p) && pp / nb <= 65535;
+  // the coefficients, and their integers (int2 [m][pp]), da [m] and pc [p]
+  const long mp = (long)m * p, oq = (mp + 1) / 2 * 2, oe = oq + (long)m * pp;
+  const long count = fixed ? oe + (m + p + 1) / 2 : mp;
+  if ((rc = ensure_small(ks, count))) return rc;
   // the staging buffer may still feed an earlier update: wait for the stream
   KCK(cudaStreamSynchronize(ks->st));
-  for (long q = 0; q < (long)m * p; q++) ks->hsmall[q] = C[q];
-  KCK(cudaMemcpyAsync(ks->small, ks->hsmall, sizeof(double) * m * p, cudaMemcpyHostToDevice,
-                      ks->st));
-  k_update<<<(unsigned)((r1 - r0 + kThreads - 1) / kThreads), kThreads, 0, ks->st>>>(
-      ks->V, ks->ld, r0, r1, a0, m, b0, p, ks->small, alpha);
+  for (long q = 0; q < mp; q++) ks->hsmall[q] = C[q];
+  int *he = (int *)(ks->hsmall + oe);
+  const bool fix = fixed && fix_coefs(C, m, p, pp, (int2 *)(ks->hsmall + oq), he, he + m);
+  KCK(cudaMemcpyAsync(ks->small, ks->hsmall, sizeof(double) * (fix ? count : mp),
+                      cudaMemcpyHostToDevice, ks->st));
+  if (fix) {
+    const dim3 grid((unsigned)((r1 - r0 + kUThreads - 1) / kUThreads), (unsigned)(pp / nb));
+    const int *e = (const int *)(ks->small + oe);
+    const int2 *cq = (const int2 *)(ks->small + oq);
+    const int mx = std::min(m, 64);
+    const size_t smem = sizeof(int2) * mx * nb + sizeof(double) * mx * kUThreads + sizeof(int) * mx;
+#define SB_UPD(NB)                                                                              \
+  k_updateq<NB><<<grid, kUThreads, smem, ks->st>>>(ks->V, ks->ld, r0, r1, a0, m, b0, p, ks->small, \
+                                                   cq, e, e + m, alpha)
+    if (nb == 16) SB_UPD(16);
+    else if (nb == 8) SB_UPD(8);
+    else SB_UPD(4);
+#undef SB_UPD
+  } else {
+    k_update<<<(unsigned)((r1 - r0 + kThreads - 1) / kThreads), kThreads, 0, ks->st>>>(
+        ks->V, ks->ld, r0, r1, a0, m, b0, p, ks->small, alpha);
+  }
   KCK(cudaGetLastError());
   return 0;
 }
