@@ -25,7 +25,7 @@ UNITS = [("sb_kernels.cu", ["-DSB_FLOAT_TU=0"]), ("sb_kernels.cu", ["-DSB_FLOAT_
          *[("sb_planeq.cu", [f"-DSB_PLANE={k}", f"-DSB_TEMP={t}"]) for k in (0, 1)
            for t in (0, 1)],
          # the Bloch-wave form once per (precision, range of line lengths, branch)
-         *[("sb_bloch.cu", [f"-DSB_FLOAT_TU={f}", f"-DSB_LEN={k}", f"-DSB_IMPL={i}"])
+         *[("sb_bloch.cu", [f"-DSB_FLOAT_TU={f}", f"-DSB_LEN={k}", f"-DSB_GEN={i}"])
            for k in (0, 1, 2) for f in (0, 1) for i in (0, 1)],
          ("sb_box.cu", []), ("sb_implicit.cu", []),
          ("sb_ops.cu", []), ("sb_noalloc.cu", []), ("sb_api.cu", []), ("sb_krylov.cu", []),

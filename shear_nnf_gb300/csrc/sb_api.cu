@@ -446,11 +446,11 @@ static int build_bloch_tables(sb_handle *h) {
   double *q;
   if ((rc = dalloc(h, &q, 2 * m))) return rc;
   bf.btw = (qw *)q;
-  if ((rc = dalloc(h, &q, 2 * (size_t)g.B * g.field))) return rc;
+  if ((rc = dalloc(h, &q, (2 + g.temp) * (size_t)g.B * g.field))) return rc;
   bf.bw = (q2 *)q;
-  if ((rc = dalloc(h, &q, 4 * (size_t)g.B * n))) return rc;
+  if ((rc = dalloc(h, &q, (1 + g.temp) * 4 * (size_t)g.B * n))) return rc;
   bf.bwm = (q2 *)q;
-  if ((rc = dalloc(h, &q, (size_t)g.B * (g.plane / 2 + 2)))) return rc;
+  if ((rc = dalloc(h, &q, (size_t)(2 + g.temp) * g.B * (g.plane / 2 + 2) / 2 + 1))) return rc;
   bf.bwp = (int *)q;
   if ((rc = dalloc(h, &q, 2 * (m / 3)))) return rc;
   bf.bm1 = (double2 *)q;

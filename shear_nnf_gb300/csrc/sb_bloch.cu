@@ -12,6 +12,11 @@
 //            t + c_k dt -> v = lapcdy(phi) -> G, dv/dy -> V
 //   omega_y  nu (d2/dy2 - k^2) omega_y, update, remap; d(omega_y)/dy -> D
 //   mean     the same for u00 and w00 (nu d2/dy2, forcing, update, d/dy)
+// and with the temperature, in a launch of its own after these,
+//   tb       d(-vT)/dy + kappa lap(tb), update, remap (crosst.f90:633-636,
+//            734-872); gbeta lap(tb) -> Lt, the buoyancy in the phi line of the
+//            next substep (whose launch comes first, so Lt is complete)
+//   tb00     the same for the mean profile
 // with the transforms in 64-bit fixed point (sb_fix.cuh): six (phi) or four
 // (omega_y) transforms of my points per line at some 80 integer instructions
 // per point, where the banded solves (sb_seg.cuh) spend six solves of 46 FP64
@@ -25,21 +30,23 @@
 // the inverse ones that follow it.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "sb_common.cuh"
 #include "sb_fix.cuh"
 #include "sb_kernels.h"
 
 // Compiled twelve times: SB_FLOAT_TU = 0 (FP64) or 1 (FP32-mixed) storage times
-// SB_LEN = 0 (my 32..80), 1 (96..192), 2 (256..384) times SB_IMPL = 0 (explicit)
-// or 1 (semi-implicit viscous branch); unit (0, 0, 0) also holds the entry points.
+// SB_LEN = 0 (my 32..80), 1 (96..192), 2 (256..384) times SB_GEN = 0 (explicit,
+// no temperature) or 1 (the rest); unit (0, 0, 0) also holds the entry points.
 #ifndef SB_FLOAT_TU
 #define SB_FLOAT_TU 0
 #endif
 #ifndef SB_LEN
 #define SB_LEN 0
 #endif
-#ifndef SB_IMPL
-#define SB_IMPL 0
+#ifndef SB_GEN
+#define SB_GEN 0
 #endif
 #define SB_CAT2(a, b, c, d) a##b##_##c##_##d
 #define SB_CAT(a, b, c, d) SB_CAT2(a, b, c, d)
@@ -154,14 +161,16 @@ struct LineQRegs {
 // instruction cache, and each warp runs it only once): pass 0 takes the
 // right-hand side and the update at the phase of time t, pass 1 the outputs at
 // the phase of t + c_k dt.  A pass: rows in, forward, products, inverse, rows out.
-// IM: the semi-implicit viscous branch (explicit = 0, cross.f90:797-989).  Pass 0
+// GEN: with the temperature, the semi-implicit branch or both (kept apart: their
+// branches cost the plain step 3%).  The semi-implicit viscous branch (explicit = 0, cross.f90:797-989).  Pass 0
 // gives the viscous term and (phi) -d(D)/dy apart, the update forms the
 // right-hand side -Re ibeta_k (wk + alpha_k nu lap f + f/Dt) of the Helmholtz
 // equation in the frame of t + c_k Dt, and pass 1 solves it on the waves,
 // f = rhs/(l2 - k^2 - Re ibeta_k/Dt), before the outputs; the state is one
 // more output.  The (0,0) line keeps its state.
-template <typename R, int N, int T, bool IM>
-__global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid g, Bufs bf, int rk1) {
+template <typename R, int N, int T, bool GEN>
+__global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid g, Bufs bf, int rk1,
+                                                                              int role0) {
   typedef LineQ<N> L;
   typedef typename V2<R>::t V;
   constexpr int R1 = L::R1, R2 = L::R2;
@@ -173,18 +182,21 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
   q2 *const ex = (q2 *)smq_raw;              // two buffers of N x kCols
   double *const sc = (double *)(ex + 2 * N * kCols);  // factors of the waves
   __shared__ unsigned s_top[2][kCols];  // largest upper words: D, the new state
-  // scales of the products: right-hand side, first, second output; IM: the
-  // second of pass 0, the Helmholtz solve
-  constexpr int kLens = IM ? 5 : 3;
+  // scales of the products: right-hand side, first, second output; semi-implicit:
+  // the second of pass 0, the Helmholtz solve
+  constexpr int kLens = GEN ? 5 : 3;
   __shared__ int s_len[kLens][kCols];
   const int ncb = (g.nkx + kCols - 1) / kCols, per = g.mz * ncb;
-  const int role = blockIdx.x / per;  // 0 phi, 1 omega_y, 2 mean
-  const int r = blockIdx.x - role * per;
-  const bool mean = role == 2;
+  // role0 = 0: 0 phi, 1 omega_y, 2 mean; role0 = 3: 3 tb, 4 tb00
+  const int slot = blockIdx.x / per, role = GEN ? role0 + slot : slot;
+  const int r = blockIdx.x - slot * per;
+  const bool mean = role == 2 || (GEN && role == 4), scal = GEN && role >= 3;
+  const bool im = GEN && g.impl;
+  const bool din = role == 0 || scal;  // a second field in pass 0, D or -vT
   const int ci = threadIdx.x & (kCols - 1), n = threadIdx.x / kCols;
   const int k = mean ? 0 : r / ncb;
   const int i0 = mean ? ci : (r - k * ncb) * kCols + ci;
-  const bool act = mean ? ci < 2 : i0 < g.nkx;
+  const bool act = mean ? ci < (scal ? 1 : 2) : i0 < g.nkx;
   const int cm = ci & 1;  // mean: u00 in column 0, w00 in column 1
   const int i = mean ? 0 : (act ? i0 : g.nkx - 1);
   const bool is00 = !mean && i == 0 && k == 0;
@@ -202,16 +214,19 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
   const double a = g.alp * i, gz = g.gam * ((k <= g.nz) ? k : k - g.mz);
   const double k2 = mean ? 0.0 : a * a + gz * gz;
   const double Dt = M.Deltat;
-  // of the viscous term of pass 0, and for IM the scales of the right-hand side
-  const double nu = is00 ? 0.0 : IM && rk1 > 0 ? kAlpha[rk] * M.nu : M.nu, nuk2 = nu * k2;
-  const double fb = IM && rk1 > 0 ? -M.Re * kIbeta[rk] : 0.0, rdt = IM ? 1.0 / Dt : 0.0;
-  V *f = (V *)(role == 0 ? bf.phi : bf.vor) + off;
-  R *mf = (R *)bf.mu + (long)b * 2 * N + cm;  // mean profile of this column
+  // of the viscous term of pass 0, and the semi-implicit right-hand side's scales
+  const double mnu = scal ? g.kappa : M.nu;
+  const double nu = is00 ? 0.0 : im && rk1 > 0 ? kAlpha[rk] * mnu : mnu;
+  const double fb = im && rk1 > 0 ? -(scal ? 1.0 / g.kappa : M.Re) * kIbeta[rk] : 0.0, rdt = im ? 1.0 / Dt : 0.0;
+  V *f = (V *)(scal ? bf.tb : role == 0 ? bf.phi : bf.vor) + off;
+  R *mf = (R *)(scal ? bf.mt : bf.mu) + (long)b * 2 * N + cm;  // mean profile of this column
   // the waves of the state, kept from pass 1 for the next substep's pass 0 (the
   // same phase), and their scale
   const long wst = mean ? 2 : ps, nl = ps + 2;
-  q2 *waves = mean ? bf.bwm + (long)b * 2 * N + cm : bf.bw + role * (g.B * (g.field / 2)) + off;
-  int *wscale = bf.bwp + ((long)role % 2 * g.B + b) * nl + (mean ? ps + cm : (long)k * nkx + i);
+  q2 *waves = mean ? bf.bwm + (long)(scal * g.B + b) * 2 * N + cm
+                   : bf.bw + (scal ? 2 : role) * (g.B * (g.field / 2)) + off;
+  int *wscale = bf.bwp + ((long)(scal ? 2 : role & 1) * g.B + b) * nl +
+                (mean ? ps + cm : (long)k * nkx + i);
 #pragma unroll 1
   for (int ph = rk1 > 0 ? 0 : 1; ph < 2; ph++) {
     // phase tables: slot 0 holds the phases of a step's start, slots 1 and 2
@@ -219,17 +234,17 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
     const long o = ((long)((ph == 0 ? rk : rk1) % 3) * g.B + b) * tb + i;
     const qw *tw = bf.btw + o;
     const double *l1 = bf.bl1 + o, *l2 = bf.bl2 + o;
-    const int nf = ph == 0 && role == 0 ? 2 : 1;  // fields in: the state, D
-    const int no = (IM || ph == 1) && role == 0 ? 2 : 1;  // fields out
+    const int nf = ph == 0 && din ? 2 : 1;  // fields in: the state, D
+    const int no = (im && ph == 0 && din) || (ph == 1 && role == 0) ? 2 : 1;  // fields out
     // ---- rows in: D to buffer 1 (phi, pass 0), the state of the start of a run
     // to buffer 0 (in pass 1 the new state is there already)
-    const bool rows = ph == 1 || role == 0;
-    if (ph == 0 ? role == 0 : rk1 == 0) {
-      const V *src = ph == 0 ? (const V *)bf.Dn + off : f;
+    const bool rows = ph == 1 || din;
+    if (ph == 0 ? din : rk1 == 0) {
+      const V *src = ph == 0 ? (const V *)(scal ? bf.R2 : bf.Dn) + off : f;
       unsigned top = 0;
 #pragma unroll 4
       for (int j = n; j < N; j += T / kCols) {
-        const V w = mean ? mkv<R>(mf[2 * j], (R)0) : src[(long)j * ps];
+        const V w = mean && ph == 1 ? mkv<R>(mf[2 * j], (R)0) : src[(long)j * ps];
         *(V *)(ex + ((1 - ph) * N + j) * kCols + ci) = w;
         top = max(top, vtop(w));
       }
@@ -249,11 +264,11 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
       __syncthreads();
     }
     const int eb = L::kShiftF + Plan<N>::shift + 2 - kN - kTgt;
-    const bool solve = IM && ph == 1 && rk1 > 0;
-    if constexpr (IM) {
+    const bool solve = im && ph == 1 && rk1 > 0;
+    if constexpr (GEN) {
       if (solve) {
         // ---- the Helmholtz solve; the waves of the new state stay in buffer 0
-        const double dtr = M.Re * kIbeta[rk] * rdt;
+        const double dtr = -fb * rdt;
 #pragma unroll 1
         for (int k1 = n; k1 < R1; k1 += T / kCols) {
           const double *l = l2 + (long)k1 * nkx;
@@ -265,7 +280,7 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
           int la = kNoLen;
 #pragma unroll
           for (int w = 0; w < R2; w++) {
-            const double c = is00 ? 1.0 : recip(l[(long)(R1 * w) * nkx] - k2 - dtr);
+            const double c = recip(is00 ? 1.0 : l[(long)(R1 * w) * nkx] - k2 - dtr);
             sc[(k1 * R2 + w) * kCols + ci] = c;
             e[w * kCols] = x[w];
             la = max(la, qlen(x[w]) + qexp(c));
@@ -306,6 +321,7 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
         w0 += sh;
       }
     }
+    const double cn = ph == 0 ? nu : is00 ? 0.0 : g.gbeta, cnk2 = cn * k2;
     // ---- products.  Pass 0: nu (l2 - k^2) f - i l1 D; pass 1: phi f/(l2 - k^2)
     // and i l1 of it, else i l1 f.  The waves stay in the thread's own slots
     // while the scale of each product is found over the whole line.
@@ -313,15 +329,23 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
     for (int k1 = n; k1 < R1; k1 += T / kCols) {
       const long p0 = (long)k1 * nkx;
       double *cw = sc + k1 * R2 * kCols + ci;
-      // nu (l2 - k^2), 1/(l2 - k^2) or l1
+      // nu (l2 - k^2) or gbeta (l2 - k^2), 1/(l2 - k^2), l1: three arms that the
+      // compiler turns into selects, so that the waves' loads and chains overlap
+      // (with a fourth, or the reciprocal inlined from a function, it branched
+      // for each wave: 64x32x32 29 us against 23)
 #pragma unroll
       for (int q = 0; q < R2; q++) {
         const long p = p0 + (long)(R1 * q) * nkx;
         double c;
-        if (ph == 0) {
-          c = fma(nu, l2[p], -nuk2);
+        if (ph == 0 || scal) {
+          c = fma(cn, l2[p], -cnk2);
         } else if (role == 0) {
-          c = is00 ? 0.0 : recip(l2[p] - k2);
+          const double den = l2[p] - k2;
+          double z;
+          asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(z) : "d"(den));
+          z = fma(z, fma(-den, z, 1.0), z);
+          z = fma(z, fma(-den, z, 1.0), z);
+          c = is00 ? 0.0 : z;
         } else {
           c = l1[p];
         }
@@ -354,15 +378,15 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
           la = max(la, len + (q ? e1 : ec));
           lb = max(lb, len + ec + e1 + 1);
         }
-        atomicMax(&s_len[IM && ph == 0 && q ? 3 : ph][ci], la - (ph == 0 ? (q ? w1 : w0) : 0));
+        atomicMax(&s_len[im && ph == 0 && q ? 3 : ph][ci], la - (ph == 0 ? (q ? w1 : w0) : 0));
         if (ph == 1 && no > 1) atomicMax(&s_len[2][ci], lb);
       }
       if (ph == 1 && k1 == 0 && act) *wscale = bad ? kNoLen : w0;
     }
     __syncthreads();
     // scales of the outputs; in pass 0 of the sum of two terms
-    const int len1 = s_len[ph][ci] + (!IM && ph == 0 ? 2 : 1);
-    const int len2 = s_len[IM && ph == 0 ? 3 : 2][ci] + 1;
+    const int len1 = s_len[ph][ci] + (!im && ph == 0 ? 2 : 1);
+    const int len2 = s_len[GEN && ph == 0 ? 3 : 2][ci] + 1;
 #pragma unroll 1
     for (int k1 = n; k1 < R1; k1 += T / kCols) {
       const double *cw = sc + k1 * R2 * kCols + ci;
@@ -383,8 +407,9 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
             d = ph == 1 ? d * m : m;
           }
           q2 z = qscaled(e[w * kCols], d, sh);
-          // times -i (D), i (d/dy of an output) or 1
-          if (ph == 0 ? q : (role != 0 || q)) z = ph == 0 ? qrot<-1>(z) : qrot<1>(z);
+          // times -i (D), i (-vT, d/dy of an output) or 1
+          if (ph == 0 ? q : (role == 1 || role == 2 || q))
+            z = ph == 0 && !scal ? qrot<-1>(z) : qrot<1>(z);
           y[w] = first ? z : y[w] + z;
         }
         if (no > 1 || q == 0) {
@@ -408,6 +433,7 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
       const bool nan1 = bad || qrange(e0 + len1), nan2 = bad || qrange(e0 + len2);
       const R nn = (R)nan("");
       if (mean) {
+        if (scal) return;
         R *dst = (R *)bf.mdu + (long)b * 2 * N + cm;
         if (act)
 #pragma unroll 1
@@ -418,7 +444,7 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
         for (int q = 0; q < no; q++) {
           // the (0,0) line of v keeps the value zero it is given at the start of a run
           if (role == 0 && q == 0 && is00 && rk1 > 0) continue;
-          V *dst = (V *)(role != 0 ? bf.D : q ? bf.V : bf.G) + off;
+          V *dst = (V *)(scal ? bf.Lt : role != 0 ? bf.D : q ? bf.V : bf.G) + off;
           const int eo = e0 + (q ? len2 : len1);
           const bool none = q ? nan2 : nan1;
 #pragma unroll 2
@@ -432,20 +458,20 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
     }
     // RK3 accumulation and update, zeta store, remaps (cross.f90:694-781)
     const int eo = eb + len1;
-    const int ed = eb + len2;  // IM: of -d(D)/dy
-    const bool nanr = bad || qrange(eo) || (IM && no > 1 && qrange(ed));
+    const int ed = eb + len2;  // semi-implicit: of -d(D)/dy
+    const bool nanr = bad || qrange(eo) || (im && no > 1 && qrange(ed));
     const R gk = (R)kGama[rk], zk = (R)kZeta[rk], dtr = (R)Dt;
     unsigned top = 0;
     if (mean) {
-      R *mwk = (R *)bf.mwk + (long)b * 2 * N + cm;
+      R *mwk = (R *)(scal ? bf.mtwk : bf.mwk) + (long)b * 2 * N + cm;
       const R *mrf = (const R *)bf.mrf + (long)b * 2 * N + cm;
-      const bool damp = g.damp && ci == 0, xf = g.force == -1 && ci == 0;
+      const bool damp = g.damp && ci == 0 && !scal, xf = g.force == -1 && ci == 0 && !scal;
 #pragma unroll 1
       for (int j = n; j < N; j += T / kCols) {
         R un = (R)0;
         if (act) {
           // forcing and damping (cross.f90:622-626; operators.f90:60-78)
-          R rf0 = mrf[2 * j];
+          R rf0 = scal ? (R)0 : mrf[2 * j];
           if (xf) rf0 = (R)((double)rf0 + g.xforce);
           if (damp) {
             const double y = (double)j * g.dy - 0.5 * g.Ly;
@@ -454,7 +480,8 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
             rf0 = (R)((double)rf0 - g.damp_up * hw * (double)mf[2 * j]);
           }
           const ll z = ex[j * kCols + ci].x;
-          if constexpr (IM) {
+          if (im) {
+            if (scal) rf0 = nanr ? (R)nan("") : qout<R>(ex[(N + j) * kCols + ci].x, ed);
             const R wk = (rk == 0) ? gk * rf0 : mwk[2 * j] + gk * rf0;
             const double vis = nanr ? nan("") : fromfix(z, eo);
             un = (R)(fb * (((double)wk + vis) + rdt * (double)mf[2 * j]));
@@ -473,47 +500,68 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
         *(V *)(ex + j * kCols + ci) = w;
       }
     } else {
-      const V *rhs = (const V *)(role == 0 ? bf.V : bf.Gn) + off;
-      V *fwk = (V *)(role == 0 ? bf.phiwk : bf.vorwk) + off;
+      const V *rhs = (const V *)(scal ? bf.Ht : role == 0 ? bf.V : bf.Gn) + off;
+      V *fwk = (V *)(scal ? bf.tbwk : role == 0 ? bf.phiwk : bf.vorwk) + off;
       const double2 *m1 = bf.bm1 + (long)b * tb + i, *m2 = bf.bm2 + (long)b * tb + i;
       const V none = mkv<R>((R)0, (R)0);
+      const V *buoy = (const V *)bf.Lt + off;
+      // one loop for each form: a branch inside waits for every row's loads
+      auto update = [&](auto with, auto implicit) {
+        constexpr bool IM = decltype(implicit)::value;
 #pragma unroll 2
-      for (int j = n; j < N; j += T / kCols) {
-        const long q = (long)j * ps;
-        const V fo = f[q], rh = rhs[q], w0 = rk > 0 ? fwk[q] : none;
-        const q2 z = ex[j * kCols + ci];
-        V h = rh;
-        if constexpr (!IM) {
-          h = mkv<R>(rh.x + qout<R>(z.x, eo), rh.y + qout<R>(z.y, eo));
-        } else if (role == 0) {
-          const q2 d = ex[(N + j) * kCols + ci];
-          h = mkv<R>(rh.x + qout<R>(d.x, ed), rh.y + qout<R>(d.y, ed));
+        for (int j = n; j < N; j += T / kCols) {
+          const long q = (long)j * ps;
+          const V fo = f[q], rh = rhs[q], w0 = rk > 0 ? fwk[q] : none;
+          const q2 z = ex[j * kCols + ci];
+          V h = rh;
+          if constexpr (!IM) {
+            h = mkv<R>(rh.x + qout<R>(z.x, eo), rh.y + qout<R>(z.y, eo));
+          } else if (din) {
+            const q2 d = ex[(N + j) * kCols + ci];
+            h = mkv<R>(rh.x + qout<R>(d.x, ed), rh.y + qout<R>(d.y, ed));
+          }
+          if constexpr (decltype(with)::value) {
+            const V t = buoy[q];
+            h = mkv<R>(h.x + t.x, h.y + t.y);
+          }
+          if (nanr) h = mkv<R>((R)nan(""), (R)nan(""));
+          V wk = mkv<R>(w0.x + gk * h.x, w0.y + gk * h.y);
+          const double2 p2 = m2[(long)j * nkx];
+          double fx, fy;
+          if constexpr (IM) {
+            fx = fb * (((double)wk.x + fromfix(z.x, eo)) + rdt * (double)fo.x);
+            fy = fb * (((double)wk.y + fromfix(z.y, eo)) + rdt * (double)fo.y);
+          } else {
+            fx = (double)(fo.x + dtr * wk.x), fy = (double)(fo.y + dtr * wk.y);
+          }
+          V fn = mkv<R>((R)fma(fx, p2.x, -(fy * p2.y)), (R)fma(fy, p2.x, fx * p2.y));
+          if (IM && is00) fn = fo;
+          if (rk < 2) {
+            // zeta_k h in the frame of the next substep; zeta_k is in the phase
+            const double2 p1 = m1[(long)j * nkx];
+            const double hx = (double)h.x, hy = (double)h.y;
+            wk = mkv<R>((R)fma(hx, p1.x, -(hy * p1.y)), (R)fma(hy, p1.x, hx * p1.y));
+          }
+          if (act) {
+            if (!IM) f[q] = fn;
+            if (!IM || rk < 2) fwk[q] = wk;
+          }
+          top = max(top, vtop(fn));
+          *(V *)(ex + j * kCols + ci) = fn;
         }
-        if (nanr) h = mkv<R>((R)nan(""), (R)nan(""));
-        V wk = mkv<R>(w0.x + gk * h.x, w0.y + gk * h.y);
-        const double2 p2 = m2[(long)j * nkx];
-        double fx, fy;
-        if constexpr (IM) {
-          fx = fb * (((double)wk.x + fromfix(z.x, eo)) + rdt * (double)fo.x);
-          fy = fb * (((double)wk.y + fromfix(z.y, eo)) + rdt * (double)fo.y);
-        } else {
-          fx = (double)(fo.x + dtr * wk.x), fy = (double)(fo.y + dtr * wk.y);
+      };
+      constexpr std::true_type yes;
+      constexpr std::false_type no_;
+      const bool with = GEN && g.temp && role == 0;
+      if constexpr (GEN) {
+        if (im) {
+          if (with) update(yes, yes);
+          else update(no_, yes);
+        } else if (with) {
+          update(yes, no_);
         }
-        V fn = mkv<R>((R)fma(fx, p2.x, -(fy * p2.y)), (R)fma(fy, p2.x, fx * p2.y));
-        if (IM && is00) fn = fo;
-        if (rk < 2) {
-          // zeta_k h in the frame of the next substep; zeta_k is in the phase
-          const double2 p1 = m1[(long)j * nkx];
-          const double hx = (double)h.x, hy = (double)h.y;
-          wk = mkv<R>((R)fma(hx, p1.x, -(hy * p1.y)), (R)fma(hy, p1.x, hx * p1.y));
-        }
-        if (act) {
-          if (!IM) f[q] = fn;
-          if (!IM || rk < 2) fwk[q] = wk;
-        }
-        top = max(top, vtop(fn));
-        *(V *)(ex + j * kCols + ci) = fn;
       }
+      if (!im && !with) update(no_, no_);
     }
     atomicMax(&s_top[1][ci], top);
   }
@@ -522,28 +570,33 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-template <typename R, int N, int T, bool IM>
+template <typename R, int N, int T, bool GEN>
 static cudaError_t launch_n(const Grid &g, const Bufs &bf, int rk, cudaStream_t st, bool prep,
-                            unsigned blocks) {
+                            unsigned blocks, int role0) {
   if (prep)
-    return cudaFuncSetAttribute(k_lineQ<R, N, T, IM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(k_lineQ<R, N, T, GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)LineQ<N>::smem);
-  k_lineQ<R, N, T, IM><<<dim3(blocks, (unsigned)g.B), T, LineQ<N>::smem, st>>>(g, bf, rk);
+  k_lineQ<R, N, T, GEN><<<dim3(blocks, (unsigned)g.B), T, LineQ<N>::smem, st>>>(g, bf, rk, role0);
   return cudaGetLastError();
 }
-template <typename R, int N, bool IM>
+template <typename R, int N, bool GEN>
 static cudaError_t launch_t(const Grid &g, const Bufs &bf, int rk, cudaStream_t st, bool prep) {
   constexpr int W = LineQ<N>::kWide, S = LineQ<N>::kNarrow;
-  const unsigned blocks = (unsigned)(2 * g.mz * ((g.nkx + kCols - 1) / kCols) + 1);
-  if constexpr (W != S && !IM) {
-    if (prep) {
-      const cudaError_t e = launch_n<R, N, S, IM>(g, bf, rk, st, true, blocks);
-      if (e != cudaSuccess) return e;
-    } else if ((long)blocks * g.B >= 5 * 152) {
-      return launch_n<R, N, S, IM>(g, bf, rk, st, false, blocks);
+  const unsigned per = (unsigned)(g.mz * ((g.nkx + kCols - 1) / kCols));
+  cudaError_t e = cudaSuccess;
+  // the velocity's roles, then the temperature's (its Lt is read by the former)
+  for (int role0 = 0; e == cudaSuccess && role0 < (g.temp ? 6 : 3); role0 += 3) {
+    const unsigned blocks = (role0 ? 1 : 2) * per + 1;
+    bool narrow = false;
+    if constexpr (W != S && (!GEN || S >= 64)) {
+      narrow = (long)blocks * g.B >= 5 * 152;
+      if (prep || narrow) e = launch_n<R, N, S, GEN>(g, bf, rk, st, prep, blocks, role0);
     }
+    if (e == cudaSuccess && !narrow)
+      e = launch_n<R, N, W, GEN>(g, bf, rk, st, prep, blocks, role0);
+    if (prep && narrow) e = launch_n<R, N, W, GEN>(g, bf, rk, st, prep, blocks, role0);
   }
-  return launch_n<R, N, W, IM>(g, bf, rk, st, prep, blocks);
+  return e;
 }
 
 #if SB_FLOAT_TU
@@ -551,9 +604,9 @@ typedef float UnitR;
 #else
 typedef double UnitR;
 #endif
-cudaError_t SB_LINEQ_UNIT(SB_FLOAT_TU, SB_LEN, SB_IMPL)(const Grid &g, const Bufs &bf, int rk,
+cudaError_t SB_LINEQ_UNIT(SB_FLOAT_TU, SB_LEN, SB_GEN)(const Grid &g, const Bufs &bf, int rk,
                                                         cudaStream_t st, bool prep) {
-  constexpr bool I = SB_IMPL != 0;
+  constexpr bool I = SB_GEN != 0;
   switch (g.my) {
 #if SB_LEN == 0
     case 32: return launch_t<UnitR, 32, I>(g, bf, rk, st, prep);
@@ -574,7 +627,7 @@ cudaError_t SB_LINEQ_UNIT(SB_FLOAT_TU, SB_LEN, SB_IMPL)(const Grid &g, const Buf
   }
 }
 
-#if !SB_FLOAT_TU && SB_LEN == 0 && !SB_IMPL
+#if !SB_FLOAT_TU && SB_LEN == 0 && !SB_GEN
 // ---------------------------------------------------------------------------
 // the phase tables of slot sn for a box: per (row or wave m, kx) the twist
 // exp(-i psi m/my) and the symbols l1, l2 at t = (psi + 2 pi m)/my.  psi is
@@ -653,14 +706,13 @@ static cudaError_t lineQ(const Grid &g, const Bufs &bf, int rk, cudaStream_t st,
        {lineQ_unit1_0_0, lineQ_unit1_1_0, lineQ_unit1_2_0}},
       {{lineQ_unit0_0_1, lineQ_unit0_1_1, lineQ_unit0_2_1},
        {lineQ_unit1_0_1, lineQ_unit1_1_1, lineQ_unit1_2_1}}};
-  return unit[g.impl ? 1 : 0][g.prec ? 1 : 0][g.my < 96 ? 0 : g.my < 256 ? 1 : 2](g, bf, rk, st,
+  return unit[g.impl || g.temp ? 1 : 0][g.prec ? 1 : 0][g.my < 96 ? 0 : g.my < 256 ? 1 : 2](g, bf, rk, st,
                                                                                  prep);
 }
 
-// the plain step, explicit (LES included: its k_lineL runs before) or
-// semi-implicit, on the transform lengths; the temperature, the y filter and
-// dealiasing keep the banded solves
-bool line_bloch_ok(const Grid &g) { return !g.temp && !g.ydeal && fix_length(g.my); }
+// the step, explicit (LES included: its k_lineL runs before) or semi-implicit,
+// on the transform lengths; the y filter and dealiasing keep the banded solves
+bool line_bloch_ok(const Grid &g) { return !g.ydeal && fix_length(g.my); }
 
 cudaError_t launch_lineQ(const Grid &g, const Bufs &bf, int rk, cudaStream_t st) {
   return lineQ(g, bf, rk, st, false);

@@ -140,3 +140,34 @@ def test_scales_of_a_batch_are_independent():
         for k in ("vor", "phi", "u00", "w00"):
             assert np.array_equal(a[k], b[k]), (m, k)
     assert np.isnan(box.get_state(2)["vor"]).any() and box.status(2).flags & 2
+
+
+# the semi-implicit block with the scalar takes lines up to 256
+@pytest.mark.parametrize("my,implicit", [(n, i) for n in LENGTHS for i in (0, 1)
+                                         if not (i and n > 256)])
+def test_temperature_at_every_length(my, implicit):
+    """The scalar's lines (tb and tb00, buoyancy in phi): two steps against the
+    oracle, and in the FP32-mixed form against the banded solves."""
+    import oracle
+    import shear_nnf_gb300 as sb
+    from test_gpu_temperature import _temp
+    pp = dict(_temp((48, my, 32), 1500.0), fixed_dt=0.3 * 2 * np.pi / my / 4, implicit_visc=implicit)
+    p = sb.make_params(**pp)
+    st = _state(p, my, 1.3)
+    st["tb00"] = st["tb00"] + 0.2 * np.cos(np.arange(my) * (2 * np.pi / my))
+    keys = ("vor", "phi", "u00", "w00", "tb", "tb00")
+    box, g, o = sb.ShearBox(p), copy_state(st), copy_state(st)
+    box.cross(g, 2)
+    oracle.Oracle(**pp).cross(o, 2)
+    for k in keys:
+        assert rel_l2(g[k], o[k]) < 4 * ONE_STEP, (k, rel_l2(g[k], o[k]))
+    out = {}
+    for form in ("split", "waves"):
+        box = sb.ShearBox(p, precision=sb.SB_MIXED)
+        if form == "split":
+            box.set_line_form(form)
+        s = copy_state(st)
+        box.cross(s, 2)
+        out[form] = s
+    for k in ("vor", "phi", "u00", "tb", "tb00"):
+        assert rel_l2(out["waves"][k], out["split"][k]) < 1e-6, k
