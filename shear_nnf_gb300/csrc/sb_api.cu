@@ -1510,7 +1510,8 @@ int sb_set_line_segments(sb_handle *h, int nseg) {
 int sb_set_line_form(sb_handle *h, int form) {
   if (!h) return fail(1, "null handle");
   if (form != 0 && form != 1) return fail(1, "line form %d (0 split, 1 fused)", form);
-  if (form == 1 && (!h->g.bloch || h->g.impl) && !line_fused_ok(h->g))
+  if (form == 1 && (!h->g.bloch || h->g.impl || h->g.temp) &&
+      !line_fused_ok(h->g))
     return fail(1, "fused y-line kernel not available for this handle");
   h->g.lform = form;
   return capture_step(h);
@@ -1531,7 +1532,10 @@ int sb_get_side_branch(sb_handle *h, int *mask) {
 
 int sb_get_line_form(sb_handle *h, int *form) {
   if (!h || !form) return fail(1, "null argument");
-  *form = h->g.impl ? 2 : ((h->g.lform && (use_bloch(h) || line_fused_ok(h->g))) ? 1 : 0);
+  // the scalar's handles report the split form with the waves as well: the
+  // fused banded kernel is not theirs to choose
+  const bool one = h->g.lform && !h->g.temp && (use_bloch(h) || line_fused_ok(h->g));
+  *form = h->g.impl ? 2 : (one ? 1 : 0);
   return 0;
 }
 
