@@ -491,12 +491,9 @@ static void member_defaults(const sb_params *p, const Grid &g, double Re, Member
   m->cflkk = p->temperature ? p->fkappa / p->CFL * mm : 0.0;
 }
 
-// the phase tables of substep rk (0: the start of a run): the Bloch-wave
-// form's, and the banded solves' where they run (with LES k_lineL does)
+// the phase tables of substep rk (0: the start of a run)
 static cudaError_t launch_phases(sb_handle *h, int rk, cudaStream_t st) {
-  if (!h->step_bloch) return launch_tables(h->g, h->bf, rk, st);
-  const cudaError_t e = h->g.les ? launch_tables(h->g, h->bf, rk, st) : cudaSuccess;
-  return e != cudaSuccess ? e : launch_bloch(h->g, h->bf, rk, st);
+  return h->step_bloch ? launch_bloch(h->g, h->bf, rk, st) : launch_tables(h->g, h->bf, rk, st);
 }
 
 static int capture_step(sb_handle *h) {
@@ -558,7 +555,9 @@ static int capture_step(sb_handle *h) {
       if ((e = launch_phases(h, rk, h->st)) != cudaSuccess) break;
       if (hfac && (e = launch_hfac(h->g, h->bf, rk, h->st)) != cudaSuccess) break;
     }
-    if (h->g.les && (e = launch_lineL(h->g, h->bf, h->st)) != cudaSuccess) break;
+    if (h->g.les && (e = h->step_bloch ? launch_lineLQ(h->g, h->bf, rk, h->st)
+                                       : launch_lineL(h->g, h->bf, h->st)) != cudaSuccess)
+      break;
     if (h->step_bloch) {
       e = launch_lineQ(h->g, h->bf, rk, h->st);
       continue;
@@ -1300,7 +1299,7 @@ int sb_launch_stage(sb_handle *h, int stage, int rk, int count) {
     else if (stage <= 10)
       e = launch_les(h->g, h->bf, stage - 5, rk, h->st);
     else if (stage == 11)
-      e = launch_lineL(h->g, h->bf, h->st);
+      e = h->step_bloch ? launch_lineLQ(h->g, h->bf, rk, h->st) : launch_lineL(h->g, h->bf, h->st);
     else if (stage == 12)
       e = h->step_bloch ? launch_lineQ(h->g, h->bf, rk, h->st) : launch_lineF(h->g, h->bf, rk, h->st);
     else if (stage == 13)
@@ -1434,12 +1433,11 @@ int sb_autotune(sb_handle *h, int *choice) {
   for (int c : {1, 2, 3}) {
     if (rc || e != cudaSuccess) break;
     if ((g.my - 3) / c < 6) continue;
-    if (g.bloch && h->nasym == 0 && !g.les && c != nseg) continue;
+    if (g.bloch && h->nasym == 0 && c != nseg) continue;
     if ((rc = build_line_tables(h, c))) break;
     // both forms of the y-line stage where the fused one is available.  The
     // Bloch-wave form needs no trial against the split kernels (192x96x96
-    // FP64: 105 us a substep against 123 + 258) and has no segments: one trial,
-    // or with LES, whose k_lineL is segmented, one per tile
+    // FP64: 90 us a substep against 123 + 258) and has no segments: one trial
     const bool bloch = g.bloch && h->nasym == 0;
     for (int f = 1; f >= (bloch ? 1 : 0); f--) {
       if (rc || e != cudaSuccess) break;

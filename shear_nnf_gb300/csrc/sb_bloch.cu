@@ -567,6 +567,122 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
   }
 }
 
+#if !SB_GEN
+// The LES y-operators (iuse_LES, cross.f90:565-608,639-647) at the phase of t,
+// between k_bloch and k_lineQ:
+//   role 0  hg += d(rhgc2)/dy                                       (L2 -> Gn)
+//   role 1  hv -= (kx^2 + kz^2 + d2/dy2) rhvc2                       (L1 -> V)
+//   mean    rf0u += d(T12_00)/dy, rf0w += d(T23_00)/dy              (txy -> mrf)
+// One transform and its inverse a line, where k_lineL spends a banded FP64 solve
+// (384x192x192 mixed: 264 us against 909; 192x96x96 FP64: 34 against 121).  Bound
+// by the integer pipes, as k_lineQ.
+template <typename R, int N, int T>
+__global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineLQ(Grid g, Bufs bf, int rk) {
+  typedef LineQ<N> L;
+  typedef typename V2<R>::t V;
+  constexpr int R1 = L::R1, R2 = L::R2;
+  constexpr int kN = floor_log2(N), kTgt = Plan<N>::bits;
+  const int b = blockIdx.y;
+  if (bf.mem[b].halted) return;  // uniform per block
+  extern __shared__ __align__(16) unsigned char smq_raw[];
+  q2 *const ex = (q2 *)smq_raw;
+  __shared__ unsigned s_top[kCols];
+  __shared__ int s_len[kCols];
+  const int ncb = (g.nkx + kCols - 1) / kCols, per = g.mz * ncb;
+  const int role = blockIdx.x / per, r = blockIdx.x - role * per;
+  const bool mean = role == 2;
+  const int ci = threadIdx.x & (kCols - 1), n = threadIdx.x / kCols;
+  const int k = mean ? 0 : r / ncb;
+  const int i0 = mean ? ci : (r - k * ncb) * kCols + ci;
+  const bool act = mean ? ci < 2 : i0 < g.nkx;
+  const int cm = ci & 1;
+  const int i = mean ? 0 : (act ? i0 : g.nkx - 1);
+  const int nkx = g.nkx;
+  const long ps = g.plane / 2, off = (long)b * (g.field / 2) + (long)k * nkx + i;
+  if (threadIdx.x < kCols) {
+    s_top[threadIdx.x] = 0u;
+    s_len[threadIdx.x] = kNoLen;
+  }
+  __syncthreads();
+  const double a = g.alp * i, gz = g.gam * ((k <= g.nz) ? k : k - g.mz);
+  const double k2 = a * a + gz * gz;
+  const long o = ((long)((rk - 1) % 3) * g.B + b) * N * nkx + i;
+  const qw *tw = bf.btw + o;
+  const V *src = (const V *)(role == 0 ? bf.L2 : bf.L1) + off;
+  const R *tx = (const R *)bf.txy + (long)b * 2 * N + cm;
+  unsigned top = 0;
+#pragma unroll 4
+  for (int j = n; j < N; j += T / kCols) {
+    const V w = mean ? mkv<R>(tx[2 * j], (R)0) : src[(long)j * ps];
+    *(V *)(ex + j * kCols + ci) = w;
+    top = max(top, vtop(w));
+  }
+  atomicMax(&s_top[ci], top);
+  __syncthreads();
+  const QScale sr = qscale(s_top[ci], L::kBits);
+#pragma unroll 1
+  for (int it = n; it < R2; it += T / kCols)
+    rows_forward<N, V>(ex, sr, tw, nkx, bf.bftw, it, ci);
+  __syncthreads();
+  // i l1 or -(l2 + k^2)
+  const double *l = (role == 1 ? bf.bl2 : bf.bl1) + o;
+  auto factor = [&](double v) { return role == 1 ? -(v + k2) : v; };
+#pragma unroll 1
+  for (int k1 = n; k1 < R1; k1 += T / kCols) {
+    q2 *e = ex + k1 * R2 * kCols + ci;
+    const double *lk = l + (long)k1 * nkx;
+    q2 x[R2];
+#pragma unroll
+    for (int w = 0; w < R2; w++) x[w] = e[w * kCols];
+    Dft<R2, -1>::run(x);
+    int la = kNoLen;
+#pragma unroll
+    for (int w = 0; w < R2; w++) {
+      e[w * kCols] = x[w];
+      la = max(la, qlen(x[w]) + qexp(factor(lk[(long)(R1 * w) * nkx])));
+    }
+    atomicMax(&s_len[ci], la);
+  }
+  __syncthreads();
+  const int len = s_len[ci] + 1;
+#pragma unroll 1
+  for (int k1 = n; k1 < R1; k1 += T / kCols) {
+    q2 *e = ex + k1 * R2 * kCols + ci;
+    const double *lk = here(l) + (long)k1 * nkx;
+    q2 y[R2];
+#pragma unroll
+    for (int w = 0; w < R2; w++) {
+      y[w] = qscaled(e[w * kCols], factor(lk[(long)(R1 * w) * nkx]), kTgt - len);
+      if (role != 1) y[w] = qrot<1>(y[w]);
+    }
+    Dft<R2, 1>::run(y);
+#pragma unroll
+    for (int w = 0; w < R2; w++) e[w * kCols] = qmul<false>(y[w], bf.bitw[w * k1]);
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int it = n; it < R2; it += T / kCols) rows_inverse<N>(ex, here(tw), nkx, it, ci);
+  __syncthreads();
+  const int eo = L::kShiftF + Plan<N>::shift + 2 - kN - kTgt - sr.weight() + len;
+  const bool none = sr.bad || qrange(eo);
+  const R nn = (R)nan("");
+  if (!act || (role == 1 && i == 0 && k == 0)) return;
+  if (mean) {
+    R *mrf = (R *)bf.mrf + (long)b * 2 * N + cm;
+    for (int j = n; j < N; j += T / kCols)
+      mrf[2 * j] += none ? nn : qout<R>(ex[j * kCols + ci].x, eo);
+    return;
+  }
+  V *dst = (V *)(role == 1 ? bf.V : bf.Gn) + off;
+#pragma unroll 2
+  for (int j = n; j < N; j += T / kCols) {
+    const q2 z = ex[j * kCols + ci];
+    const V d = dst[(long)j * ps];
+    dst[(long)j * ps] = none ? mkv<R>(nn, nn) : mkv<R>(d.x + qout<R>(z.x, eo), d.y + qout<R>(z.y, eo));
+  }
+}
+#endif
+
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
@@ -599,32 +715,50 @@ static cudaError_t launch_t(const Grid &g, const Bufs &bf, int rk, cudaStream_t 
   return e;
 }
 
+#if !SB_GEN
+template <typename R, int N, int T>
+static cudaError_t launch_ln(const Grid &g, const Bufs &bf, int rk, cudaStream_t st, bool prep,
+                             unsigned blocks) {
+  constexpr int smem = (int)sizeof(q2) * N * kCols;
+  if (prep)
+    return cudaFuncSetAttribute(k_lineLQ<R, N, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  k_lineLQ<R, N, T><<<dim3(blocks, (unsigned)g.B), T, smem, st>>>(g, bf, rk);
+  return cudaGetLastError();
+}
+template <typename R, int N>
+static cudaError_t launch_lt(const Grid &g, const Bufs &bf, int rk, cudaStream_t st, bool prep) {
+  const unsigned blocks = (unsigned)(2 * g.mz * ((g.nkx + kCols - 1) / kCols) + 1);
+  return launch_ln<R, N, LineQ<N>::kWide>(g, bf, rk, st, prep, blocks);
+}
+#endif
+
 #if SB_FLOAT_TU
 typedef float UnitR;
 #else
 typedef double UnitR;
 #endif
+// les: k_lineLQ instead (in the units without SB_GEN)
 cudaError_t SB_LINEQ_UNIT(SB_FLOAT_TU, SB_LEN, SB_GEN)(const Grid &g, const Bufs &bf, int rk,
-                                                        cudaStream_t st, bool prep) {
-  constexpr bool I = SB_GEN != 0;
+                                                        cudaStream_t st, bool prep, bool les) {
+#if SB_GEN
+#define SB_CASE(N) \
+  case N: return launch_t<UnitR, N, true>(g, bf, rk, st, prep);
+#else
+#define SB_CASE(N)                                                   \
+  case N:                                                            \
+    return les ? launch_lt<UnitR, N>(g, bf, rk, st, prep) : launch_t<UnitR, N, false>(g, bf, rk, st, prep);
+#endif
   switch (g.my) {
 #if SB_LEN == 0
-    case 32: return launch_t<UnitR, 32, I>(g, bf, rk, st, prep);
-    case 48: return launch_t<UnitR, 48, I>(g, bf, rk, st, prep);
-    case 64: return launch_t<UnitR, 64, I>(g, bf, rk, st, prep);
-    case 80: return launch_t<UnitR, 80, I>(g, bf, rk, st, prep);
+    SB_CASE(32) SB_CASE(48) SB_CASE(64) SB_CASE(80)
 #elif SB_LEN == 1
-    case 96: return launch_t<UnitR, 96, I>(g, bf, rk, st, prep);
-    case 128: return launch_t<UnitR, 128, I>(g, bf, rk, st, prep);
-    case 160: return launch_t<UnitR, 160, I>(g, bf, rk, st, prep);
-    case 192: return launch_t<UnitR, 192, I>(g, bf, rk, st, prep);
+    SB_CASE(96) SB_CASE(128) SB_CASE(160) SB_CASE(192)
 #else
-    case 256: return launch_t<UnitR, 256, I>(g, bf, rk, st, prep);
-    case 320: return launch_t<UnitR, 320, I>(g, bf, rk, st, prep);
-    case 384: return launch_t<UnitR, 384, I>(g, bf, rk, st, prep);
+    SB_CASE(256) SB_CASE(320) SB_CASE(384)
 #endif
     default: return cudaErrorInvalidValue;
   }
+#undef SB_CASE
 }
 
 #if !SB_FLOAT_TU && SB_LEN == 0 && !SB_GEN
@@ -696,28 +830,35 @@ __global__ void __launch_bounds__(64) k_bloch(Grid g, Bufs bf, int rk) {
   bf.bl2[o] = n2 / p2;
 }
 
-typedef cudaError_t LineQUnit(const Grid &, const Bufs &, int, cudaStream_t, bool);
+typedef cudaError_t LineQUnit(const Grid &, const Bufs &, int, cudaStream_t, bool, bool);
 LineQUnit lineQ_unit0_1_0, lineQ_unit0_2_0, lineQ_unit1_0_0, lineQ_unit1_1_0, lineQ_unit1_2_0;
 LineQUnit lineQ_unit0_0_1, lineQ_unit0_1_1, lineQ_unit0_2_1, lineQ_unit1_0_1, lineQ_unit1_1_1,
     lineQ_unit1_2_1;
-static cudaError_t lineQ(const Grid &g, const Bufs &bf, int rk, cudaStream_t st, bool prep) {
+static cudaError_t lineQ(const Grid &g, const Bufs &bf, int rk, cudaStream_t st, bool prep,
+                         bool les) {
   static LineQUnit *const unit[2][2][3] = {
       {{lineQ_unit0_0_0, lineQ_unit0_1_0, lineQ_unit0_2_0},
        {lineQ_unit1_0_0, lineQ_unit1_1_0, lineQ_unit1_2_0}},
       {{lineQ_unit0_0_1, lineQ_unit0_1_1, lineQ_unit0_2_1},
        {lineQ_unit1_0_1, lineQ_unit1_1_1, lineQ_unit1_2_1}}};
-  return unit[g.impl || g.temp ? 1 : 0][g.prec ? 1 : 0][g.my < 96 ? 0 : g.my < 256 ? 1 : 2](g, bf, rk, st,
-                                                                                 prep);
+  return unit[!les && (g.impl || g.temp) ? 1 : 0][g.prec ? 1 : 0][g.my < 96 ? 0 : g.my < 256 ? 1 : 2](g, bf, rk, st,
+                                                                                 prep, les);
 }
 
-// the step, explicit (LES included: its k_lineL runs before) or semi-implicit,
+// the step, explicit (with or without LES) or semi-implicit,
 // on the transform lengths; the y filter and dealiasing keep the banded solves
 bool line_bloch_ok(const Grid &g) { return !g.ydeal && fix_length(g.my); }
 
 cudaError_t launch_lineQ(const Grid &g, const Bufs &bf, int rk, cudaStream_t st) {
-  return lineQ(g, bf, rk, st, false);
+  return lineQ(g, bf, rk, st, false, false);
 }
-cudaError_t prepare_lineQ(const Grid &g, const Bufs &bf) { return lineQ(g, bf, 0, 0, true); }
+cudaError_t launch_lineLQ(const Grid &g, const Bufs &bf, int rk, cudaStream_t st) {
+  return lineQ(g, bf, rk, st, false, true);
+}
+cudaError_t prepare_lineQ(const Grid &g, const Bufs &bf) {
+  const cudaError_t e = g.les ? lineQ(g, bf, 0, 0, true, true) : cudaSuccess;
+  return e != cudaSuccess ? e : lineQ(g, bf, 0, 0, true, false);
+}
 cudaError_t launch_bloch(const Grid &g, const Bufs &bf, int rk, cudaStream_t st) {
   const long n = (long)g.my * g.nkx;
   k_bloch<<<dim3((unsigned)((n + 63) / 64), (unsigned)g.B), 64, 0, st>>>(g, bf, rk);

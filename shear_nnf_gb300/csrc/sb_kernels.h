@@ -43,6 +43,7 @@ bool line_fused_ok(const Grid &g);
 bool line_bloch_ok(const Grid &g);
 cudaError_t prepare_lineQ(const Grid &g, const Bufs &bf);
 cudaError_t launch_lineQ(const Grid &g, const Bufs &bf, int rk, cudaStream_t st);
+cudaError_t launch_lineLQ(const Grid &g, const Bufs &bf, int rk, cudaStream_t st);
 cudaError_t launch_bloch(const Grid &g, const Bufs &bf, int rk, cudaStream_t st);
 // the semi-implicit viscous branch: factor tables of the substep (k_hfac)
 // and the y-line kernel (k_lineI)

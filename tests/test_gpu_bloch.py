@@ -105,6 +105,26 @@ def test_semi_implicit_options():
     _parity(pp, _state(p, 3, 0.7), nstep=2, tol=4 * ONE_STEP, box=box)
 
 
+@pytest.mark.parametrize("my", LENGTHS)
+def test_les_at_every_length(my):
+    """The LES y-operators (k_lineLQ): one step against the oracle, and in the
+    FP32-mixed form against the banded solves."""
+    import shear_nnf_gb300 as sb
+    pp = box_params(64, my, 32, rez=2000.0, les=1, cs=0.1, fixed_dt=0.3 * 2 * np.pi / my / 4)
+    p = sb.make_params(**pp)
+    st = _state(p, my, 1.7)
+    _parity(pp, st)
+    out = {}
+    for form in ("split", "fused"):
+        box = sb.ShearBox(p, precision=sb.SB_MIXED)
+        box.set_line_form(form)
+        s = copy_state(st)
+        box.cross(s, 2)
+        out[form] = s
+    for k in ("vor", "phi", "u00"):
+        assert rel_l2(out["fused"][k], out["split"][k]) < 1e-6, k
+
+
 def test_unequal_offsets_keep_the_banded_solves():
     """xoffb != -xofft: one handle steps such a state (banded), then opposite
     offsets again, with the bits of a fresh handle."""
