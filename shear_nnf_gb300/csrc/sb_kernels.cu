@@ -219,11 +219,22 @@ __global__ void __launch_bounds__(T) k_p1(Grid g, Bufs bf, int rk) {
 // o12p eps) and of tbp utbp vtbp wtbp, reduced per plane by k_hsum.  A block
 // takes 16 modes of a box; its 8 thread slices take every 8th plane; the
 // per-mode slices are added in a fixed order, the per-plane modes in mode
-// order through shared memory.  FP64 arithmetic whatever the storage precision.  Runs
+// order through shared memory.  FP64 arithmetic whatever the storage precision;
+// bound by it, so the factors i kx/k^2 are formed once, the modes' weights are
+// applied in the sums over the modes and FP32 state is widened by its bits (192x96x96
+// step 1065 -> 1054 us, mixed 684 -> 675).  Runs
 // before the per-box scalars update Delta t: spl2 and splt carry the Delta t
 // of the previous step, as in hist 'f'.
 // ---------------------------------------------------------------------------
 constexpr int kSpecModes = 16, kSpecSlices = 8;
+// an FP32 number as FP64 by its bits (the conversion takes a 64-cycle FP64 issue)
+__device__ __forceinline__ double widen(double x) { return x; }
+__device__ __forceinline__ double widen(float x) {
+  const unsigned u = __float_as_uint(x), m = u & 0x7fffffffu;
+  if (m - 1u < 0x7fffffu || m >= 0x7f800000u) return (double)x;  // subnormal, inf, NaN
+  return __hiloint2double((int)((u & 0x80000000u) | (m ? (m >> 3) + 0x38000000u : 0u)),
+                          (int)(u << 29));
+}
 template <typename R, bool TEMP>
 __global__ void __launch_bounds__(kSpecModes * kSpecSlices) k_spectra(Grid g, Bufs bf) {
   typedef typename Vec2<R>::t V;
@@ -239,13 +250,16 @@ __global__ void __launch_bounds__(kSpecModes * kSpecSlices) k_spectra(Grid g, Bu
   const double a = g.alp * i;
   const double gz = g.gam * ((k <= nz) ? k : k - mz);
   const double Kk = a * a + gz * gz;
-  const double iK = bf.kinv[q];
+  const double aK = a * bf.kinv[q], gK = gz * bf.kinv[q];
+  // a mode's weight, a power of two, is applied where the modes are summed;
   // invalid threads (past the last mode) carry weight 0
+  __shared__ double wsum[kSpecModes];
   const double wm = valid ? ((i == 0) ? 1.0 : 2.0) : 0.0;
   const bool z00 = (i == 0 && k == 0);
   // set_conj of the omega_y and phi copies (cross.f90:502)
   const int qs = (i == 0 && k > nz) ? (mz - k) * nkx : q;
-  const double cs = (i == 0 && k > nz) ? -1.0 : 1.0;
+  const bool cj = i == 0 && k > nz;
+  if (sl == 0) wsum[mi] = wm;  // read after the first barrier of the loop
   const int nblk = gridDim.x;
   double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0}, tacc[4] = {0, 0, 0, 0};
   // per-plane products of the 16 modes, double-buffered across iterations
@@ -258,15 +272,15 @@ __global__ void __launch_bounds__(kSpecModes * kSpecSlices) k_spectra(Grid g, Bu
     const int jr = sl + kSpecSlices * it;
     const bool jok = jr < g.my;
     const int j = jok ? jr : g.my - 1;
-    const double w = jok ? wm : 0.0;
     const long pb = (long)b * g.field + (long)j * g.plane;
     const V *vor = (const V *)((const R *)bf.vor + pb), *phi = (const V *)((const R *)bf.phi + pb);
     const V *Dv = (const V *)((const R *)bf.D + pb), *Vv = (const V *)((const R *)bf.V + pb);
     const V *Gv = (const V *)((const R *)bf.G + pb);
     const V vr0 = vor[qs], ph0 = phi[qs];
     const V dvr = Vv[q];
-    const double vrx = vr0.x, vry = cs * (double)vr0.y, phx = ph0.x, phy = cs * (double)ph0.y;
-    const double dvx = dvr.x, dvy = dvr.y;
+    const double vrx = widen(vr0.x), vry = cj ? -widen(vr0.y) : widen(vr0.y);
+    const double phx = widen(ph0.x), phy = cj ? -widen(ph0.y) : widen(ph0.y);
+    const double dvx = widen(dvr.x), dvy = widen(dvr.y);
     double u1x, u1y, u2x, u2y, u3x, u3y, o1x, o1y, o3x, o3y;
     if (z00) {
       const V mu = ((const V *)bf.mu)[(long)b * g.my + j];
@@ -278,66 +292,65 @@ __global__ void __launch_bounds__(kSpecModes * kSpecSlices) k_spectra(Grid g, Bu
       u2x = M.vbulk; u2y = 0.0;
     } else {
       const V w1 = Dv[q], gv = Gv[q];
-      double tx, ty;
-      tx = gz * w1.x - a * phx; ty = gz * w1.y - a * phy;
-      o3x = -ty * iK; o3y = tx * iK;
-      tx = a * w1.x + gz * phx; ty = a * w1.y + gz * phy;
-      o1x = -ty * iK; o1y = tx * iK;
-      tx = gz * dvx + a * vrx; ty = gz * dvy + a * vry;
-      u3x = -ty * iK; u3y = tx * iK;
-      tx = a * dvx - gz * vrx; ty = a * dvy - gz * vry;
-      u1x = -ty * iK; u1y = tx * iK;
-      u2x = gv.x; u2y = gv.y;
+      const double wx = widen(w1.x), wy = widen(w1.y);
+      o3x = fma(-gK, wy, aK * phy); o3y = fma(gK, wx, -(aK * phx));
+      o1x = -fma(aK, wy, gK * phy); o1y = fma(aK, wx, gK * phx);
+      u3x = -fma(gK, dvy, aK * vry); u3y = fma(gK, dvx, aK * vrx);
+      u1x = fma(-aK, dvy, gK * vry); u1y = fma(aK, dvx, -(gK * vrx));
+      u2x = widen(gv.x); u2y = widen(gv.y);
     }
     const double uu = u1x * u1x + u1y * u1y, vv = u2x * u2x + u2y * u2y,
                  ww = u3x * u3x + u3y * u3y;
     double pq[SB_NHIST_Q];
-    pq[0] = w * uu;
-    pq[1] = w * vv;
-    pq[2] = w * ww;
-    pq[3] = w * (u1x * u2x + u1y * u2y);
-    pq[4] = w * (u1x * u3x + u1y * u3y);
-    pq[5] = w * (u2x * u3x + u2y * u3y);
-    pq[6] = w * (o1x * o1x + o1y * o1y);
-    pq[7] = w * (vrx * vrx + vry * vry);
-    pq[8] = w * (o3x * o3x + o3y * o3y);
-    pq[9] = w * (o1x * vrx + o1y * vry);
+    pq[0] = uu;
+    pq[1] = vv;
+    pq[2] = ww;
+    pq[3] = u1x * u2x + u1y * u2y;
+    pq[4] = u1x * u3x + u1y * u3y;
+    pq[5] = u2x * u3x + u2y * u3y;
+    pq[6] = o1x * o1x + o1y * o1y;
+    pq[7] = vrx * vrx + vry * vry;
+    pq[8] = o3x * o3x + o3y * o3y;
+    pq[9] = o1x * vrx + o1y * vry;
     {
       // dissipation (cross.f90:1926-1944); omega_z of the mean includes -s
       const double o3sx = z00 ? o3x - g.s : o3x;
       const double c1x = o1x - gz * u2y, c1y = o1y + gz * u2x;   // o1 + i gz u2
       const double c3x = o3sx + a * u2y, c3y = o3y - a * u2x;    // o3 - i a u2
-      pq[10] = w * (Kk * (uu + vv + ww) + (dvx * dvx + dvy * dvy) + (c1x * c1x + c1y * c1y) +
-                    (c3x * c3x + c3y * c3y));
+      pq[10] = Kk * (uu + vv + ww) + (dvx * dvx + dvy * dvy) + (c1x * c1x + c1y * c1y) +
+               (c3x * c3x + c3y * c3y);
     }
     // spectra: omega_z of the mean without -s (cross.f90:1968)
-    acc[0] += pq[0];
-    acc[1] += pq[1];
-    acc[2] += pq[2];
-    acc[3] += pq[3];
-    acc[4] += pq[6];
-    acc[5] += pq[7];
-    acc[6] += pq[8];
-    acc[7] += pq[9];
+    if (jok) {
+      acc[0] += pq[0];
+      acc[1] += pq[1];
+      acc[2] += pq[2];
+      acc[3] += pq[3];
+      acc[4] += pq[6];
+      acc[5] += pq[7];
+      acc[6] += pq[8];
+      acc[7] += pq[9];
+    }
     if (TEMP) {
       double tx, ty = 0.0;
       if (z00) {
         tx = ((const V *)bf.mt)[(long)b * g.my + j].x;
       } else {
         const V t = ((const V *)((const R *)bf.tb + pb))[q];
-        tx = t.x;
-        ty = t.y;
+        tx = widen(t.x);
+        ty = widen(t.y);
       }
-      pq[11] = w * (tx * tx + ty * ty);
-      pq[12] = w * (u1x * tx + u1y * ty);
-      pq[13] = w * (u2x * tx + u2y * ty);
-      pq[14] = w * (u3x * tx + u3y * ty);
+      pq[11] = tx * tx + ty * ty;
+      pq[12] = u1x * tx + u1y * ty;
+      pq[13] = u2x * tx + u2y * ty;
+      pq[14] = u3x * tx + u3y * ty;
+      if (jok)
 #pragma unroll
-      for (int f = 0; f < 4; f++) tacc[f] += pq[11 + f];
+        for (int f = 0; f < 4; f++) tacc[f] += pq[11 + f];
     }
     // the plane's partial over the block's 16 modes: the products go through
     // shared memory and one thread per (slice, quantity) adds its 16 modes in
-    // order (15 FP64 adds per quantity, where a shuffle tree spends 4 adds on
+    // order (16 FP64 operations per quantity, where a shuffle tree spends 4 adds on
     // every lane)
     double(*tp)[NQ][kSpecModes + 1] = tpart[it & 1];
 #pragma unroll
@@ -347,9 +360,9 @@ __global__ void __launch_bounds__(kSpecModes * kSpecSlices) k_spectra(Grid g, Bu
       const int s2 = threadIdx.x / NQ, f = threadIdx.x - s2 * NQ;
       const int j2 = s2 + kSpecSlices * it;
       if (j2 < g.my) {
-        double x = tp[s2][f][0];
+        double x = wsum[0] * tp[s2][f][0];
 #pragma unroll
-        for (int m = 1; m < kSpecModes; m++) x += tp[s2][f][m];
+        for (int m = 1; m < kSpecModes; m++) x = fma(wsum[m], tp[s2][f][m], x);
         double *hp = bf.hpart + (((long)b * g.my + j2) * nblk + blockIdx.x) * SB_NHIST_Q;
         hp[f] = x;
         if (!TEMP && f == 0)
@@ -371,6 +384,7 @@ __global__ void __launch_bounds__(kSpecModes * kSpecSlices) k_spectra(Grid g, Bu
   for (int f = 0; f < (TEMP ? 12 : 8); f++) {
     double x = 0.0;
     for (int s2 = 0; s2 < kSpecSlices; s2++) x += red[s2][f][mi];
+    x *= wm;
     if (f < 8) {
       sp[f] += x;
       sp2[f] += x * dt;
