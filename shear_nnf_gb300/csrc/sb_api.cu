@@ -422,6 +422,27 @@ static int build_plane_tables(sb_handle *h) {
   bf.ze = (int *)q;
   if ((rc = dalloc(h, &q, (nxe + 1) / 2))) return rc;
   bf.xe = (int *)q;
+  // the modes' factors of stages 1 and 3
+  const double norm = 1.0 / (double)(g.mgalx * g.mgalz);
+  std::vector<double> kf(2 * (size_t)g.mz * g.nkx), gk(4 * (size_t)g.mz);
+  for (int k = 0; k < g.mz; k++) {
+    const double gz = g.gam * ((k <= g.nz) ? k : k - g.mz);
+    gk[4 * k] = gz;
+    gk[4 * k + 1] = gz * norm;
+    gk[4 * k + 2] = gz * g.s;
+    gk[4 * k + 3] = gz * (gz * norm);
+    for (int i = 0; i < g.nkx; i++) {
+      const double ax = g.alp * i, K = gz * gz + ax * ax;
+      const size_t m = 2 * ((size_t)k * g.nkx + i);
+      kf[m] = i || k ? ax / K : 0.0;
+      kf[m + 1] = i || k ? gz / K : 0.0;
+    }
+  }
+  const double *c;
+  if ((rc = upload(h, &c, kf))) return rc;
+  bf.kfac = (const double2 *)c;
+  if ((rc = upload(h, &c, gk))) return rc;
+  bf.gzk = (const double2 *)c;
   return 0;
 }
 

@@ -160,6 +160,8 @@ struct Bufs {
   const float *kinvf;            // kinv rounded to FP32
   const double *ginv;            // 1/g per kz  (g = gam * kz_signed; 0 at k=0)
   const double *kinv;            // 1/(alp2+gam2) per (k,i); 0 at (0,0)
+  const double2 *kfac;           // kx, kz over kx^2+kz^2 per (k,i); 0 at (0,0)
+  const double2 *gzk;            // per k: kz, kz/(mgalx mgalz); kz s, kz^2/(mgalx mgalz)
   Fac d1, d2, hz;                // d/dy, d2/dy2, Helmholtz (per line)
   Fac hi;                        // semi-implicit Helmholtz (k^2 + dtr1) per box and line
                                  // (kx, kz >= 0), then the mean line; rebuilt every substep

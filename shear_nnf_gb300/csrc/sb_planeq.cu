@@ -99,7 +99,6 @@ __global__ void __launch_bounds__(Z1<NZ>::T, Z1<NZ>::kMinB) k_z1(Grid g, Bufs bf
     const double2 *p0 = round == 0 ? (const double2 *)bf.V + pb : round == 1 ? (const double2 *)bf.D + pb
                                                                              : (const double2 *)bf.G + pb;
     const double2 *p1 = round == 1 ? phi : vor;
-    const double a = g.alp * i;
 #pragma unroll 2
     for (int k = threadIdx.x / kCols; k < mz; k += T / kCols) {
       double2 fa = make_double2(0.0, 0.0), fb = fa;
@@ -118,10 +117,12 @@ __global__ void __launch_bounds__(Z1<NZ>::T, Z1<NZ>::kMinB) k_z1(Grid g, Bufs bf
           if (sym) y.y = -y.y;
           if (round < 2) {
             // i (a x -+ gz y)/k2, i (gz x +- a y)/k2
-            const double iK = bf.kinv[q], gz = g.gam * ((k <= nz) ? k : k - mz);
-            const double an = a * iK, gn = round == 0 ? -(gz * iK) : gz * iK;
+            // (the factors from a table: half of this kernel's time is FP64 issue;
+            // 192x96x96: 50 -> 44 us, and k_z3 39 -> 35 with its own)
+            const double2 f2 = bf.kfac[q];
+            const double an = f2.x, gn = round == 0 ? -f2.y : f2.y;
             fa = make_double2(-fma(an, x.y, gn * y.y), fma(an, x.x, gn * y.x));
-            const double gp = gz * iK, ap = round == 0 ? an : -an;
+            const double gp = f2.y, ap = round == 0 ? an : -an;
             fb = make_double2(-fma(gp, x.y, ap * y.y), fma(gp, x.x, ap * y.x));
             if (z00) {
               const double2 m = ((const double2 *)(round == 0 ? bf.mu : bf.mdu))[(long)b * g.my + j];
@@ -639,7 +640,8 @@ __global__ void __launch_bounds__(Z3<NZ, TEMP>::T, Z3<NZ, TEMP>::kMinB) k_z3(Gri
     double2 H1 = get(0), H2 = get(1), H3 = get(2);
     const double nn = nan("");
     if (bad) H1 = H2 = H3 = make_double2(nn, nn);
-    const double gz = g.gam * ((k <= nz) ? k : k - mz), gn = gz * norm;
+    const double2 g0 = bf.gzk[2 * k], g1 = bf.gzk[2 * k + 1];  // gz, gz norm; gz s, gz^2 norm
+    const double gn = g0.y;
     const long q = (long)k * nkx + i;
     const double2 v = Gv[q];
     if (TEMP) {
@@ -654,11 +656,11 @@ __global__ void __launch_bounds__(Z3<NZ, TEMP>::T, Z3<NZ, TEMP>::kMinB) k_z3(Gri
     // dvordy = i a H1 + i gz H3
     Dn[q] = make_double2(-fma(an, H1.y, gn * H3.y), fma(an, H1.x, gn * H3.x));
     // hg = -i a H3 + i gz (H1 - s v)
-    const double gs = gz * g.s;
+    const double gs = g1.x;
     Gn[q] = make_double2(-fma(-gs, v.y, fma(gn, H1.y, -(an * H3.y))),
                          fma(-gs, v.x, fma(gn, H1.x, -(an * H3.x))));
     // hv = -(kx^2 + kz^2) H2
-    const double Kn = fma(a, an, gz * gn);
+    const double Kn = fma(a, an, g1.y);
     double2 hv = make_double2(-(Kn * H2.x), -(Kn * H2.y));
     if (force && i == 0 && k == 1) hv.x += fj;
     Vv[q] = hv;
