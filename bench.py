@@ -160,8 +160,8 @@ def measured_peaks():
 
 def plane2_traffic():
     """dram bytes per launch of plane stage 2 from the committed ncu summary
-    (profiles/k_p2_192x96x96.txt, line 'traffic_bytes_per_launch: N'), else None."""
-    path = os.path.join(ROOT, "profiles", "k_p2_192x96x96.txt")
+    (profiles/k_x2_192x96x96.txt, line 'traffic_bytes_per_launch: N'), else None."""
+    path = os.path.join(ROOT, "profiles", "k_x2_192x96x96.txt")
     try:
         with open(path) as f:
             for line in f:
@@ -581,16 +581,14 @@ def run_ours(args):
     status = box.status()
     ms_max = allmax(dist, ms)
     steps_per_s = ws * args.steps / (ms_max * 1e-3)
-    # per step: 3 substeps x (3 plane stages, scalars, tables, 2 line kernels),
-    # the spectra and plane sums of the statistics at substep 1, the
-    # end-of-step kernel; LES adds 5 per substep; the fused y-line form runs
-    # one line kernel per substep instead of two; + 4 entry launches
-    # (the implicit variant: k_hfac + k_lineI per substep in place of the two
-    # line kernels)
-    per_step = (39 if args.variant == "les" else 24) - (3 if tuning.get("line_form") == "fused"
-                                                         else 0)
+    # per step: 3 substeps x (3 plane stages, scalars, phase tables, 2 line
+    # kernels), the spectra and plane sums of the statistics at substep 1, the
+    # end-of-step kernel; LES adds 5 per substep; one line kernel per substep
+    # (k_lineQ) without the temperature, which adds its own; + 4 entry launches
+    per_step = (39 if args.variant == "les" else 24) - (
+        3 if tuning.get("line_form") in ("fused", "implicit") else 0)
     if args.variant == "implicit-temperature":
-        per_step += 3  # the scalar's factor tables
+        per_step += 3
     launches = per_step * args.steps + 4
     if args.lite:
         # profiling runs (ncu): the timed steps only, no side measurements
@@ -637,7 +635,7 @@ def run_ours(args):
     k1.record(stream)
     k1.synchronize()
     line_ms = (line_ms, k0.elapsed_time(k1) / 5)
-    # the fused y-line kernel (the step's default form where available)
+    # k_lineQ (the step's y-line kernel; the two before are the banded form's)
     lineF_ms = None
     if box.tuning()["line_form"] == "fused":
         box.set_state(st0)
@@ -774,16 +772,18 @@ def run_ours(args):
                                 "max": float(calls_ms.max())}},
         "gpu_launches": launches,
         "roofline": {
-            "bound": "fp64", "kernel": "k_p2 (plane stage 2: x transforms, u x omega)",
+            "bound": "fp64",
+            "kernel": "k_x2 (plane stage 2 in 64-bit fixed point: x transforms, u x omega)",
             "achieved": p2_tflops, "peak": fp64_peak, "unit": "TFLOP/s",
             "frac": p2_tflops / fp64_peak,
-            "peak_source": "FP64 FMA probe measured in this run (GB300 FP64 is the binding roof)",
+            "peak_source": ("FP64 FMA probe measured in this run; the kernel computes on "
+                            "64-bit integers, so it may exceed it"),
             "algorithmic_flops_per_launch": p2_flops, "launch_ms": p2_ms,
             "hbm": {"achieved": p2_gbs, "peak": hbm_peak, "unit": "GB/s",
                     "frac": p2_gbs / hbm_peak, "peak_source": f"MEASURED_PEAKS.json ({hbm_src})",
                     "algorithmic_bytes_per_launch": p2_bytes},
             "traffic": traffic,
-            "line_kernels_ms": {"k_lineA": line_ms[0], "k_lineB": line_ms[1], "k_lineF": lineF_ms},
+            "line_kernels_ms": {"k_lineA": line_ms[0], "k_lineB": line_ms[1], "k_lineQ": lineF_ms},
         },
         "mixed_value": mixed["value"] if mixed else None,
         "mixed_speedup": mixed["speedup_vs_fp64"] if mixed else None,

@@ -263,10 +263,11 @@ int sb_kspace_get(sb_kspace *ks, int col, long off, long len, double *host);
 /* Measurement hooks (no counterpart in the reference; used by the benchmark).
  * sb_launch_stage enqueues `count` launches of one kernel of substep rk on the
  * handle's stream: stage 1..3 the plane stages, 4 the per-box phase tables,
- * 5 and 6 the two y-line kernels of the split form, 12 the fused y-line kernel
- * (handles without temperature or y filter/dealiasing); with LES, 7..10 the four
- * LES plane kernels and 11 the LES y-line kernel; with implicit_visc, 13 the
- * factorisation of the substep's Helmholtz operators and 14 its y-line
+ * 5 and 6 the two banded y-line kernels of the split form, 12 the step's one
+ * y-line kernel (handles on Bloch waves, see sb_set_line_form, or without
+ * temperature or y filter/dealiasing); with LES, 7..10 the four LES plane
+ * kernels and 11 the LES y-line kernel; with implicit_visc, 13 the
+ * factorisation of the substep's Helmholtz operators and 14 its banded y-line
  * kernel.  The launches act on the current device state, so a run that used
  * them must set the state again before stepping.
  * sb_fp64_peak measures the device's FP64 FMA throughput in TFLOP/s. */
@@ -293,12 +294,14 @@ int sb_physical_fields(sb_handle *h, int member, unsigned mask, double *out);
  * sb_set_line_segments sets the warps per line solve directly (1..3; my - 3 >=
  * 6 rows per segment).
  * sb_set_line_form chooses the y-line kernels of a substep: 1 (the default
- * where available) one fused kernel that takes each group of lines through all
- * its solves, 0 the split pair; form 1 needs a handle without temperature or y
- * filter/dealiasing (otherwise error 1, and such handles always run form 0).
- * sb_get_line_form gives the form the step graph uses (2 for a handle with
- * implicit_visc, whose substeps run the semi-implicit y-line kernel).  Both
- * forms compute the same step (to the last bits in FP64).
+ * where available) one kernel that takes each group of lines through all its
+ * solves, 0 the banded kernels, split.  The default runs on Bloch waves where
+ * my is 32, 48, 64, 80, 96, 128, 160, 192, 256, 320 or 384, without y filter or
+ * dealiasing, while every box has xoffb = -xofft; else with banded solves.
+ * Setting form 1 needs a handle without temperature, implicit_visc or y
+ * filter/dealiasing (otherwise error 1).  sb_get_line_form gives 1 or 0, 0 with
+ * the temperature, 2 with implicit_visc.  All compute the same step (to FP64
+ * rounding).
  * sb_set_side_branch chooses which side work of a substep the step graph runs
  * as a branch concurrent with the plane stages: bit 0 the spectra of a
  * statistics step (beside plane stages 1-2), bit 1 the per-box scalars and

@@ -1,7 +1,9 @@
-// sb_kernels.cu -- FP64 kernels of the shearing-box RK3 substep on sm_103a.
+// sb_kernels.cu -- plane stages of the shearing-box RK3 substep on sm_103a: the
+// FP32-mixed form, LES handles, the physical fields and the statistics (FP64
+// handles without LES run stages 1-3 of sb_planeq.cu).
 //
 // One RK3 substep of the reference (cross.f90:428-1000, explicit branch,
-// iadd_mode=5) is five launches:
+// iadd_mode=5):
 //   k_spectra  (first substep of a statistics step, beside stages 1-2) hist
 //           plane sums and kx-kz spectra (cross.f90:1796-2014)
 //   k_p1    per (plane, kx block): u, w, omega_x, omega_z from v, omega_y
@@ -13,9 +15,9 @@
 //   k_p3    per (plane, kx block): forward z-transforms, 1/(mgalx*mgalz) scaling and
 //           truncation (pack00), right-hand sides of iadd_mode 5
 //           (cross.f90:1536-1546) and the mean-mode forcing (cross.f90:1489-1490)
-//   k_phase per box: Delta t from the CFL (cross.f90:1598-1711), the UNER record
+//   k_scalar per box (sb_box.cu): Delta t from the CFL (cross.f90:1598-1711), the UNER record
 //           (cross.f90:2064-2118), shear offsets and phase tables
-//   k_line  per (kx, kz) y-line: every y-operator of the substep in one pass --
+//   k_lineQ per (kx, kz) y-line (sb_bloch.cu): every y-operator of the substep --
 //           derivyc of d(omega_y)/dy, the viscous terms (visc3d), the RK3 update
 //           (cross.f90:694-723), the zeta store and moving_frame remaps
 //           (cross.f90:752-781), the Helmholtz solve for v (lapcdy, cross.f90:784-795)

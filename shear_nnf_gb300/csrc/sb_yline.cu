@@ -1,4 +1,7 @@
-// sb_yline.cu -- y-line stage, per-box scalars and phase tables of the RK3 step.
+// sb_yline.cu -- the banded y-line stage of the RK3 step: line lengths without a
+// transform plan, the y filter and dealiasing, boxes whose image offsets do not
+// mirror each other, and the split form on request (all else runs k_lineQ,
+// sb_bloch.cu).
 //
 // The y-operators of one substep (cross.f90:565-795 and the first derivatives of
 // the next substep, cross.f90:434-445) run as two kernels so that independent
