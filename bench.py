@@ -618,7 +618,8 @@ def run_ours(args):
     k1.record(stream)
     k1.synchronize()
     p2_ms = k0.elapsed_time(k1) / nrep
-    # line kernel alone, for the record
+    # line kernel alone, for the record (the first banded launch builds its tables)
+    box.launch_stage(5, 2, 1)
     box.set_state(st0)
     box.step(1)
     box.sync()
@@ -772,16 +773,16 @@ def run_ours(args):
                                 "max": float(calls_ms.max())}},
         "gpu_launches": launches,
         "roofline": {
-            "bound": "fp64",
+            "bound": "integer issue",
             "kernel": "k_x2 (plane stage 2 in 64-bit fixed point: x transforms, u x omega)",
-            "achieved": p2_tflops, "peak": fp64_peak, "unit": "TFLOP/s",
-            "frac": p2_tflops / fp64_peak,
-            "peak_source": ("FP64 FMA probe measured in this run; the kernel computes on "
-                            "64-bit integers, so it may exceed it"),
-            "algorithmic_flops_per_launch": p2_flops, "launch_ms": p2_ms,
-            "hbm": {"achieved": p2_gbs, "peak": hbm_peak, "unit": "GB/s",
-                    "frac": p2_gbs / hbm_peak, "peak_source": f"MEASURED_PEAKS.json ({hbm_src})",
-                    "algorithmic_bytes_per_launch": p2_bytes},
+            "achieved": p2_gbs, "peak": hbm_peak, "unit": "GB/s", "frac": p2_gbs / hbm_peak,
+            "peak_source": f"MEASURED_PEAKS.json ({hbm_src})",
+            "algorithmic_bytes_per_launch": p2_bytes, "launch_ms": p2_ms,
+            # the same flops on the FP64 pipe, which the kernel replaces by integers
+            "fp64_equivalent": {"achieved": p2_tflops, "peak": fp64_peak, "unit": "TFLOP/s",
+                                "ratio": p2_tflops / fp64_peak,
+                                "peak_source": "FP64 FMA probe measured in this run",
+                                "algorithmic_flops_per_launch": p2_flops},
             "traffic": traffic,
             "line_kernels_ms": {"k_lineA": line_ms[0], "k_lineB": line_ms[1], "k_lineQ": lineF_ms},
         },
