@@ -231,7 +231,9 @@ int sb_packed_shift_tangent(sb_handle *h, const double *x, double *out, int dir)
  * stream NULL gives the space its own stream; pass a handle's stream
  * (sb_get_stream) to order the space's work with that handle's.
  *   sb_kspace_gram       C[a][b] = <col a0+a, col b0+b>, m x p, row-major host
- *                        array; fixed-order reductions (bitwise reproducible)
+ *                        array; fixed-order reductions (bitwise reproducible),
+ *                        to the error of FP64 sums: a few 2^-53 of sum |x y|,
+ *                        whatever the sizes of the entries
  *   sb_kspace_update     col b0+b += alpha sum_a col a0+a C[a][b] (ranges
  *                        must not overlap; C host m x p row-major)
  *   sb_kspace_transform  cols b0..b0+p-1 <- (cols b0..) M, p <= 64, in place

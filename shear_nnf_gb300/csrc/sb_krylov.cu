@@ -133,6 +133,19 @@ k_gram_sum(const double *__restrict__ part, int nchunk, int m, int p, double *__
 // FP64 fused multiply-add) and drops lo*lo, 2^-59 of the largest product.  The
 // chunk's sums are exact, |sum| < 2^123, kept to 2^60, and meet in FP64.  At
 // most 16 rows meet in one cross sum (< 2^62) before its upper bits move to hi.
+//
+// A chunk is off by at most 80 x 2^60: each row's half units of both entries
+// (2^58), its lo*lo (2^58), half a unit for each of up to 32 slices.  An FP64
+// sum is off by units of 2^-53 of sum |x y|, so the integers stand where that
+// is at least 2^kQSum = 2^114 (then the error is below 40 x 2^-53 of it, where
+// 128 FP64 additions allow 128), and a pair of columns whose large entries do
+// not meet takes the FP64 sum.  sum |x y| is bounded from below by |sum x y|
+// and, where that is small, by the sum over the entries' upper 8 bits (four rows
+// an instruction); the two largest entries meeting suffice (128 x 128 = 2^14).
+// 187488 rows, 48 x 16: 161 us on normal entries, 202 on rows that fall by
+// e^-0.25, 411 on entries over 40 decades, where most pairs take the FP64 sum
+// (the FP64 kernel 490-510 on each; without the test 150, with errors up to
+// 2^-48 of sum |x y| on the last and of any size on columns that hardly meet).
 // Chunks that hold an infinity, a NaN or numbers beyond 2^+-400 take FP64 sums.
 //
 // Tile: 64 x 16 columns, 4 x 4 products per thread, the rows split over ks
@@ -145,11 +158,18 @@ constexpr int kQA = 64, kQB = 16;  // columns of a tile
 constexpr int kQR = 128;           // rows of a chunk
 constexpr int kQS = kQR + 2;       // column stride: odd in 16-byte units
 constexpr int kQLim = 400;
+constexpr int kQSum = 114;           // of the smallest sum of |products| (see above)
+constexpr int kQTop = kQBits - 8;    // of an entry's upper 8 bits
+constexpr unsigned kQTops = 1u << (kQSum - 2 * kQTop);  // kQSum in products of those
+constexpr int kQBS = kQR / 4 + 1;    // words of a column's upper bits, odd
+constexpr int kQZero = 1 << 20;      // the power of two of a column of zeros
 
 __device__ __forceinline__ int2 qsplit(long long x) {
   const int lo = ((int)x << (32 - kQLow)) >> (32 - kQLow);
   return make_int2(lo, (int)((x - lo) >> kQLow));
 }
+// the upper 8 bits of an entry's modulus
+__device__ __forceinline__ unsigned qtop(int2 x) { return min((unsigned)abs(x.y) >> (kQTop - kQLow), 255u); }
 // 8 bytes global -> shared, zeros where !on
 __device__ __forceinline__ void copy8(void *dst, const void *src, bool on) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(
@@ -166,6 +186,12 @@ k_gramq(const double *__restrict__ V, long ld, long r0, long r1, int ks, int a0,
         int p, double *__restrict__ part) {
   extern __shared__ __align__(16) int2 sx[];
   __shared__ int sp[kQA + kQB];  // the columns' powers of two
+  __shared__ unsigned st[(kQA + kQB) * kQBS];  // upper bits of rows l, l + 32, l + 64, l + 96
+  // the chunk's pairs of columns that take the FP64 sum
+  __shared__ unsigned short s_pair[kQA * kQB];
+  __shared__ double s_dot[kQA * kQB];
+  __shared__ int s_low;
+  if (threadIdx.x == 0) s_low = 0;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ta = blockIdx.y * kQA, tb = blockIdx.z * kQB;
   const int mt = min(kQA, m - ta), pt = min(kQB, p - tb), nc = mt + pt;
@@ -204,9 +230,15 @@ k_gramq(const double *__restrict__ V, long ld, long r0, long r1, int ks, int a0,
       const int E = (int)(t >> 20) - 1023;
       bad |= t != 0 && (E > kQLim || E < -kQLim);
       const sb::QScale sc = sb::qscale(t, kQBits);
+      unsigned tops = 0;
 #pragma unroll
-      for (int u = 0; u < kQR / 32; u++) sx[c * kQS + lane + 32 * u] = qsplit(sb::tofix(x[u], sc));
-      if (lane == 0) sp[c] = t ? sc.p : 0;
+      for (int u = 0; u < kQR / 32; u++) {
+        const int2 v = qsplit(sb::tofix(x[u], sc));
+        sx[c * kQS + lane + 32 * u] = v;
+        tops |= qtop(v) << (8 * u);
+      }
+      st[c * kQBS + lane] = tops;
+      if (lane == 0) sp[c] = t ? sc.p : kQZero;
     }
     if (__syncthreads_or(bad)) {
       for (int i = 0; i < 4; i++) {
@@ -268,15 +300,49 @@ k_gramq(const double *__restrict__ V, long ld, long r0, long r1, int ks, int a0,
         for (int j = 0; j < 4; j++)
           red[((sl * 4 + i) * 4 + j) * nq + q] = hi[i][j] + (cr[i][j] >> (kQLow - 1));
     __syncthreads();
+    int low[4] = {-1, -1, -1, -1};
     if (sl < 4) {
 #pragma unroll
       for (int i = 0; i < 4; i++) {
         long long t = 0;
         for (int k = 0; k < ks; k++) t += red[((k * 4 + i) * 4 + sl) * nq + q];
-        const int a = min(ga + i * GA, mt - 1), b = mt + min(gb + sl * GB, pt - 1);
-        out[i] += sb::fromfix(t, 2 * kQLow - sp[a] - sp[b]);
+        const bool in = ga + i * GA < mt && gb + sl * GB < pt;
+        const int a = min(ga + i * GA, mt - 1), b = min(gb + sl * GB, pt - 1);
+        const int pab = sp[a] + sp[mt + b];
+        if (in && abs(t) < 1ll << (kQSum - 2 * kQLow) && pab < kQZero / 2) {
+          unsigned d = 0;
+#pragma unroll 8
+          for (int l = 0; l < kQR / 4; l++)
+            d = __dp4a(st[a * kQBS + l], st[(mt + b) * kQBS + l], d);
+          if (d < kQTops) {
+            low[i] = atomicAdd(&s_low, 1);
+            s_pair[low[i]] = (unsigned short)(a | b << 8);
+          }
+        }
+        if (low[i] < 0) out[i] += sb::fromfix(t, 2 * kQLow - pab);
       }
     }
+    __syncthreads();
+    const int nlow = s_low;
+    if (nlow == 0) continue;
+    // the FP64 sums, L lanes a pair
+    const int L = nlow > kThreads / 8 ? 4 : nlow > kThreads / 16 ? 8 : nlow > kThreads / 32 ? 16 : 32;
+    for (int k = tid / L; k < (nlow + 31) / 32 * 32; k += kThreads / L) {
+      double v = 0.0;
+      if (k < nlow) {
+        const int a = s_pair[k] & 255, b = s_pair[k] >> 8;
+        const double *x = col(a) + lo, *y = col(mt + b) + lo;
+#pragma unroll 4
+        for (int r = tid % L; r < nr; r += L) v = fma(x[r], y[r], v);
+      }
+      for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (k < nlow && tid % L == 0) s_dot[k] = v;
+    }
+    __syncthreads();
+    if (tid == 0) s_low = 0;
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      if (low[i] >= 0) out[i] += s_dot[low[i]];
     __syncthreads();
   }
 #pragma unroll
@@ -665,9 +731,9 @@ cudaError_t prepare_fixed() {
   return e;
 }
 // The fixed-point forms from 16 coefficients on.  187488 rows, whole calls,
-// FP64 against fixed point: products 48 x 16 489 -> 144 us, 32 x 1 179 -> 80,
-// 16 x 2 118 -> 57, 4 x 4 the same (56); updates 260 -> 100, 106 -> 37,
-// 63 -> 26, 27 -> 18.  Below, the conversions cost what the sums save.
+// FP64 against fixed point: products 48 x 16 492 -> 161 us, 32 x 1 182 -> 88,
+// 16 x 2 120 -> 71, 4 x 4 the same (58); updates 263 -> 108, 110 -> 41,
+// 64 -> 30, 30 -> 23.  Below, the conversions cost what the sums save.
 bool fixed_ok(int m, int p) { return (long)m * p >= 16; }
 
 }  // namespace
