@@ -235,7 +235,8 @@ int sb_packed_shift_tangent(sb_handle *h, const double *x, double *out, int dir)
  *                        to the error of FP64 sums: a few 2^-53 of sum |x y|,
  *                        whatever the sizes of the entries
  *   sb_kspace_update     col b0+b += alpha sum_a col a0+a C[a][b] (ranges
- *                        must not overlap; C host m x p row-major)
+ *                        must not overlap; C host m x p row-major), to the
+ *                        error of FP64 sums likewise, W rounded once
  *   sb_kspace_transform  cols b0..b0+p-1 <- (cols b0..) M, p <= 64, in place
  *   sb_kspace_combine    col dst = sum_k coef[k] col src[k], nsrc <= 8
  *   sb_kspace_perturb    col dst = x0 + ((x0 + e d) - x0) (the representable

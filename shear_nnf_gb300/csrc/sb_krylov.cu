@@ -390,36 +390,58 @@ __device__ __forceinline__ long long qmad(int a, int b, long long c) {
 // C' = C 2^-da[a] has entries of about one in every row, and the row's scaled
 // entries V 2^da share a power of two, so that neither badly scaled columns
 // nor the range over the rows (wavenumbers) lose digits.  Three multiply-adds
-// a product as above; at most 64 products meet in one sum.  Rows with an
-// infinity, a NaN or numbers beyond 2^+-400 take the FP64 sums.  The rows come
-// by asynchronous copies, a thread its own, before the scale is taken.
-template <int NB>
-__global__ void __launch_bounds__(kUThreads)
+// a product as above; at most 64 products meet in one sum, off by at most
+// 33 x 2^60 (a quarter for each product's roundings and for its lo*lo, one at
+// the end).  As in k_gramq it stands where sum |v C'| is at least 2^kQSum by
+// the upper bits of both, or W is so large, 2^(kQSum + 2), that its own rounding
+// exceeds that; a column that picks small entries out of a row takes the FP64
+// sum.  So do rows with an infinity, a NaN or numbers beyond 2^+-400.  The rows
+// come by asynchronous copies, a thread its own, before the scale is taken.
+// 187488 rows, 48 x 16: 121 us on normal entries and on rows that fall by
+// e^-0.25, 281 on entries over 40 decades (FP64 263-277; without the test 108).
+// MANY: for m > 64 the parts' sums are kept, so that W is rounded once.
+template <int NB, bool MANY>
+__global__ void __launch_bounds__(kUThreads, MANY ? 2 : 3)
 k_updateq(double *__restrict__ V, long ld, long r0, long r1, int a0, int m, int b0, int p,
           const double *__restrict__ C, const int2 *__restrict__ CQ, const int *__restrict__ da,
           const int *__restrict__ pc, double alpha) {
   extern __shared__ __align__(16) int2 sx[];
-  const int mx = min(m, 64);
+  const int mx = min((m + 3) / 4 * 4, 64);
   int2 *sc = sx;                                 // coefficients [mx][NB]
   double *sv = (double *)(sx + mx * NB);         // rows of V [mx][kUThreads]
-  int *sd = (int *)(sv + mx * kUThreads);        // exponents [mx]
+  unsigned *st = (unsigned *)(sv + mx * kUThreads);  // upper bits of four rows of them [mx/4][NB]
+  int *sd = (int *)(st + mx / 4 * NB);           // exponents [mx]
   const int pp = (p + NB - 1) / NB * NB;
   const long r = r0 + (long)blockIdx.x * kUThreads + threadIdx.x;
   const int g = blockIdx.y * NB, nb = min(NB, p - g);
   const bool on = r < r1;
+  double *w = V + (long)(b0 + g) * ld + (on ? r : r1 - 1);
+  double sum[MANY ? NB : 1];  // over m > 64 columns of V: W is rounded once
+#pragma unroll
+  for (int b = 0; b < (MANY ? NB : 1); b++) sum[b] = 0.0;
+  auto add = [&](int b, double x) {
+    if constexpr (MANY) sum[b] += x;
+    else w[(long)b * ld] = fma(alpha, x, w[(long)b * ld]);
+  };
   for (int c0 = 0; c0 < m; c0 += 64) {
-    const int mc = min(64, m - c0);
+    const int mc = min(64, m - c0), m4 = (mc + 3) / 4 * 4;  // zeros from mc on
     const double *v = V + (long)(a0 + c0) * ld + (on ? r : r1 - 1);
     __syncthreads();
 #pragma unroll 8
-    for (int a = 0; a < mc; a++) copy8(sv + a * kUThreads + threadIdx.x, v + (long)a * ld, on);
-    for (int k = threadIdx.x; k < mc * NB; k += kUThreads)
-      sc[k] = CQ[(long)(c0 + k / NB) * pp + g + k % NB];
-    for (int k = threadIdx.x; k < mc; k += kUThreads) sd[k] = da[c0 + k];
+    for (int a = 0; a < m4; a++)
+      copy8(sv + a * kUThreads + threadIdx.x, v + (long)min(a, mc - 1) * ld, on && a < mc);
+    for (int k = threadIdx.x; k < m4 * NB; k += kUThreads) {
+      const int a = k / NB;
+      sc[k] = a < mc ? CQ[(long)(c0 + a) * pp + g + k % NB] : make_int2(0, 0);
+    }
+    for (int k = threadIdx.x; k < m4; k += kUThreads) sd[k] = k < mc ? da[c0 + k] : 0;
     copy_wait();
     __syncthreads();
-    if (!on) continue;
-    double *w = V + (long)(b0 + g) * ld + r;
+    for (int k = threadIdx.x; k < m4 / 4 * NB; k += kUThreads) {
+      const int2 *c = sc + k / NB * 4 * NB + k % NB;
+      st[k] = qtop(c[0]) | qtop(c[NB]) << 8 | qtop(c[2 * NB]) << 16 | qtop(c[3 * NB]) << 24;
+    }
+    __syncthreads();
     const double *mv = sv + threadIdx.x;
     int top = -100000, raw = 0;
 #pragma unroll 8
@@ -428,35 +450,78 @@ k_updateq(double *__restrict__ V, long ld, long r0, long r1, int a0, int m, int 
       raw = max(raw, e);
       if (e) top = max(top, e + sd[a]);
     }
-    if (raw == 0x7ff || top > 1023 + kQLim || top < 1023 - kQLim) {
-      for (int b = 0; b < nb; b++) {
-        double acc = 0.0;
-        for (int a = 0; a < mc; a++)
-          acc = fma(mv[a * kUThreads], C[(long)(c0 + a) * p + g + b], acc);
-        w[(long)b * ld] = fma(alpha, acc, w[(long)b * ld]);
+    bool plain = raw == 0x7ff || top > 1023 + kQLim || top < 1023 - kQLim;
+    if (p > 1) {
+      // a row with few entries near its largest would fall to FP64 in most
+      // columns after the integers: a warp of those takes it at once
+      int near = 0;
+#pragma unroll 8
+      for (int a = 0; a < mc; a++)
+        near += (int)(sb::hiword(mv[a * kUThreads]) >> 20) + sd[a] > top - 8;
+      plain |= __popc(__ballot_sync(0xffffffffu, on && 4 * near < mc)) > 16;
+    }
+    if (!on) continue;
+    auto dot = [&](int b) {
+      double acc = 0.0;
+#pragma unroll 2
+      for (int a = 0; a < mc; a++) acc = fma(mv[a * kUThreads], C[(long)(c0 + a) * p + g + b], acc);
+      return acc;
+    };
+    if (plain) {
+#pragma unroll
+      for (int b = 0; b < NB; b += 4) {
+        if (b >= nb) break;
+        double acc[4] = {0.0, 0.0, 0.0, 0.0};
+        const double *c = C + (long)c0 * p + g + b;
+#pragma unroll 4
+        for (int a = 0; a < mc; a++) {
+          const double x = mv[a * kUThreads];
+#pragma unroll
+          for (int q = 0; q < 4; q++) acc[q] = fma(x, c[(long)a * p + min(q, nb - b - 1)], acc[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+          if (b + q < nb) add(b + q, acc[q]);
       }
       continue;
     }
     const int pr = kQBits - (top - 1022);
     long long hi[NB], cr[NB];
+    unsigned tops[NB];
 #pragma unroll
-    for (int b = 0; b < NB; b++) hi[b] = cr[b] = 0;
-    for (int a = 0; a < mc;) {
-      const int end = min(mc, a + 16);
-#pragma unroll 2
-      for (; a < end; a++) {
-        sb::QScale s;
-        s.p = pr + sd[a];
-        const int2 x = qsplit(sb::tofix(mv[a * kUThreads], s));
+    for (int b = 0; b < NB; b++) {
+      hi[b] = cr[b] = 0;
+      tops[b] = 0;
+    }
+    for (int a = 0; a < m4;) {
+      const int end = min(m4, a + 16);
+#pragma unroll 1
+      for (; a < end; a += 4) {
+        unsigned xt = 0;
 #pragma unroll
-        for (int b = 0; b < NB; b += 2) {
-          const int4 c = *reinterpret_cast<const int4 *>(sc + a * NB + b);
-          hi[b] = qmad(x.y, c.y, hi[b]);
-          cr[b] = qmad(x.x, c.y, cr[b]);
-          cr[b] = qmad(x.y, c.x, cr[b]);
-          hi[b + 1] = qmad(x.y, c.w, hi[b + 1]);
-          cr[b + 1] = qmad(x.x, c.w, cr[b + 1]);
-          cr[b + 1] = qmad(x.y, c.z, cr[b + 1]);
+        for (int u = 0; u < 4; u++) {
+          sb::QScale s;
+          s.p = pr + sd[a + u];
+          const int2 x = qsplit(sb::tofix(mv[(a + u) * kUThreads], s));
+          xt |= qtop(x) << (8 * u);
+#pragma unroll
+          for (int b = 0; b < NB; b += 2) {
+            const int4 c = *reinterpret_cast<const int4 *>(sc + (a + u) * NB + b);
+            hi[b] = qmad(x.y, c.y, hi[b]);
+            cr[b] = qmad(x.x, c.y, cr[b]);
+            cr[b] = qmad(x.y, c.x, cr[b]);
+            hi[b + 1] = qmad(x.y, c.w, hi[b + 1]);
+            cr[b + 1] = qmad(x.x, c.w, cr[b + 1]);
+            cr[b + 1] = qmad(x.y, c.z, cr[b + 1]);
+          }
+        }
+#pragma unroll
+        for (int b = 0; b < NB; b += 4) {
+          const uint4 c = *reinterpret_cast<const uint4 *>(st + a / 4 * NB + b);
+          tops[b] = __dp4a(xt, c.x, tops[b]);
+          tops[b + 1] = __dp4a(xt, c.y, tops[b + 1]);
+          tops[b + 2] = __dp4a(xt, c.z, tops[b + 2]);
+          tops[b + 3] = __dp4a(xt, c.w, tops[b + 3]);
         }
       }
 #pragma unroll
@@ -467,14 +532,25 @@ k_updateq(double *__restrict__ V, long ld, long r0, long r1, int a0, int m, int 
     }
     // hi < 2^(56 + bits of mc): the sum as one integer, 2^(60 - up)
     const int up = mc > 32 ? 0 : mc > 16 ? 1 : mc > 8 ? 2 : 3;
+    // exponent field of a W that makes up for any error of the sum
+    const int we = 1023 + kQSum + 2 + sb::qexp(alpha) + 1;
 #pragma unroll
     for (int b = 0; b < NB; b++)
       if (b < nb) {
-        const long long t = (hi[b] << up) + ((cr[b] + (1ll << (kQLow - 1 - up))) >> (kQLow - up));
-        const double acc = sb::fromfix(t, 2 * kQLow - up - pr - pc[g + b]);
-        w[(long)b * ld] = fma(alpha, acc, w[(long)b * ld]);
+        const int pb = pr + pc[g + b];
+        if (tops[b] < kQTops && (int)(sb::hiword(w[(long)b * ld]) >> 20) < we - pb) {
+          add(b, dot(b));
+        } else {
+          const long long t = (hi[b] << up) + ((cr[b] + (1ll << (kQLow - 1 - up))) >> (kQLow - up));
+          add(b, sb::fromfix(t, 2 * kQLow - up - pb));
+        }
       }
   }
+  if constexpr (MANY)
+    if (on)
+#pragma unroll
+      for (int b = 0; b < NB; b++)
+        if (b < nb) w[(long)b * ld] = fma(alpha, sum[b], w[(long)b * ld]);
 }
 
 // the coefficients' integers and exponents for k_updateq; false where a
@@ -721,19 +797,28 @@ void gramq_plan(long rows, int m, int p, int *ks, int *nblk, size_t *smem) {
   *smem = std::max(sizeof(int2) * (size_t)(mt + pt) * kQS, sizeof(long long) * 16 * nq * *ks);
 }
 constexpr int kGramSmem = (int)sizeof(int2) * (kQA + kQB) * kQS;
-constexpr int kUpdSmem = 64 * (16 * (int)sizeof(int2) + kUThreads * (int)sizeof(double) + 4);
+// shared memory of k_updateq for mx (a multiple of 4) columns at a time
+size_t update_smem(int mx, int nb) {
+  return (sizeof(int2) * nb + sizeof(double) * kUThreads + sizeof(int) * nb / 4 + sizeof(int)) * mx;
+}
 cudaError_t prepare_fixed() {
   constexpr auto A = cudaFuncAttributeMaxDynamicSharedMemorySize;
   cudaError_t e = cudaFuncSetAttribute(k_gramq, A, kGramSmem);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_updateq<4>, A, kUpdSmem);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_updateq<8>, A, kUpdSmem);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_updateq<16>, A, kUpdSmem);
+#define SB_PREP(NB, MANY) \
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_updateq<NB, MANY>, A, (int)update_smem(64, NB))
+  SB_PREP(4, false);
+  SB_PREP(8, false);
+  SB_PREP(16, false);
+  SB_PREP(4, true);
+  SB_PREP(8, true);
+  SB_PREP(16, true);
+#undef SB_PREP
   return e;
 }
 // The fixed-point forms from 16 coefficients on.  187488 rows, whole calls,
 // FP64 against fixed point: products 48 x 16 492 -> 161 us, 32 x 1 182 -> 88,
-// 16 x 2 120 -> 71, 4 x 4 the same (58); updates 263 -> 108, 110 -> 41,
-// 64 -> 30, 30 -> 23.  Below, the conversions cost what the sums save.
+// 16 x 2 120 -> 71, 4 x 4 the same (58); updates 263 -> 121, 110 -> 42,
+// 64 -> 31, 30 -> 26.  Below, the conversions cost what the sums save.
 bool fixed_ok(int m, int p) { return (long)m * p >= 16; }
 
 }  // namespace
@@ -942,14 +1027,21 @@ int sb_kspace_update(sb_kspace *ks, long r0, long r1, int a0, int m, int b0, int
     const dim3 grid((unsigned)((r1 - r0 + kUThreads - 1) / kUThreads), (unsigned)(pp / nb));
     const int *e = (const int *)(ks->small + oe);
     const int2 *cq = (const int2 *)(ks->small + oq);
-    const int mx = std::min(m, 64);
-    const size_t smem = sizeof(int2) * mx * nb + sizeof(double) * mx * kUThreads + sizeof(int) * mx;
-#define SB_UPD(NB)                                                                              \
-  k_updateq<NB><<<grid, kUThreads, smem, ks->st>>>(ks->V, ks->ld, r0, r1, a0, m, b0, p, ks->small, \
-                                                   cq, e, e + m, alpha)
-    if (nb == 16) SB_UPD(16);
-    else if (nb == 8) SB_UPD(8);
-    else SB_UPD(4);
+    const size_t smem = update_smem(std::min((m + 3) / 4 * 4, 64), nb);
+#define SB_UPD(NB, MANY)                                                                       \
+  k_updateq<NB, MANY><<<grid, kUThreads, smem, ks->st>>>(ks->V, ks->ld, r0, r1, a0, m, b0, p,    \
+                                                         ks->small, cq, e, e + m, alpha)
+#define SB_UPDM(NB) \
+  if (m > 64) SB_UPD(NB, true); \
+  else SB_UPD(NB, false)
+    if (nb == 16) {
+      SB_UPDM(16);
+    } else if (nb == 8) {
+      SB_UPDM(8);
+    } else {
+      SB_UPDM(4);
+    }
+#undef SB_UPDM
 #undef SB_UPD
   } else {
     k_update<<<(unsigned)((r1 - r0 + kThreads - 1) / kThreads), kThreads, 0, ks->st>>>(
