@@ -18,7 +18,6 @@
 #include <cstdarg>
 #include <cstdio>
 #include <string>
-#include <vector>
 
 #include "../../include/shearbox.h"
 #include "sb_common.cuh"
@@ -556,7 +555,8 @@ k_updateq(double *__restrict__ V, long ld, long r0, long r1, int a0, int m, int 
 // the coefficients' integers and exponents for k_updateq; false where a
 // number is not finite or too far from one
 bool fix_coefs(const double *C, int m, int p, int pp, int2 *q, int *da, int *pc) {
-  std::vector<int> top(p, -100000);
+  int *top = pc;  // of the columns, then their powers of two
+  for (int b = 0; b < p; b++) top[b] = -100000;
   for (int a = 0; a < m; a++) {
     int e = 0;
     for (int b = 0; b < p; b++) e = std::max(e, (int)(sb::hiword(C[(long)a * p + b]) >> 20));
