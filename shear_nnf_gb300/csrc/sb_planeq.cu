@@ -243,13 +243,14 @@ __global__ void __launch_bounds__(X2<NX, TEMP, NP>::T, 65536 / (X2<NX, TEMP, NP>
   extern __shared__ __align__(16) unsigned char smx_raw[];
   q2 *ex = (q2 *)smx_raw;
   __shared__ int s_e[NP * NF], s_len[NP * NF], s_ho[NP * NO], s_hl[NP * NO];
-  __shared__ ll s_third[NP][3];
+  // sums of the third moments: in units of 2^16 and what is left
+  __shared__ ll s_third[NP][3], s_rest[NP][3];
   const int nkx = g.nkx, NZ = g.mgalz, z0 = 2 * NP * blockIdx.x;
   const int lane = threadIdx.x & 31;
   auto P = [](int x) { return x + x / R2; };
   if (threadIdx.x < NP * NF) s_len[threadIdx.x] = kNoLen;
   if (threadIdx.x < NP * NO) s_hl[threadIdx.x] = kNoLen;
-  if (threadIdx.x < 3 * NP) (&s_third[0][0])[threadIdx.x] = 0;
+  if (threadIdx.x < 3 * NP) (&s_third[0][0])[threadIdx.x] = (&s_rest[0][0])[threadIdx.x] = 0;
   // ---- rows in: one warp per sequence.  Two rows in one complex sequence
   // (Hermitian extension; FFTW's c2r ignores the imaginary part of kx = 0)
   {
@@ -387,10 +388,14 @@ __global__ void __launch_bounds__(X2<NX, TEMP, NP>::T, 65536 / (X2<NX, TEMP, NP>
         if (TEMP) tm = max(tm, max(max(F[NF - 1].x, -F[NF - 1].x), max(F[NF - 1].y, -F[NF - 1].y)));
       }
       if (hist) {
-        // v u^2, v w^2, v^3 (cross.f90:2038-2042), < 2^55 each; 2^-6 of them is summed
-        t1 += (qprod(u2.x, qprod(u1.x, u1.x)) >> 6) + (qprod(u2.y, qprod(u1.y, u1.y)) >> 6);
-        t2 += (qprod(u2.x, qprod(u3.x, u3.x)) >> 6) + (qprod(u2.y, qprod(u3.y, u3.y)) >> 6);
-        t3 += (qprod(u2.x, qprod(u2.x, u2.x)) >> 6) + (qprod(u2.y, qprod(u2.y, u2.y)) >> 6);
+        // v u^2, v w^2, v^3 (cross.f90:2038-2042) of the doubled fields, < 2^58
+        // each, a thread's (at most 8) and a row pair's summed exactly: the
+        // roundings are below 2^-55 of the sum of |products| (with 55 bits and
+        // the last six of each dropped 7e-14 of it)
+        const q2 d1 = qdbl(u1), d2 = qdbl(u2), d3 = qdbl(u3);
+        t1 += qprod(d2.x, qprod(d1.x, d1.x)) + qprod(d2.y, qprod(d1.y, d1.y));
+        t2 += qprod(d2.x, qprod(d3.x, d3.x)) + qprod(d2.y, qprod(d3.y, d3.y));
+        t3 += qprod(d2.x, qprod(d2.x, d2.x)) + qprod(d2.y, qprod(d2.y, d2.y));
       }
       q2 h1, h2, h3;
       h1.x = al(qprod(u2.x, w3.x), o1 - a1) - al(qprod(u3.x, w2.x), o1 - a2);
@@ -461,9 +466,22 @@ __global__ void __launch_bounds__(X2<NX, TEMP, NP>::T, 65536 / (X2<NX, TEMP, NP>
       if (TEMP) mt = fmax(mt, fromfix_big(tm, e[NF - 1]));
     }
     if (hist) {
-      atomicAdd((ull *)&s_third[p][0], (ull)t1);
-      atomicAdd((ull *)&s_third[p][1], (ull)t2);
-      atomicAdd((ull *)&s_third[p][2], (ull)t3);
+      // the warp's sums by 32-bit reductions of 24-bit pieces, then one lane's
+      // atomics (a 192x96x96 step 829 us; with every lane's six 933, with three
+      // 885)
+      static_assert(2 * ((NX + T - 1) / T) <= 8, "a thread's sum below 2^62");
+      const ll t[3] = {t1, t2, t3};
+#pragma unroll
+      for (int q = 0; q < 3; q++) {
+        const unsigned lo = __reduce_add_sync(0xffffffffu, (unsigned)t[q] & 0xffffffu);
+        const unsigned mid = __reduce_add_sync(0xffffffffu, (unsigned)(t[q] >> 24) & 0xffffffu);
+        const int hi = __reduce_add_sync(0xffffffffu, (int)(t[q] >> 48));
+        if (lane == 0) {
+          const ll r = ((ll)mid << 24) + lo;
+          atomicAdd((ull *)&s_third[p][q], (ull)(((ll)hi << 32) + (r >> 16)));
+          atomicAdd((ull *)&s_rest[p][q], (ull)(r & 0xffff));
+        }
+      }
     }
   }
   if (rk == 1) {
@@ -482,8 +500,9 @@ __global__ void __launch_bounds__(X2<NX, TEMP, NP>::T, 65536 / (X2<NX, TEMP, NP>
     bool bad = false;
     for (int f = 0; f < NF; f++) bad |= s_e[p * NF + f] >= kBad;
     const int e2 = q == 0 ? ef(0) : q == 1 ? ef(1) : ef(4);
+    const int et = ef(4) + 2 * e2 + 128 - 3;
     bf.ppart[(((long)b * g.my + j) * (NZ / 2) + z0 / 2 + p) * 3 + q] =
-        bad ? nan("") : fromfix_big(s_third[p][q], ef(4) + 2 * e2 + 128 + 6);
+        bad ? nan("") : fromfix_big(s_third[p][q], et + 16) + fromfix_big(s_rest[p][q], et);
   }
   // ---- forward transforms, to natural order
 #pragma unroll 1

@@ -1,0 +1,35 @@
+"""The third moments of hist 'p' (stats columns 17-19 of a plane: the sums of
+v u^2, v w^2 and v^3 over its points) in the FP64 step: to FP64 rounding of the
+sum of |terms|.  The terms are good to a few 2^-53 at random (errors of the
+transforms), and the oracle adds a plane's points one after the other, an error
+of about sqrt(points) 2^-53 of the sum at most: 2^-47 for up to 2^12 rounding
+errors of one sign, 2^-49 here, with the errors of either sign."""
+import numpy as np
+import pytest
+
+from conftest import box_params, copy_state
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("grid,kw", [((32, 32, 32), {}), ((96, 48, 64), {}), ((192, 32, 48), {}),
+                                     ((64, 32, 32), {"temperature": 1, "fkappa": 0.01, "bym": 0.3})])
+def test_third_moments_to_rounding(grid, kw):
+    import oracle
+    import shear_nnf_gb300 as sb
+    pp = box_params(*grid, rez=2000.0, fixed_dt=0.004, **kw)
+    p = sb.make_params(**pp)
+    st = sb.seed_state(p, 2)
+    box, orc = sb.ShearBox(p), oracle.Oracle(**pp)
+    box.set_state(st)
+    f = {k: v.reshape(p.my, -1) for k, v in box.physical(fields=("u", "v", "w")).items()}
+    # the moments are those of the velocity without the mean shear
+    y = np.arange(p.my) * (p.Ly / p.my) - p.Ly / 2
+    u, v, w = f["u"] - y[:, None], f["v"], f["w"]
+    size = np.stack([np.abs(v * u * u).sum(1), np.abs(v * w * w).sum(1), np.abs(v ** 3).sum(1)], 1)
+    box.cross(copy_state(st), 1)
+    orc.cross(copy_state(st), 1)
+    a, b = box.statistics()["stats"][:, 16:19], orc.statistics()["stats"][:, 16:19]
+    assert (np.abs(b) <= 1.0001 * size).all() and np.abs(b).max() > 1e-3 * size.max()
+    err = np.abs(a - b) / size
+    assert err.max() < 2.0 ** -49, (err.max(0), err.mean(0))
