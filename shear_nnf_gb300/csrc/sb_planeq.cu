@@ -347,12 +347,12 @@ __global__ void __launch_bounds__(X2<NX, TEMP, NP>::T, 65536 / (X2<NX, TEMP, NP>
 #pragma unroll 1
   for (int p = 0; p < NP; p++) {
     int sh[NF], e[NF];
-    bool bad = false;
+    unsigned bad = 0;  // the fields with a number that is not finite
 #pragma unroll
     for (int f = 0; f < NF; f++) {
       sh[f] = 61 - s_len[p * NF + f];
       e[f] = s_e[p * NF + f];
-      bad |= e[f] >= kBad;
+      bad |= e[f] >= kBad ? 1u << f : 0u;
       e[f] -= sh[f];
     }
     const int a1 = e[4] + e[3], a2 = e[1] + e[5], a3 = e[1] + e[2], a4 = e[0] + e[3], a5 = e[0] + e[5],
@@ -457,13 +457,16 @@ __global__ void __launch_bounds__(X2<NX, TEMP, NP>::T, 65536 / (X2<NX, TEMP, NP>
         s_ho[p * NO + 5] = bad ? kBad : e[4] + e[NF - 1] + 64;
       }
     }
-    if (rk == 1 && !bad && umx >= umn) {
-      const double hi = fromfix_big(umx, e[0]), lo = fromfix_big(umn, e[0]);
-      m0 = fmax(m0, fmax(fabs(hi), fabs(lo)));
-      m1 = fmax(m1, fmax(fabs(hi + sy), fabs(lo + sy)));
-      m2 = fmax(m2, fromfix_big(vm, e[4]));
-      m3 = fmax(m3, fromfix_big(wm, e[1]));
-      if (TEMP) mt = fmax(mt, fromfix_big(tm, e[NF - 1]));
+    if (rk == 1 && umx >= umn) {
+      // a maximum passes over the numbers that are not finite
+      if (!(bad & 1u)) {
+        const double hi = fromfix_big(umx, e[0]), lo = fromfix_big(umn, e[0]);
+        m0 = fmax(m0, fmax(fabs(hi), fabs(lo)));
+        m1 = fmax(m1, fmax(fabs(hi + sy), fabs(lo + sy)));
+      }
+      if (!(bad & 16u)) m2 = fmax(m2, fromfix_big(vm, e[4]));
+      if (!(bad & 2u)) m3 = fmax(m3, fromfix_big(wm, e[1]));
+      if (TEMP && !(bad >> (NF - 1))) mt = fmax(mt, fromfix_big(tm, e[NF - 1]));
     }
     if (hist) {
       // the warp's sums by 32-bit reductions of 24-bit pieces, then one lane's

@@ -33,3 +33,25 @@ def test_third_moments_to_rounding(grid, kw):
     assert (np.abs(b) <= 1.0001 * size).all() and np.abs(b).max() > 1e-3 * size.max()
     err = np.abs(a - b) / size
     assert err.max() < 2.0 ** -49, (err.max(0), err.mean(0))
+
+
+@pytest.mark.parametrize("key,value", [("vor", np.nan), ("phi", np.nan), ("vor", np.inf)])
+def test_maxima_of_the_fields_that_are_finite(key, value):
+    """The time step of a state with a number that is not finite in every plane
+    of omega_y: that of max |v|, which does not depend on it; of phi: no
+    maximum at all.  As the oracle's, record by record."""
+    import oracle
+    import shear_nnf_gb300 as sb
+    pp = box_params(64, 32, 32, rez=2000.0, cfl=0.5, etime=50.0)
+    p = sb.make_params(**pp)
+    st = sb.seed_state(p, 4)
+    st[key][3, 5, :] = value
+    box, g = sb.ShearBox(p), copy_state(st)
+    tr, status = box.cross(g, 1)
+    ref, _ = oracle.Oracle(**pp).cross(copy_state(st), 1)
+    ref = np.asarray(ref)
+    assert tr.shape == ref.shape == (1, 24)
+    # time, Delta t; the maxima u + shear, v, w and u
+    for q in (0, 1, 14, 15, 16, 19):
+        np.testing.assert_allclose(tr[:, q], ref[:, q], rtol=1e-12)
+    assert status.time == pytest.approx(tr[0, 1], rel=1e-15)
