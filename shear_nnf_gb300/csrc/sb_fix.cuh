@@ -339,11 +339,12 @@ SB_HD float bits32f(unsigned u) {
 #endif
 }
 SB_HD unsigned hiword(double d) { return (unsigned)(dbits64(d) >> 32) & 0x7fffffffu; }
-// a float's bits moved to where the double of the same value has them
+// a float's bits moved to where the double of the same value has them (for a
+// subnormal number those of one just below the normal range)
 SB_HD unsigned hiword(float f) {
   const unsigned u = fbits32(f) & 0x7fffffffu;
   if (u >= 0x7f800000u) return 0x7ff00000u;
-  return u < 0x00800000u ? 0u : (u >> 3) + (896u << 20);
+  return u == 0u ? 0u : (u >> 3) + (896u << 20);
 }
 // scale of a block: the integers are x 2^p.  Zero blocks and blocks below
 // 2^-958 count as zero (a scale at which every shift empties the integer); a
