@@ -393,17 +393,17 @@ SB_HD int qclz(ull a) {
 }
 // v 2^t, rounded to nearest (|v| < 2^63).  The exponent t comes from a block's
 // scale: blocks whose results could pass the range of R are flagged by
-// qrange() first, and exponents below it give results of no size (zero for a
-// float, below 2^-900 for a double)
+// qrange() first; results below the smallest normal number are zero (a
+// float's down to its smallest subnormal are kept)
 SB_HD bool qrange(int t) { return t > 900; }
 SB_HD double fromfix(ll v, int t) {
   const ll g = v >> 63;
   ull a = (ull)((v ^ g) - g);
   const int lz = qclz(a);
   a = ((a << ((lz - 1) & 63)) + 0x200) >> 10;  // the leading bit at 52
-  const int E = (t < -1000 ? -1000 : t) + 1085 - lz;  // biased exponent less the implicit one
+  const int E = t + 1085 - lz;  // biased exponent less the implicit one
   const ull r = a + ((ull)(unsigned)E << 52);
-  return v == 0 ? 0.0 : bits64d(r | ((ull)g & 0x8000000000000000ull));
+  return v == 0 || E < 0 ? 0.0 : bits64d(r | ((ull)g & 0x8000000000000000ull));
 }
 SB_HD float fromfixf(ll v, int t) {
   const ll g = v >> 63;
