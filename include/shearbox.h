@@ -302,9 +302,12 @@ int sb_physical_fields(sb_handle *h, int member, unsigned mask, double *out);
  * my is 32, 48, 64, 80, 96, 128, 160, 192, 256, 320 or 384, without y filter or
  * dealiasing, while every box has xoffb = -xofft; else with banded solves.
  * Setting form 1 needs a handle without temperature, implicit_visc or y
- * filter/dealiasing (otherwise error 1).  sb_get_line_form gives 1 or 0, 0 with
- * the temperature, 2 with implicit_visc.  All compute the same step (to FP64
- * rounding).
+ * filter/dealiasing (otherwise error 1); on handles with one of these there is
+ * nothing to choose and setting form 0 changes nothing.  sb_get_line_form gives
+ * 1 or 0, 0 with the temperature, 2 with implicit_visc.  sb_autotune replaces
+ * an earlier choice; on boxes with xoffb != -xofft it chooses among the banded
+ * kernels, and the waves return with opposite offsets.  All compute the same
+ * step (to FP64 rounding).
  * sb_set_side_branch chooses which side work of a substep the step graph runs
  * as a branch concurrent with the plane stages: bit 0 the spectra of a
  * statistics step (beside plane stages 1-2), bit 1 the per-box scalars and

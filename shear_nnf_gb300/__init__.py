@@ -385,7 +385,8 @@ class ShearBox:
     def set_line_form(self, form: str):
         """The y-line kernels of a substep: "fused" (one kernel; handles
         without temperature, implicit_visc or y filter/dealiasing) or "split"
-        (the banded kernels; sb_set_line_form)."""
+        (the banded kernels; changes nothing on the other handles;
+        sb_set_line_form)."""
         if form not in ("fused", "split"):
             raise ValueError(f"line form {form!r}: 'fused' or 'split'")
         _check(lib().sb_set_line_form(self.h, 1 if form == "fused" else 0))

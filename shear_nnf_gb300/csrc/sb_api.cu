@@ -71,6 +71,10 @@ struct sb_handle {
   // the step runs the banded solves; step_bloch is the form captured
   std::vector<char> asym;
   int nasym = 0;
+  // Bloch waves wherever they are available; off after
+  // set_line_form("split").  Apart from Grid::lform, the choice among the
+  // banded kernels
+  bool waves = true;
   bool step_bloch = false;
   std::vector<void *> allocs;
   // the factor tables of the y-line solves depend on the segment plan: kept
@@ -136,7 +140,7 @@ static int upload(sb_handle *h, const double **dst, const std::vector<double> &v
 }
 
 // the y-line stage runs on Bloch waves (sb_bloch.cu)
-static bool use_bloch(const sb_handle *h) { return h->g.bloch && h->g.lform && h->nasym == 0; }
+static bool use_bloch(const sb_handle *h) { return h->g.bloch && h->waves && h->nasym == 0; }
 static void note_offsets(sb_handle *h, int member, double xoffb, double xofft) {
   const char a = (xoffb != -xofft);
   h->nasym += a - h->asym[member];
@@ -1447,6 +1451,12 @@ int sb_autotune(sb_handle *h, int *choice) {
   // tables), timed on whole captured steps -- the solves of a step differ in
   // kind and count per kernel, so no single kernel stands for them -- from a
   // snapshot of the state that is put back afterwards
+  // an earlier set_line_form("split") gives way to the tuner's choice
+  if (!h->waves) {
+    h->waves = true;
+    g.lform = 1;
+  }
+  const bool bloch = use_bloch(h);
   int nseg = g.nseg, lform = g.lform;
   best = 1e30f;
   Snapshot snap;
@@ -1454,16 +1464,15 @@ int sb_autotune(sb_handle *h, int *choice) {
   for (int c : {1, 2, 3}) {
     if (rc || e != cudaSuccess) break;
     if ((g.my - 3) / c < 6) continue;
-    if (g.bloch && h->nasym == 0 && c != nseg) continue;
+    if (bloch && c != nseg) continue;
     if ((rc = build_line_tables(h, c))) break;
     // both forms of the y-line stage where the fused one is available.  The
     // Bloch-wave form needs no trial against the split kernels (192x96x96
     // FP64: 90 us a substep against 123 + 258) and has no segments: one trial
-    const bool bloch = g.bloch && h->nasym == 0;
     for (int f = 1; f >= (bloch ? 1 : 0); f--) {
       if (rc || e != cudaSuccess) break;
       if (f == 1 && !bloch && !line_fused_ok(g)) continue;
-      if (!g.impl) g.lform = f;
+      if (!bloch) g.lform = f;
       if ((rc = capture_step(h))) break;
       for (int q = 0; q < 3 && e == cudaSuccess; q++) {
         if ((rc = snap.restore(h))) break;
@@ -1532,6 +1541,9 @@ int sb_set_line_form(sb_handle *h, int form) {
   if (form == 1 && (!h->g.bloch || h->g.impl || h->g.temp) &&
       !line_fused_ok(h->g))
     return fail(1, "fused y-line kernel not available for this handle");
+  // these handles have one form on waves and one banded: nothing to choose
+  if (h->g.impl || h->g.temp || h->g.ydeal) return 0;
+  h->waves = form == 1;
   h->g.lform = form;
   return capture_step(h);
 }
@@ -1553,7 +1565,7 @@ int sb_get_line_form(sb_handle *h, int *form) {
   if (!h || !form) return fail(1, "null argument");
   // the scalar's handles report the split form with the waves as well: the
   // fused banded kernel is not theirs to choose
-  const bool one = h->g.lform && !h->g.temp && (use_bloch(h) || line_fused_ok(h->g));
+  const bool one = !h->g.temp && (use_bloch(h) || (h->g.lform && line_fused_ok(h->g)));
   *form = h->g.impl ? 2 : (one ? 1 : 0);
   return 0;
 }

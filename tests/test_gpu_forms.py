@@ -1,0 +1,105 @@
+"""Which y-line form a handle runs and what may change it: "split" on handles
+that have no choice of form, the autotuner on boxes with unequal image offsets."""
+import numpy as np
+import pytest
+
+from conftest import box_params, copy_state, rel_l2
+from test_gpu_bloch import LENGTHS, _state
+from test_gpu_temperature import _temp
+
+pytestmark = pytest.mark.gpu
+KINDS = ("plain", "implicit", "temperature", "implicit_temperature")
+
+
+def _params(kind, my=48, **kw):
+    import shear_nnf_gb300 as sb
+    base = dict(fixed_dt=0.004, **({"implicit_visc": 1} if "implicit" in kind else {}))
+    base.update(kw)
+    if "temperature" in kind:
+        return sb.make_params(**_temp((64, my, 32), 1500.0, **base))
+    return sb.make_params(**box_params(64, my, 32, rez=1500.0, **base))
+
+
+def _cross(box, st, n=2):
+    s = copy_state(st)
+    box.cross(s, n)
+    return s
+
+
+def _keys(kind):
+    return ("vor", "phi", "u00", "w00") + (("tb", "tb00") if "temperature" in kind else ())
+
+
+def _same(kind, a, b):
+    for k in _keys(kind):
+        assert np.array_equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("kind", ("implicit", "temperature", "implicit_temperature"))
+def test_split_changes_nothing_where_there_is_no_choice(kind):
+    """These handles refuse "fused", so "split" must not take them off the
+    step that they run."""
+    import shear_nnf_gb300 as sb
+    p = _params(kind)
+    st = _state(p, 3, 1.3)
+    ref = _cross(sb.ShearBox(p), st)
+    box = sb.ShearBox(p)
+    form = box.tuning()["line_form"]
+    box.set_line_form("split")
+    assert box.tuning()["line_form"] == form
+    _same(kind, _cross(box, st), ref)
+    with pytest.raises(sb.ShearBoxError):
+        box.set_line_form("fused")
+    _same(kind, _cross(box, st), ref)
+
+
+def test_split_and_back():
+    import shear_nnf_gb300 as sb
+    p = _params("plain")
+    st = _state(p, 3, 1.3)
+    box = sb.ShearBox(p)
+    ref = _cross(box, st)
+    box.set_line_form("split")
+    assert box.tuning()["line_form"] == "split"
+    a = _cross(box, st)
+    assert not np.array_equal(a["phi"], ref["phi"]) and rel_l2(a["phi"], ref["phi"]) < 1e-13
+    box.set_line_form("fused")
+    assert box.tuning()["line_form"] == "fused"
+    _same("plain", _cross(box, st), ref)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_tuning_on_unequal_offsets_keeps_the_waves(kind):
+    """The autotuner on a box with xoffb != -xofft picks among the banded
+    kernels; opposite offsets afterwards run as on a fresh handle."""
+    import shear_nnf_gb300 as sb
+    p = _params(kind)
+    st = _state(p, 4, 1.1)
+    ref = _cross(sb.ShearBox(p), st)
+    box = sb.ShearBox(p)
+    box.set_state(_state(p, 4, 1.1, xoffb=-0.9))
+    box.autotune()
+    _same(kind, _cross(box, st), ref)
+
+
+@pytest.mark.parametrize("kind", ("implicit", "temperature", "implicit_temperature"))
+@pytest.mark.parametrize("my,precision", [(48, 0)] + [(n, 1) for n in LENGTHS])
+def test_waves_close_to_the_banded_solves(kind, my, precision):
+    """A box beside one with unequal offsets (banded solves for both) against
+    the same box alone (waves): FP64 rounding, FP32 rounding in the mixed form.
+    (The semi-implicit block with the scalar takes lines up to 256.)"""
+    import shear_nnf_gb300 as sb
+    if kind == "implicit_temperature" and my > 256:
+        return
+    p = _params(kind, my, fixed_dt=0.002)
+    st = _state(p, 5, 1.3)
+    one, two = sb.ShearBox(p, precision=precision), sb.ShearBox(p, batch=2, precision=precision)
+    one.set_state(st)
+    two.set_state(st, 0)
+    two.set_state(_state(p, 6, 1.3, xoffb=-0.9), 1)
+    one.step(2)
+    two.step(2)
+    a, b = one.get_state(), two.get_state(0)
+    for k in set(_keys(kind)) - {"w00"}:
+        assert rel_l2(a[k], b[k]) < (1e-6 if precision else 4e-12), k
+    assert not np.array_equal(a["phi"], b["phi"])
