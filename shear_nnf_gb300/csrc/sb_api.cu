@@ -66,7 +66,7 @@ struct sb_handle {
   // the host copies of phi run on the side stream beside those of omega_y
   cudaEvent_t ev_c0 = nullptr, ev_c1 = nullptr;
   cudaGraphExec_t step_exec = nullptr;
-  // boxes whose image offsets are not opposite (xoffb != -xofft): the
+  // boxes with shear whose image offsets are not opposite (xoffb != -xofft): the
   // Bloch-wave form needs one phase for both images, so while there is one
   // the step runs the banded solves; step_bloch is the form captured
   std::vector<char> asym;
@@ -142,7 +142,8 @@ static int upload(sb_handle *h, const double **dst, const std::vector<double> &v
 // the y-line stage runs on Bloch waves (sb_bloch.cu)
 static bool use_bloch(const sb_handle *h) { return h->g.bloch && h->waves && h->nasym == 0; }
 static void note_offsets(sb_handle *h, int member, double xoffb, double xofft) {
-  const char a = (xoffb != -xofft);
+  // without shear the image phases are one whatever the offsets
+  const char a = std::fabs(h->g.s) > 0.01 && xoffb != -xofft;
   h->nasym += a - h->asym[member];
   h->asym[member] = a;
 }

@@ -1,5 +1,6 @@
 """Which y-line form a handle runs and what may change it: "split" on handles
-that have no choice of form, the autotuner on boxes with unequal image offsets."""
+that have no choice of form, the autotuner on boxes with unequal image offsets,
+boxes without shear."""
 import numpy as np
 import pytest
 
@@ -103,3 +104,11 @@ def test_waves_close_to_the_banded_solves(kind, my, precision):
     for k in set(_keys(kind)) - {"w00"}:
         assert rel_l2(a[k], b[k]) < (1e-6 if precision else 4e-12), k
     assert not np.array_equal(a["phi"], b["phi"])
+
+
+def test_offsets_do_not_matter_without_shear():
+    """s = 0: the image phases are one whatever the offsets."""
+    import shear_nnf_gb300 as sb
+    p = _params("plain", s=0.0)
+    a = _cross(sb.ShearBox(p), _state(p, 7, 1.1))
+    _same("plain", _cross(sb.ShearBox(p), _state(p, 7, 1.1, xoffb=-0.9)), a)
