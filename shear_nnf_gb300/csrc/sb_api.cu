@@ -65,17 +65,19 @@ struct sb_handle {
   int branch = 3;
   // the host copies of phi run on the side stream beside those of omega_y
   cudaEvent_t ev_c0 = nullptr, ev_c1 = nullptr;
-  cudaGraphExec_t step_exec = nullptr;
-  // boxes with shear whose image offsets are not opposite (xoffb != -xofft): the
-  // Bloch-wave form needs one phase for both images, so while there is one
-  // the step runs the banded solves; step_bloch is the form captured
+  // one RK3 step on the banded solves and on Bloch waves, each captured when
+  // first needed; step_bloch is the one in use
+  cudaGraphExec_t step_exec[2] = {nullptr, nullptr};
+  bool step_bloch = false;
+  // boxes with shear whose image offsets are not opposite (xoffb != -xofft):
+  // the Bloch-wave form needs one phase for both images, so while there is one
+  // the step runs the banded solves
   std::vector<char> asym;
   int nasym = 0;
   // Bloch waves wherever they are available; off after
   // set_line_form("split").  Apart from Grid::lform, the choice among the
   // banded kernels
   bool waves = true;
-  bool step_bloch = false;
   std::vector<void *> allocs;
   // the factor tables of the y-line solves depend on the segment plan: kept
   // apart so that a new plan (sb_set_line_segments, the autotuner) can
@@ -237,6 +239,17 @@ static int upload_uniform(sb_handle *h, Fac *F, const double a[7], int n) {
   return 0;
 }
 
+// the step graph of a form, to be captured again when it is next needed
+static void drop_graph(sb_handle *h, bool bloch) {
+  if (h->step_exec[bloch]) cudaGraphExecDestroy(h->step_exec[bloch]);
+  h->step_exec[bloch] = nullptr;
+}
+static void set_form(sb_handle *h, bool bloch) {
+  h->step_bloch = bloch;
+  h->bf.Gn = bloch ? h->bf.S : h->bf.G;
+  h->bf.Dn = bloch ? h->bf.T : h->bf.D;
+}
+
 // The factor tables of the y-line solves for a segment plan of nseg warps per
 // line: d/dy and d2/dy2 (and the y-filter), each the same for every line, and
 // the Helmholtz operator (rh2 - k^2 pr2) per (kx, kz >= 0) line (lapcdy,
@@ -256,6 +269,10 @@ static int build_line_tables(sb_handle *h, int nseg) {
     g.shi[q] = plan0.hi[q];
   }
   if (h->st) cudaStreamSynchronize(h->st);
+  // a failure below leaves no graph of the old tables and none called complete
+  const bool full = h->banded;
+  h->banded = false;
+  drop_graph(h, false);
   for (void *q : h->line_allocs) cudaFree(q);
   h->line_allocs.clear();
   h->alloc_to = &h->line_allocs;
@@ -273,7 +290,7 @@ static int build_line_tables(sb_handle *h, int nseg) {
       (rc = upload_uniform(h, &bf.d2, co.pr2, g.my)) ||
       (g.ydeal == 3 && (rc = upload_uniform(h, &bf.flt, flhs, g.my))))
     return rc;
-  if (h->banded) {
+  if (full) {
     // lines (kx, kz) and (kx, -kz) share k^2 and so their factors: the table
     // holds the kz >= 0 lines only (hz_line maps a line to its entry)
     const int nlh = g.nkx * (g.nz + 1);
@@ -331,7 +348,7 @@ static int build_line_tables(sb_handle *h, int nseg) {
     }
     H.stride = nlh;
   }
-  if (g.impl && h->banded) {
+  if (g.impl && full) {
     // the semi-implicit Helmholtz tables, filled by k_hfac every substep:
     // boxes x (lines (kx, kz >= 0) + the mean line)
     const size_t n = g.my, L = (size_t)g.B * (g.nkx * (g.nz + 1) + 1);
@@ -369,17 +386,15 @@ static int build_line_tables(sb_handle *h, int nseg) {
   }
   if (prepare_line(g) != cudaSuccess)
     return fail(3, "line kernel attributes: %s", cudaGetErrorString(cudaGetLastError()));
+  h->banded = full;
   return 0;
 }
-
 
 // the banded solves' tables, where the handle has done without so far
 static int ensure_banded(sb_handle *h) {
   if (h->banded) return 0;
   h->banded = true;
-  const int rc = build_line_tables(h, h->g.nseg);
-  h->banded = rc == 0;
-  return rc;
+  return build_line_tables(h, h->g.nseg);
 }
 
 // fixed-point twiddles of length n
@@ -522,19 +537,9 @@ static cudaError_t launch_phases(sb_handle *h, int rk, cudaStream_t st) {
   return h->step_bloch ? launch_bloch(h->g, h->bf, rk, st) : launch_tables(h->g, h->bf, rk, st);
 }
 
-static int capture_step(sb_handle *h) {
-  if (!use_bloch(h)) {
-    const int rc = ensure_banded(h);
-    if (rc) return rc;
-  }
-  if (h->step_exec) {
-    cudaGraphExecDestroy(h->step_exec);
-    h->step_exec = nullptr;
-  }
+// one step in the form that is set
+static int capture_graph(sb_handle *h, cudaGraphExec_t *exec) {
   cudaGraph_t graph;
-  h->step_bloch = use_bloch(h);
-  h->bf.Gn = h->step_bloch ? h->bf.S : h->bf.G;
-  h->bf.Dn = h->step_bloch ? h->bf.T : h->bf.D;
   CK(cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
   cudaError_t e = cudaSuccess;
   const bool hfac = h->g.impl && !h->step_bloch;  // the factors of k_lineI
@@ -603,9 +608,32 @@ static int capture_step(sb_handle *h) {
   cudaError_t e2 = cudaStreamEndCapture(h->st, &graph);
   if (e != cudaSuccess) return fail(3, "kernel launch during capture: %s", cudaGetErrorString(e));
   if (e2 != cudaSuccess) return fail(3, "capture: %s", cudaGetErrorString(e2));
-  CK(cudaGraphInstantiate(&h->step_exec, graph, 0));
+  e = cudaGraphInstantiate(exec, graph, 0);
   cudaGraphDestroy(graph);
+  if (e != cudaSuccess) {
+    *exec = nullptr;
+    return fail(3, "graph: %s", cudaGetErrorString(e));
+  }
   return 0;
+}
+
+// the step in the given form, with its tables and its graph; where they cannot
+// be made the form that was set stays
+static int select_form(sb_handle *h, bool bloch) {
+  int rc;
+  if (!bloch && (rc = ensure_banded(h))) return rc;
+  const bool old = h->step_bloch;
+  set_form(h, bloch);
+  if (h->step_exec[bloch] || !(rc = capture_graph(h, &h->step_exec[bloch]))) return 0;
+  set_form(h, old);
+  return rc;
+}
+
+// after a change of what the step's kernels are given
+static int capture_step(sb_handle *h) {
+  drop_graph(h, false);
+  drop_graph(h, true);
+  return select_form(h, use_bloch(h));
 }
 
 // v from phi and the first derivatives of the state at the start of a run, by
@@ -616,9 +644,8 @@ static cudaError_t launch_prologue(sb_handle *h) {
 
 // the step graph's form for the boxes' current offsets
 static int ensure_form(sb_handle *h) {
-  if (h->step_bloch == use_bloch(h)) return 0;
-  CK(cudaStreamSynchronize(h->st));
-  return capture_step(h);
+  const bool bloch = use_bloch(h);
+  return h->step_bloch == bloch && h->step_exec[bloch] ? 0 : select_form(h, bloch);
 }
 
 static int ensure_trace(sb_handle *h, int cap) {
@@ -938,7 +965,8 @@ int sb_create(const sb_params *p, int batch, int precision, sb_handle **out) {
 int sb_destroy(sb_handle *h) {
   if (!h) return 0;
   if (h->st) cudaStreamSynchronize(h->st);
-  if (h->step_exec) cudaGraphExecDestroy(h->step_exec);
+  drop_graph(h, false);
+  drop_graph(h, true);
   for (void *q : h->allocs) cudaFree(q);
   for (void *q : h->line_allocs) cudaFree(q);
   if (h->hs) cudaFreeHost(h->hs);
@@ -1206,7 +1234,7 @@ int sb_step(sb_handle *h, int nsteps) {
   CK(launch_setconj(h->g, h->bf, h->st));
   if (h->g.ydeal == 3) CK(launch_filter(h->g, h->bf, 0, h->st));
   CK(launch_prologue(h));
-  for (int s = 0; s < nsteps; s++) CK(cudaGraphLaunch(h->step_exec, h->st));
+  for (int s = 0; s < nsteps; s++) CK(cudaGraphLaunch(h->step_exec[h->step_bloch], h->st));
   return 0;
 }
 
@@ -1386,7 +1414,7 @@ static cudaError_t launch_step_call(sb_handle *h, int nsteps) {
       (h->g.ydeal == 3 && (e = launch_filter(h->g, h->bf, 0, h->st)) != cudaSuccess) ||
       (e = launch_prologue(h)) != cudaSuccess)
     return e;
-  for (int s = 0; s < nsteps && e == cudaSuccess; s++) e = cudaGraphLaunch(h->step_exec, h->st);
+  for (int s = 0; s < nsteps && e == cudaSuccess; s++) e = cudaGraphLaunch(h->step_exec[h->step_bloch], h->st);
   return e;
 }
 

@@ -1,6 +1,8 @@
 """Which y-line form a handle runs and what may change it: "split" on handles
 that have no choice of form, the autotuner on boxes with unequal image offsets,
-boxes without shear."""
+boxes without shear, changes of form between calls."""
+import time
+
 import numpy as np
 import pytest
 
@@ -112,3 +114,29 @@ def test_offsets_do_not_matter_without_shear():
     p = _params("plain", s=0.0)
     a = _cross(sb.ShearBox(p), _state(p, 7, 1.1))
     _same("plain", _cross(sb.ShearBox(p), _state(p, 7, 1.1, xoffb=-0.9)), a)
+
+
+def test_changes_of_form_cost_one_capture():
+    """Equal and unequal offsets in turn: the bits of fresh handles, and after
+    the first pair no step call waits or captures again."""
+    import shear_nnf_gb300 as sb
+    p = _params("plain")
+    st = [_state(p, 8, 1.1), _state(p, 8, 1.1, xoffb=-0.9)]
+    ref = [_cross(sb.ShearBox(p), s) for s in st]
+    box = sb.ShearBox(p)
+    for q in (0, 1, 0, 1):
+        _same("plain", _cross(box, st[q]), ref[q])
+
+    def enqueue(order):
+        best = []
+        for q in order:
+            box.set_state(st[q])
+            t = time.perf_counter()
+            box.step(1)
+            best.append(time.perf_counter() - t)
+            box.sync()
+        return min(best)
+
+    same = max(enqueue([0] * 10), enqueue([1] * 10))
+    # a call takes 12 us, a capture of the step graph 120 more
+    assert enqueue([0, 1] * 10) < 3 * same + 2e-5
