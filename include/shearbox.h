@@ -272,7 +272,10 @@ int sb_kspace_get(sb_kspace *ks, int col, long off, long len, double *host);
  * kernels and 11 the LES y-line kernel; with implicit_visc, 13 the
  * factorisation of the substep's Helmholtz operators and 14 its banded y-line
  * kernel.  The launches act on the current device state, so a run that used
- * them must set the state again before stepping.
+ * them must set the state again before stepping.  On a handle on Bloch waves
+ * 5, 6, 13 and 14 change the single stages to the banded kernels, up to the
+ * next step: the first takes the derived fields from the banded solves of the
+ * current state, and the right-hand sides as the last stage 3 left them.
  * sb_fp64_peak measures the device's FP64 FMA throughput in TFLOP/s. */
 int sb_launch_stage(sb_handle *h, int stage, int rk, int count);
 

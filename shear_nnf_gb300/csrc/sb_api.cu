@@ -1328,6 +1328,29 @@ int sb_crosst(sb_handle *h, double *vor, double *phi, double *u00, double *w00, 
 
 void *sb_get_stream(sb_handle *h) { return h ? (void *)h->st : nullptr; }
 
+// Single stages of a handle on Bloch waves change to the banded kernels, up to
+// its next step: the derived fields (v, the first derivatives, d2(omega_y)/dy2)
+// from the banded solves of the current state, the right-hand sides of plane
+// stage 3 where the banded kernels of substep rk look for them, their tables.
+static int stages_banded(sb_handle *h, int rk) {
+  const Grid &g = h->g;
+  const int rc = select_form(h, false);
+  if (rc) return rc;
+  const size_t bytes = (g.prec ? sizeof(float) : sizeof(double)) * g.field * (size_t)g.B;
+  // xbuf is free after plane stage 3 and holds more than a field
+  auto copy = [&](void *dst, const void *src) {
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, h->st);
+  };
+  CK(copy(h->bf.xbuf, h->bf.V));
+  CK(launch_tables(g, h->bf, 0, h->st));
+  CK(launch_lineB(g, h->bf, 0, h->st));
+  CK(copy(h->bf.V, h->bf.xbuf));
+  CK(copy(h->bf.G, h->bf.S));
+  CK(copy(h->bf.D, h->bf.T));
+  CK(launch_tables(g, h->bf, rk, h->st));
+  return 0;
+}
+
 int sb_launch_stage(sb_handle *h, int stage, int rk, int count) {
   if (!h || count < 0) return fail(1, "bad argument");
   if (stage < 1 || stage > 14 || rk < 1 || rk > 3) return fail(1, "stage 1..14, rk 1..3");
@@ -1335,10 +1358,13 @@ int sb_launch_stage(sb_handle *h, int stage, int rk, int count) {
   if (stage == 12 && !h->step_bloch && !line_fused_ok(h->g))
     return fail(1, "stage 12 (fused y-line kernel) not available for this handle");
   if (stage >= 13 && !h->g.impl) return fail(1, "stages 13, 14 need an implicit_visc handle");
-  if ((stage == 5 || stage == 6 || stage >= 13) && !h->banded) {
-    // the tables it replaces may be those of the step graph
-    int rc = ensure_banded(h);
-    if (rc || (rc = capture_step(h))) return rc;
+  if (!h->step_exec[h->step_bloch]) {
+    const int rc = ensure_form(h);
+    if (rc) return rc;
+  }
+  if ((stage == 5 || stage == 6 || stage >= 13) && h->step_bloch) {
+    const int rc = stages_banded(h, rk);
+    if (rc) return rc;
   }
   for (int q = 0; q < count; q++) {
     cudaError_t e;

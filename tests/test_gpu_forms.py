@@ -1,6 +1,6 @@
 """Which y-line form a handle runs and what may change it: "split" on handles
 that have no choice of form, the autotuner on boxes with unequal image offsets,
-boxes without shear, changes of form between calls."""
+boxes without shear, changes of form between calls, single stages."""
 import time
 
 import numpy as np
@@ -140,3 +140,27 @@ def test_changes_of_form_cost_one_capture():
     same = max(enqueue([0] * 10), enqueue([1] * 10))
     # a call takes 12 us, a capture of the step graph 120 more
     assert enqueue([0, 1] * 10) < 3 * same + 2e-5
+
+
+@pytest.mark.parametrize("kind", ("plain", "implicit"))
+def test_banded_stages_on_a_handle_on_waves(kind):
+    """Substep 2 of a step by single stages, the banded y-line kernels on a
+    handle that steps on waves, against a handle that runs them (beside a box
+    with unequal offsets): stages 1-4, then 5 and 6, or 13 and 14."""
+    import shear_nnf_gb300 as sb
+    p = _params(kind)
+    st = _state(p, 9, 1.3)
+    one, two = sb.ShearBox(p), sb.ShearBox(p, batch=2)
+    two.set_state(_state(p, 6, 1.3, xoffb=-0.9), 1)
+    out = []
+    for box in (one, two):
+        box.set_state(st, 0)
+        box.step(1)
+        for stage in (1, 2, 3, 4) + ((13, 14) if kind == "implicit" else (5, 6)):
+            box.launch_stage(stage, 2)
+        box.sync()
+        out.append(box.get_state(0))
+    for k in ("vor", "phi", "u00"):
+        assert np.isfinite(out[0][k]).all() and rel_l2(out[0][k], out[1][k]) < 4e-12, k
+    # and the next step is the handle's own again
+    _same(kind, _cross(one, st), _cross(sb.ShearBox(p), st))
