@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/shearbox.h"
@@ -78,6 +79,8 @@ struct sb_handle {
   // set_line_form("split").  Apart from Grid::lform, the choice among the
   // banded kernels
   bool waves = true;
+  // waves and tables of the Bloch-wave form
+  void *wave_mem = nullptr;
   std::vector<void *> allocs;
   // the factor tables of the y-line solves depend on the segment plan: kept
   // apart so that a new plan (sb_set_line_segments, the autotuner) can
@@ -110,8 +113,37 @@ int handle_batch(const sb_handle *h) { return h->g.B; }
 int handle_trace_len(const sb_handle *h) { return h->g.tlen; }
 }  // namespace sb
 
-static int dmalloc(sb_handle *h, void **p, size_t bytes) {
+// the step graph of a form, to be captured again when it is next needed
+static void drop_graph(sb_handle *h, bool bloch) {
+  if (h->step_exec[bloch]) cudaGraphExecDestroy(h->step_exec[bloch]);
+  h->step_exec[bloch] = nullptr;
+}
+static void set_form(sb_handle *h, bool bloch) {
+  h->step_bloch = bloch;
+  h->bf.Gn = bloch ? h->bf.S : h->bf.G;
+  h->bf.Dn = bloch ? h->bf.T : h->bf.D;
+}
+
+// Device memory of a handle.  Where there is no room the waves go first: a
+// handle that fits without them steps on the banded solves.
+static bool drop_waves(sb_handle *h) {
+  if (!h->wave_mem) return false;
+  cudaStreamSynchronize(h->st);
+  drop_graph(h, true);
+  cudaFree(h->wave_mem);
+  h->wave_mem = nullptr;
+  h->g.bloch = 0;
+  if (h->step_bloch) set_form(h, false);
+  return true;
+}
+static cudaError_t malloc_room(sb_handle *h, void **p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  return drop_waves(h) ? cudaMalloc(p, bytes) : e;
+}
+static int dmalloc(sb_handle *h, void **p, size_t bytes) {
+  const cudaError_t e = malloc_room(h, p, bytes);
   if (e != cudaSuccess) return fail(4, "cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
   cudaMemset(*p, 0, bytes);
   (h->alloc_to ? *h->alloc_to : h->allocs).push_back(*p);
@@ -237,17 +269,6 @@ static int upload_uniform(sb_handle *h, Fac *F, const double a[7], int n) {
   if ((rc = upload(h, &F->rows, rows))) return rc;
   F->stride = 0;
   return 0;
-}
-
-// the step graph of a form, to be captured again when it is next needed
-static void drop_graph(sb_handle *h, bool bloch) {
-  if (h->step_exec[bloch]) cudaGraphExecDestroy(h->step_exec[bloch]);
-  h->step_exec[bloch] = nullptr;
-}
-static void set_form(sb_handle *h, bool bloch) {
-  h->step_bloch = bloch;
-  h->bf.Gn = bloch ? h->bf.S : h->bf.G;
-  h->bf.Dn = bloch ? h->bf.T : h->bf.D;
 }
 
 // The factor tables of the y-line solves for a segment plan of nseg warps per
@@ -390,12 +411,6 @@ static int build_line_tables(sb_handle *h, int nseg) {
   return 0;
 }
 
-// the banded solves' tables, where the handle has done without so far
-static int ensure_banded(sb_handle *h) {
-  if (h->banded) return 0;
-  h->banded = true;
-  return build_line_tables(h, h->g.nseg);
-}
 
 // fixed-point twiddles of length n
 static int upload_qw(sb_handle *h, const qw **dst, const std::vector<int> &v) {
@@ -470,7 +485,6 @@ static int build_plane_tables(sb_handle *h) {
 static int build_bloch_tables(sb_handle *h) {
   Grid &g = h->g;
   Bufs &bf = h->bf;
-  h->asym.assign((size_t)g.B, 0);
   g.bloch = line_bloch_ok(g) ? 1 : 0;
   if (!g.bloch) return 0;
   sbh::Coeffs co;
@@ -482,25 +496,41 @@ static int build_bloch_tables(sb_handle *h) {
   g.bn1p = (double)((ld)g.rh1[4] - 2.0L * g.rh1[5] + 3.0L * g.rh1[6]);
   g.bp1p = (double)(1.0L - 2.0L * ((ld)co.pr1[4] - co.pr1[5] + co.pr1[6]));
   g.bp2p = (double)(1.0L - 2.0L * ((ld)co.pr2[4] - co.pr2[5] + co.pr2[6]));
-  const size_t m = 3 * (size_t)g.B * n * g.nkx;
   int rc;
-  double *q;
-  if ((rc = dalloc(h, &q, 2 * m))) return rc;
-  bf.btw = (qw *)q;
-  if ((rc = dalloc(h, &q, (2 + g.temp) * (size_t)g.B * g.field))) return rc;
-  bf.bw = (q2 *)q;
-  if ((rc = dalloc(h, &q, (1 + g.temp) * 4 * (size_t)g.B * n))) return rc;
-  bf.bwm = (q2 *)q;
-  if ((rc = dalloc(h, &q, (size_t)(2 + g.temp) * g.B * (g.plane / 2 + 2) / 2 + 1))) return rc;
-  bf.bwp = (int *)q;
-  if ((rc = dalloc(h, &q, 2 * (m / 3)))) return rc;
-  bf.bm1 = (double2 *)q;
-  if ((rc = dalloc(h, &q, 2 * (m / 3)))) return rc;
-  bf.bm2 = (double2 *)q;
-  if ((rc = dalloc(h, &bf.bl1, m)) || (rc = dalloc(h, &bf.bl2, m)) ||
-      (rc = upload_fix(h, &bf.bftw, n, -1, false)) || (rc = upload_fix(h, &bf.bitw, n, 1, true)) ||
+  if ((rc = upload_fix(h, &bf.bftw, n, -1, false)) ||
+      (rc = upload_fix(h, &bf.bitw, n, 1, true)) ||
       (rc = upload_fix(h, &bf.bturn, 1024, -1, false)))
     return rc;
+  // the waves and the phase tables, in one piece (drop_waves)
+  const size_t m = (size_t)g.B * n * g.nkx, nf = 2 + g.temp;
+  size_t used = 0;
+  auto place = [&](auto **p, size_t bytes) {
+    *p = (std::remove_reference_t<decltype(*p)>)((char *)h->wave_mem + used);
+    used += (bytes + 255) / 256 * 256;
+  };
+  auto layout = [&] {
+    used = 0;
+    place(&bf.btw, 3 * m * sizeof(qw));
+    place(&bf.bw, nf * g.B * g.field * sizeof(double));
+    place(&bf.bwm, (1 + g.temp) * 2 * (size_t)g.B * n * sizeof(q2));
+    place(&bf.bwp, nf * g.B * (g.plane / 2 + 2) * sizeof(int));
+    place(&bf.bm1, m * sizeof(double2));
+    place(&bf.bm2, m * sizeof(double2));
+    place(&bf.bl1, 3 * m * sizeof(double));
+    place(&bf.bl2, 3 * m * sizeof(double));
+  };
+  layout();
+  cudaError_t e = cudaMalloc(&h->wave_mem, used);
+  if (e == cudaErrorMemoryAllocation) {
+    // no memory for them: the banded solves, as for the other line lengths
+    cudaGetLastError();
+    h->wave_mem = nullptr;
+    g.bloch = 0;
+    return 0;
+  }
+  CK(e);
+  CK(cudaMemset(h->wave_mem, 0, used));
+  layout();
   if (prepare_lineQ(g, bf) != cudaSuccess)
     return fail(3, "line kernel attributes: %s", cudaGetErrorString(cudaGetLastError()));
   return 0;
@@ -530,6 +560,22 @@ static void member_defaults(const sb_params *p, const Grid &g, double Re, Member
   m->keep_laminar = p->keep_laminar;
   // thermal diffusion CFL (initcr.f90:498-502)
   m->cflkk = p->temperature ? p->fkappa / p->CFL * mm : 0.0;
+}
+
+// the banded solves' tables, where the handle has done without so far; where
+// they don't fit even in the place of the waves it keeps those
+static int ensure_banded(sb_handle *h) {
+  if (h->banded) return 0;
+  const bool had = h->wave_mem != nullptr;
+  h->banded = true;
+  const int rc = build_line_tables(h, h->g.nseg);
+  if (rc == 4 && had && !h->wave_mem) {
+    for (void *q : h->line_allocs) cudaFree(q);
+    h->line_allocs.clear();
+    build_bloch_tables(h);
+    return fail(4, "no memory for the tables of the banded solves");
+  }
+  return rc;
 }
 
 // the phase tables of substep rk (0: the start of a run)
@@ -931,9 +977,13 @@ int sb_create(const sb_params *p, int batch, int precision, sb_handle **out) {
     sb_destroy(h);
     return rc;
   }
-  h->banded = !line_bloch_ok(g);
-  if ((rc = build_line_tables(h, g.nseg)) || (rc = build_bloch_tables(h)) ||
-      (rc = build_plane_tables(h))) {
+  h->asym.assign(B, 0);
+  if ((rc = build_bloch_tables(h))) {
+    sb_destroy(h);
+    return rc;
+  }
+  h->banded = !g.bloch;
+  if ((rc = build_line_tables(h, g.nseg)) || (rc = build_plane_tables(h))) {
     sb_destroy(h);
     return rc;
   }
@@ -969,6 +1019,7 @@ int sb_destroy(sb_handle *h) {
   drop_graph(h, true);
   for (void *q : h->allocs) cudaFree(q);
   for (void *q : h->line_allocs) cudaFree(q);
+  if (h->wave_mem) cudaFree(h->wave_mem);
   if (h->hs) cudaFreeHost(h->hs);
   if (h->st) cudaStreamDestroy(h->st);
   if (h->side) cudaStreamDestroy(h->side);
@@ -1408,7 +1459,7 @@ struct Snapshot {
     }
     for (auto &pt : parts) {
       void *q = nullptr;
-      if (cudaMalloc(&q, pt.second) != cudaSuccess) {
+      if (malloc_room(h, &q, pt.second) != cudaSuccess) {
         release();
         return fail(4, "autotune: no memory for the state snapshot");
       }
@@ -1511,11 +1562,11 @@ int sb_autotune(sb_handle *h, int *choice) {
     h->waves = true;
     g.lform = 1;
   }
+  Snapshot snap;
+  rc = snap.take(h);
   const bool bloch = use_bloch(h);
   int nseg = g.nseg, lform = g.lform;
   best = 1e30f;
-  Snapshot snap;
-  rc = snap.take(h);
   for (int c : {1, 2, 3}) {
     if (rc || e != cudaSuccess) break;
     if ((g.my - 3) / c < 6) continue;
@@ -1642,10 +1693,29 @@ int sb_physical_fields(sb_handle *h, int member, unsigned mask, double *out) {
   if (!nout) return 0;
   const Grid &g = h->g;
   cudaStream_t st = h->st;
+  // the transforms' planes and the fields
+  const size_t nout_d = (size_t)nout * g.my * g.mgalz * g.mgalx;
+  double *zb = nullptr, *od = nullptr;
+  auto room = [&](double **q, size_t n) -> cudaError_t {
+    cudaError_t e = cudaMallocAsync((void **)q, sizeof(double) * n, st);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    return drop_waves(h) ? cudaMallocAsync((void **)q, sizeof(double) * n, st) : e;
+  };
+  CK(room(&zb, (size_t)g.my * g.mgalz * 10 * g.nkx * 2));
+  cudaError_t e = room(&od, nout_d);
+  if (e != cudaSuccess) {
+    cudaFreeAsync(zb, st);
+    return fail(3, "physical fields: %s", cudaGetErrorString(e));
+  }
   // the derived fields of the current state (v, dv/dy, d(omega_y)/dy, mean
   // derivatives), as at the entry of a call
   const int frc = ensure_form(h);
-  if (frc) return frc;
+  if (frc) {
+    cudaFreeAsync(zb, st);
+    cudaFreeAsync(od, st);
+    return frc;
+  }
   CK(launch_scalar(g, h->bf, 0, st));
   CK(launch_phases(h, 0, st));
   CK(launch_setconj(g, h->bf, st));
@@ -1670,12 +1740,8 @@ int sb_physical_fields(sb_handle *h, int member, unsigned mask, double *out) {
   bl.mu += member * Md;
   bl.mdu += member * Md;
   bl.mem += member;
-  const size_t nout_d = (size_t)nout * g.my * g.mgalz * g.mgalx;
-  double *zb = nullptr, *od = nullptr;
-  CK(cudaMallocAsync((void **)&zb, sizeof(double) * (size_t)g.my * g.mgalz * 10 * g.nkx * 2, st));
-  CK(cudaMallocAsync((void **)&od, sizeof(double) * nout_d, st));
   bl.zbuf = zb;
-  cudaError_t e = launch_physical(gl, bl, mask, od, st);
+  e = launch_physical(gl, bl, mask, od, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(out, od, sizeof(double) * nout_d, cudaMemcpyDeviceToHost, st);
   cudaFreeAsync(zb, st);
   cudaFreeAsync(od, st);

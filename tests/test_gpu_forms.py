@@ -1,6 +1,7 @@
 """Which y-line form a handle runs and what may change it: "split" on handles
 that have no choice of form, the autotuner on boxes with unequal image offsets,
-boxes without shear, changes of form between calls, single stages."""
+boxes without shear, changes of form between calls, single stages, memory that
+does not hold the waves."""
 import time
 
 import numpy as np
@@ -164,3 +165,44 @@ def test_banded_stages_on_a_handle_on_waves(kind):
         assert np.isfinite(out[0][k]).all() and rel_l2(out[0][k], out[1][k]) < 4e-12, k
     # and the next step is the handle's own again
     _same(kind, _cross(one, st), _cross(sb.ShearBox(p), st))
+
+
+def test_memory_for_the_banded_form_alone():
+    """Where memory does not hold the waves the handle steps without them, as
+    it would have before there were any."""
+    torch = pytest.importorskip("torch")
+    import shear_nnf_gb300 as sb
+    p = _params("plain")
+    batch = 512
+    st = _state(p, 10, 1.3)
+
+    def run(box):
+        for m in (0, 1, batch - 1):
+            box.set_state(st, m)
+        box.step(2)
+        return box.get_state(batch - 1)
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    for _ in range(2):  # the first loads the kernels
+        before = free()
+        box = sb.ShearBox(p, batch=batch)
+        used = before - free()
+        a = run(box)
+        box.close()
+    waves = 8 * batch * 2 * 2 * st["vor"].size  # 16 bytes for each number of vor and phi
+    fill = torch.empty(free() - used + waves // 2, dtype=torch.uint8, device="cuda")
+    try:
+        box = sb.ShearBox(p, batch=batch)
+        left = free()
+        b = run(box)
+        box.close()
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    assert left > waves // 4  # not for want of anything else
+    for k in ("vor", "phi", "u00"):
+        assert rel_l2(b[k], a[k]) < 4e-12, k
+    assert not np.array_equal(a["phi"], b["phi"])
