@@ -9,9 +9,10 @@ step (three substeps) of that box.
          (one sb_step call, CUDA events on the library's stream).
   e2e    steps/s through the C-ABI drop-in sb_cross(nstep=1) with pinned host
          buffers: host->device state, one step, device->host state, per step.
-  roofline  the dominant kernel (plane stage 2), timed alone with CUDA events:
-         FP64 rate against the FP64 FMA peak measured in the same run (the
-         binding roof on GB300) and bytes against the measured HBM copy peak.
+  roofline  the dominant kernel (plane stage 2): the share of the issue slots in
+         use (committed ncu summary; latency bounds it); timed alone with CUDA
+         events its bytes against the measured HBM copy peak and the FP64 rate
+         that the same work would take against the FP64 FMA peak of this run.
   les     Smagorinsky LES on 384x192x192 (Re_z=20000), FP32-mixed vs FP64.
   temperature  the crosst variant (Boussinesq scalar, Pr=0.7) on the benchmark
          box, FP64 and FP32-mixed, against the plain step.
@@ -158,18 +159,26 @@ def measured_peaks():
         return 6800.0, "fallback"
 
 
-def plane2_traffic():
-    """dram bytes per launch of plane stage 2 from the committed ncu summary
-    (profiles/k_x2_192x96x96.txt, line 'traffic_bytes_per_launch: N'), else None."""
-    path = os.path.join(ROOT, "profiles", "k_x2_192x96x96.txt")
+def plane2_counters():
+    """Counters of plane stage 2 from the committed ncu summary
+    (profiles/k_x2_192x96x96.txt): dram bytes per launch, warps per SM and the
+    shares of the issue slots and of the pipes' peaks, in percent."""
+    keys = {"traffic_bytes_per_launch:": "traffic",
+            "sm__issue_active.avg.pct_of_peak_sustained_elapsed": "issue",
+            "sm__inst_executed_pipe_alu.avg.pct_of_peak_sustained_active": "alu",
+            "sm__inst_executed_pipe_fma.avg.pct_of_peak_sustained_active": "fma",
+            "sm__inst_executed_pipe_fp64.avg.pct_of_peak_sustained_active": "fp64",
+            "sm__warps_active.avg.per_cycle_active": "warps_per_sm"}
+    out = dict.fromkeys(keys.values())
     try:
-        with open(path) as f:
+        with open(os.path.join(ROOT, "profiles", "k_x2_192x96x96.txt")) as f:
             for line in f:
-                if line.startswith("traffic_bytes_per_launch:"):
-                    return float(line.split(":")[1])
+                w = line.split()
+                if w and w[0] in keys:
+                    out[keys[w[0]]] = float(w[1])
     except OSError:
         pass
-    return None
+    return out
 
 
 def cpu_baseline(nsteps_sample: int, threads: int, warmup: int = 1):
@@ -663,7 +672,7 @@ def run_ours(args):
     hbm_peak, hbm_src = measured_peaks()
     p2_tflops = p2_flops / (p2_ms * 1e-3) / 1e12
     p2_gbs = p2_bytes / (p2_ms * 1e-3) / 1e9
-    traffic = plane2_traffic()
+    counters = plane2_counters()
     # end to end through the drop-in with pinned host buffers
     nf = st0["vor"].size
     pin = {}
@@ -775,17 +784,24 @@ def run_ours(args):
                                 "max": float(calls_ms.max())}},
         "gpu_launches": launches,
         "roofline": {
-            "bound": "integer issue",
+            # no pipe is near its peak: warps wait on the instruction before,
+            # on global and shared loads and on barriers
+            "bound": "latency (issue slots in use)",
             "kernel": "k_x2 (plane stage 2 in 64-bit fixed point: x transforms, u x omega)",
-            "achieved": p2_gbs, "peak": hbm_peak, "unit": "GB/s", "frac": p2_gbs / hbm_peak,
-            "peak_source": f"MEASURED_PEAKS.json ({hbm_src})",
+            "achieved": counters["issue"], "peak": 100.0, "unit": "% of the issue slots",
+            "frac": counters["issue"] / 100.0 if counters["issue"] else None,
+            "peak_source": "ncu summary profiles/k_x2_192x96x96.txt",
+            "counters": {k: counters[k] for k in ("alu", "fma", "fp64", "warps_per_sm")},
             "algorithmic_bytes_per_launch": p2_bytes, "launch_ms": p2_ms,
+            "dram": {"achieved": p2_gbs, "peak": hbm_peak, "unit": "GB/s",
+                     "frac": p2_gbs / hbm_peak,
+                     "peak_source": f"MEASURED_PEAKS.json ({hbm_src})"},
             # the same flops on the FP64 pipe, which the kernel replaces by integers
             "fp64_equivalent": {"achieved": p2_tflops, "peak": fp64_peak, "unit": "TFLOP/s",
                                 "ratio": p2_tflops / fp64_peak,
                                 "peak_source": "FP64 FMA probe measured in this run",
                                 "algorithmic_flops_per_launch": p2_flops},
-            "traffic": traffic,
+            "traffic": counters["traffic"],
             "line_kernels_ms": {"k_lineA": line_ms[0], "k_lineB": line_ms[1], "k_lineQ": lineF_ms},
         },
         "mixed_value": mixed["value"] if mixed else None,
