@@ -19,7 +19,15 @@
  *     complex(0:my1, 0:mx1, 0:mz1) stored as interleaved (re, im) doubles, y
  *     fastest (cross.f90:32-33, the `buffsize` arrays of main.f90:67 with one
  *     rank); u00/w00 are real(0:my1).  Host memory is caller-owned and copied;
- *     device memory is owned by the handle.
+ *     device memory is owned by the handle.  A box's Bloch waves and their
+ *     tables (sb_set_line_form) are 8-10% of its memory; a handle that does not
+ *     fit with them, or another of whose allocations fails, does without and
+ *     steps on the banded solves.
+ *   - the FP64 step's transforms and the y-operators hold a sequence (row,
+ *     column, y-line) at one power of two: errors are relative to its norm, and
+ *     a part of a y-line quieter than 2^-55 of the line's rms is lost in them.
+ *     A sequence of FP64 numbers below 2^-958 counts as zero; one with a number
+ *     that is not finite, or results beyond 2^900, gives NaN.
  *   - a handle holds `batch` independent boxes of one grid; it is not reentrant
  *     and owns one CUDA stream.  No CPU fallback exists: creation fails if no
  *     GPU is present.

@@ -1,7 +1,7 @@
 // sb_api.cu -- C-ABI of the shearing-box time stepper (see include/shearbox.h).
 //
 // Host side of the step: owns the device state of a batch of boxes, uploads
-// the factor tables computed by sb_host.cpp, captures one RK3 step (sixteen
+// the factor tables computed by sb_host.cpp, captures one RK3 step (21
 // kernel launches) in a CUDA graph and replays it.  The reference's MPI/OpenMP
 // structure (cross.f90 with change.allfac_ieor.f transposes) has no
 // counterpart: one handle is one GPU, one stream.

@@ -28,6 +28,13 @@
 // thread (k1, column) the waves k1 + R1 k2 (R2-point kernels); one exchange
 // through shared memory between them, none between a forward transform and
 // the inverse ones that follow it.
+//
+// Bound by latency: 12 warps per SM (registers), issue slots 30% in use, the
+// FP64 pipe 34%, the ALU pipe 29% (192x96x96); warps wait for the instruction
+// before, for rows from global memory, for shared memory and at barriers.
+//
+// Errors are relative to a line: a part of it that is quiet by more than 2^-55
+// of the line's rms drowns there, where a banded solve kept its own accuracy.
 #include <cuda_runtime.h>
 
 #include <type_traits>
@@ -575,7 +582,7 @@ __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineQ(Grid
 //   mean    rf0u += d(T12_00)/dy, rf0w += d(T23_00)/dy              (txy -> mrf)
 // One transform and its inverse a line, where k_lineL spends a banded FP64 solve
 // (384x192x192 mixed: 264 us against 909; 192x96x96 FP64: 34 against 121).  Bound
-// by the integer pipes, as k_lineQ.
+// by latency, as k_lineQ.
 template <typename R, int N, int T>
 __global__ void __launch_bounds__(T, 65536 / (T * LineQRegs<N>::n)) k_lineLQ(Grid g, Bufs bf, int rk) {
   typedef LineQ<N> L;
