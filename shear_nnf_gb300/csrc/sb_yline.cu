@@ -951,7 +951,8 @@ __global__ void __launch_bounds__((TEMP ? 96 : 64) * kSeg, 1) k_lineI(Grid g, Bu
         zs = cmul_c(wz, __shfl_xor_sync(0xffffffffu, wz, 1), m1, c);
       }
       if (L.active) {
-        rhs_out[q] = (R)rm;
+        // the mean block reads -vT of the (0,0) line, whose own tb is not solved
+        if (!(TEMP && pipe == 2 && is00)) rhs_out[q] = (R)rm;
         if (rk < 2) fwk[q] = (R)zs;
       }
     }
