@@ -45,9 +45,11 @@ __device__ __forceinline__ q2 qshift(q2 x, int s) {
   return mkq((ll)((ull)x.x << l) >> r, (ll)((ull)x.y << l) >> r);
 }
 __device__ __forceinline__ int bitlen(unsigned v) { return 32 - __clz((int)v); }
-// v 2^t, past the range as a large number (its step is stopped as diverged)
+// v 2^t, past the range as an infinity
 __device__ __forceinline__ double fromfix_big(ll v, int t) {
-  return qrange(t) ? (v == 0 ? 0.0 : v < 0 ? -1e300 : 1e300) : fromfix(v, t);
+  const double inf = __longlong_as_double(0x7ff0000000000000ll);
+  const bool big = v != 0 && t + 64 - qclz((ull)(v < 0 ? -v : v)) > 1024;
+  return big ? (v < 0 ? -inf : inf) : fromfix(v, t);
 }
 // a b / 2^64; |a|, |b| <= 2^62
 __device__ __forceinline__ ll qprod(ll a, ll b) { return qmulr(a, qhi(b), qlo(b)); }
@@ -502,12 +504,13 @@ __global__ void __launch_bounds__(X2<NX, TEMP, NP>::T, 65536 / (X2<NX, TEMP, NP>
     // one triple per (plane, row pair); k_hsum adds the pairs
     const int p = threadIdx.x / 3, q = threadIdx.x - 3 * p;
     auto ef = [&](int f) { return s_e[p * NF + f] - (61 - s_len[p * NF + f]); };
-    bool bad = false;
-    for (int f = 0; f < NF; f++) bad |= s_e[p * NF + f] >= kBad;
+    // a sum over numbers that are not finite
+    const bool bad = s_e[p * NF + 4] >= kBad || s_e[p * NF + (q == 0 ? 0 : q == 1 ? 1 : 4)] >= kBad;
     const int e2 = q == 0 ? ef(0) : q == 1 ? ef(1) : ef(4);
     const int et = ef(4) + 2 * e2 + 128 - 3;
+    const double hi = fromfix_big(s_third[p][q], et + 16);
     bf.ppart[(((long)b * g.my + j) * (NZ / 2) + z0 / 2 + p) * 3 + q] =
-        bad ? nan("") : fromfix_big(s_third[p][q], et + 16) + fromfix_big(s_rest[p][q], et);
+        bad ? nan("") : isinf(hi) ? hi : hi + fromfix_big(s_rest[p][q], et);
   }
   // ---- forward transforms, to natural order
 #pragma unroll 1

@@ -55,3 +55,42 @@ def test_maxima_of_the_fields_that_are_finite(key, value):
     for q in (0, 1, 14, 15, 16, 19):
         np.testing.assert_allclose(tr[:, q], ref[:, q], rtol=1e-12)
     assert status.time == pytest.approx(tr[0, 1], rel=1e-15)
+
+
+def _moments(pp, st):
+    import oracle
+    import shear_nnf_gb300 as sb
+    box, orc = sb.ShearBox(sb.make_params(**pp)), oracle.Oracle(**pp)
+    box.cross(copy_state(st), 1)
+    orc.cross(copy_state(st), 1)
+    return [np.asarray(x.statistics()["stats"])[:, 16:19] for x in (box, orc)]
+
+
+def test_moments_of_the_fields_that_are_finite():
+    """A NaN in one plane of omega_y: u and w are lost in that plane alone, v
+    nowhere, and with them the moments."""
+    import shear_nnf_gb300 as sb
+    pp = box_params(64, 32, 48, rez=2000.0, fixed_dt=0.004)
+    st = sb.seed_state(sb.make_params(**pp), 6)
+    st["vor"][2, 3, 11] = np.nan
+    a, b = _moments(pp, st)
+    assert np.array_equal(np.isfinite(a), np.isfinite(b))
+    assert np.isfinite(a[:, 2]).all() and np.isfinite(a[:, :2]).sum() == 2 * 31
+    ok = np.isfinite(a)
+    np.testing.assert_allclose(a[ok], b[ok], rtol=1e-11, atol=1e-11 * np.abs(b[ok]).max())
+
+
+@pytest.mark.parametrize("scale,finite", [(1e90, True), (1e120, False)])
+def test_moments_past_the_range(scale, finite):
+    """Velocities whose third powers pass the range of FP64 give no number."""
+    import shear_nnf_gb300 as sb
+    pp = box_params(64, 32, 48, rez=2000.0, fixed_dt=0.004)
+    st = sb.seed_state(sb.make_params(**pp), 6)
+    for k in ("vor", "phi", "u00", "w00"):
+        st[k] = st[k] * scale
+    a, b = _moments(pp, st)
+    assert np.isfinite(a).all() == np.isfinite(b).all() == finite
+    if finite:
+        assert np.abs(a / scale ** 3 - b / scale ** 3).max() < 1e-11 * np.abs(b / scale ** 3).max()
+    else:
+        assert not np.isfinite(a).any()
