@@ -1693,33 +1693,28 @@ int sb_physical_fields(sb_handle *h, int member, unsigned mask, double *out) {
   if (!nout) return 0;
   const Grid &g = h->g;
   cudaStream_t st = h->st;
-  // the transforms' planes and the fields
+  // the transforms' planes and the fields, allocated while the first kernels run
   const size_t nout_d = (size_t)nout * g.my * g.mgalz * g.mgalx;
+  const size_t nz_d = (size_t)g.my * g.mgalz * 10 * g.nkx * 2;
   double *zb = nullptr, *od = nullptr;
-  auto room = [&](double **q, size_t n) -> cudaError_t {
-    cudaError_t e = cudaMallocAsync((void **)q, sizeof(double) * n, st);
-    if (e != cudaErrorMemoryAllocation) return e;
-    cudaGetLastError();
-    return drop_waves(h) ? cudaMallocAsync((void **)q, sizeof(double) * n, st) : e;
-  };
-  CK(room(&zb, (size_t)g.my * g.mgalz * 10 * g.nkx * 2));
-  cudaError_t e = room(&od, nout_d);
-  if (e != cudaSuccess) {
-    cudaFreeAsync(zb, st);
-    return fail(3, "physical fields: %s", cudaGetErrorString(e));
-  }
-  // the derived fields of the current state (v, dv/dy, d(omega_y)/dy, mean
-  // derivatives), as at the entry of a call
-  const int frc = ensure_form(h);
-  if (frc) {
-    cudaFreeAsync(zb, st);
-    cudaFreeAsync(od, st);
-    return frc;
-  }
-  CK(launch_scalar(g, h->bf, 0, st));
-  CK(launch_phases(h, 0, st));
-  CK(launch_setconj(g, h->bf, st));
-  CK(launch_prologue(h));
+  cudaError_t e;
+  do {
+    // the derived fields of the current state (v, dv/dy, d(omega_y)/dy, mean
+    // derivatives), as at the entry of a call
+    const int frc = ensure_form(h);
+    if (frc) return frc;
+    CK(launch_scalar(g, h->bf, 0, st));
+    CK(launch_phases(h, 0, st));
+    CK(launch_setconj(g, h->bf, st));
+    CK(launch_prologue(h));
+    e = cudaMallocAsync((void **)&zb, sizeof(double) * nz_d, st);
+    if (e == cudaSuccess) {
+      e = cudaMallocAsync((void **)&od, sizeof(double) * nout_d, st);
+      if (e != cudaSuccess) cudaFreeAsync(zb, st);
+    }
+    if (e != cudaSuccess) cudaGetLastError();
+  } while (e == cudaErrorMemoryAllocation && drop_waves(h));
+  if (e != cudaSuccess) return fail(3, "physical fields: %s", cudaGetErrorString(e));
   // one box: member-offset buffers, plane stage 1 with the extra z-transforms
   Grid gl = g;
   gl.B = 1;
