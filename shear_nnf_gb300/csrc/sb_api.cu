@@ -588,7 +588,11 @@ static int capture_graph(sb_handle *h, cudaGraphExec_t *exec) {
   cudaGraph_t graph;
   CK(cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
   cudaError_t e = cudaSuccess;
-  const bool hfac = h->g.impl && !h->step_bloch;  // the factors of k_lineI
+  // the factors of k_lineI; beside the fixed-point plane stage 3, whose blocks
+  // take the shared memory that k_hfac wants as cache, they take three times as
+  // long (128x72x128 step 3540 us against 2400 in order; where that does not
+  // happen they gain 1%: 160x75x80 2393 against 2421)
+  const bool hfac = h->g.impl && !h->step_bloch, hside = hfac && !h->g.planeq;
   for (int rk = 1; rk <= 3 && e == cudaSuccess; rk++) {
     if (h->g.ydeal == 3 && (e = launch_filter(h->g, h->bf, rk, h->st)) != cudaSuccess) break;
     if ((h->g.ydeal == 1 || h->g.ydeal == 2) &&
@@ -618,10 +622,11 @@ static int capture_graph(sb_handle *h, cudaGraphExec_t *exec) {
           (e = cudaStreamWaitEvent(h->side, h->ev_fork, 0)) != cudaSuccess ||
           (e = launch_scalar(h->g, h->bf, rk, h->side)) != cudaSuccess ||
           (e = launch_phases(h, rk, h->side)) != cudaSuccess ||
-          (hfac && (e = launch_hfac(h->g, h->bf, rk, h->side)) != cudaSuccess) ||
+          (hside && (e = launch_hfac(h->g, h->bf, rk, h->side)) != cudaSuccess) ||
           (e = cudaEventRecord(h->ev_join, h->side)) != cudaSuccess ||
           (e = launch_plane(h->g, h->bf, 3, rk, h->st)) != cudaSuccess ||
-          (e = cudaStreamWaitEvent(h->st, h->ev_join, 0)) != cudaSuccess)
+          (e = cudaStreamWaitEvent(h->st, h->ev_join, 0)) != cudaSuccess ||
+          (hfac && !hside && (e = launch_hfac(h->g, h->bf, rk, h->st)) != cudaSuccess))
         break;
     } else {
       // in order on the main stream; with LES, k_scalar also takes the

@@ -206,3 +206,30 @@ def test_memory_for_the_banded_form_alone():
     for k in ("vor", "phi", "u00"):
         assert rel_l2(b[k], a[k]) < 4e-12, k
     assert not np.array_equal(a["phi"], b["phi"])
+
+
+def test_side_work_does_not_slow_the_banded_semi_implicit_step():
+    """The side branch of the step graph may not cost what it hides: its time
+    against the same work in order (medians of nine; the branches differ by a
+    few percent)."""
+    torch = pytest.importorskip("torch")
+    import shear_nnf_gb300 as sb
+    p = sb.make_params(**box_params(128, 72, 128, rez=1500.0, fixed_dt=0.001, implicit_visc=1))
+    box = sb.ShearBox(p)
+    st = sb.seed_state(p, 1)
+    stream = torch.cuda.ExternalStream(box.stream)
+    took = {}
+    for mask in (0, 1, 2, 3):
+        box.set_side_branch(mask)
+        box.set_state(st)
+        box.step(2)
+        times = []
+        for _ in range(9):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record(stream)
+            box.step(2)
+            b.record(stream)
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        took[mask] = sorted(times)[4]
+    assert max(took.values()) < 1.15 * min(took.values()), took
