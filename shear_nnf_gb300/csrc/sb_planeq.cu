@@ -233,7 +233,8 @@ __global__ void __launch_bounds__(Z1<NZ>::T, Z1<NZ>::kMinB) k_z1(Grid g, Bufs bf
 // ---------------------------------------------------------------------------
 // NP row pairs of a block: two where the blocks fill the GPU and fit in shared
 // memory, else one (64x32x32 alone: 10.4 us against 14.1; 384x192x192: 802 us
-// against 1065, where two pairs leave two blocks an SM)
+// against 1065, where two pairs leave two blocks an SM; with the shifts
+// rounding 10.7 and 833, and 103.6 at 192x96x96 for the 99.7 below)
 template <int NX, bool TEMP, int NP>
 struct X2 {
   static constexpr int R1 = Plan<NX>::R1, R2 = Plan<NX>::R2;
